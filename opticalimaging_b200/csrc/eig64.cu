@@ -1,98 +1,475 @@
 // FP64 top-K eigenpairs of a Hermitian positive semi-definite operator, for the SOCS decomposition
 // (DecomposeTCC_SOCS.py:7-9, where the reference takes a full torch.svd of its complex64 TCC and keeps the
-// leading K singular pairs).  Block subspace iteration with Rayleigh-Ritz, on the GPU, in double precision:
+// leading K singular pairs).  Subspace iteration on a block of p vectors with Rayleigh-Ritz, on the GPU, in double
+// precision:
 //
-//   X = orthonormal(random n x p)
-//   repeat:   Y = T X,   X = CholQR2(Y)                      (Cholesky QR twice: X^H X = I to rounding)
-//   every `check` iterations: Z = T X, H = X^H Z (p x p), H = Q diag(w) Q^H (cyclic Jacobi), residuals
-//             ||Z q_i - w_i X q_i|| of the leading k; stop when their maximum is below tol * w_0.
-//   result:   the Ritz pairs (w_i, X q_i), i < k, eigenvalues descending and clamped at zero.
+//   X = random n x p;   EIG_START times:  X R = T X          (Cholesky QR twice: X^H X = I to rounding)
+//   X R = f(T) X, f the Chebyshev polynomial that is small on [0, lambda_p], of the degree that should reach tol
+//   repeat:   Z = T X, H = X^H Z (p x p), H = Q diag(w) Q^H (cyclic Jacobi), X = X Q, Z = Z Q, residuals
+//             ||Z_i - w_i X_i|| of the leading k; stop when their maximum is below tol * w_0, else another filter
+//   result:   the Ritz pairs (w_i, X_i), i < k, eigenvalues descending and clamped at zero.
 //
-// The subspace converges like (lambda_{p+1} / lambda_k)^iterations; the TCC's spectrum decays, so a block of
-// p = 64 vectors resolves the leading 24 of the 2048 nm configuration (lambda_65 / lambda_24 = 0.21) to a
-// rank-24 projector error of 1e-12 in about 16 iterations.  T is a dense n x n matrix or the factored form
-// T = sum_e h_e h_e^H (h [ne][n][s], the scaled pupil matrix of CalculateTCCMatrix.py:33-51), applied without
-// forming T.  Kernels: a tiled complex FP64 GEMM (row-major, optional conjugate transpose of A, split over K
-// with partial sums added in a fixed order), and one-CTA kernels for the p x p steps (Cholesky and triangular
-// inverse, Jacobi eigendecomposition, residual norms).
-#include "oi_common.cuh"
-#include <cstdint>
-#include <vector>
+// Plain subspace iteration gains lambda_{p+1} / lambda_k per product with T; the filter on the unwanted interval
+// gains rho = x + sqrt(x^2 - 1), x = 2 lambda_k / lambda_p - 1, per product (configuration 3, k = 24, p = 64: 4.8
+// against 18).  Both ends of the interval come from the last projection, or before the first one from the diagonal of
+// R, which after EIG_START iterations holds the leading eigenvalues to some per cent: most operators then need one
+// projection (configuration 3: 13 products with T and 6 orthonormalisations; 21 products, 17 orthonormalisations and
+// 4 projections without the filter).  A filter is cut into pieces whose amplification of lambda_0 over lambda_k stays
+// below EIG_AMP, with an orthonormalisation after each: the columns, ordered by eigenvalue, then stay independent to
+// working precision.  Where the interval does not separate (lambda_p too near lambda_k) or a filter did not help,
+// plain iterations run instead.
+//
+// T is a dense n x n matrix or the factored form T = sum_e h_e h_e^H (h [ne][n][s], the scaled pupil matrix of
+// CalculateTCCMatrix.py:33-51), applied without forming T.  Both hold many zero blocks (pupil samples outside the
+// shifted discs): a pass over the operand marks its non-zero 16 x 16 blocks once, and the products skip the rest.
+#include "zgemm64.cuh"
+#include <algorithm>
 #include <cmath>
+#include <vector>
 
 namespace oi {
+
+namespace zg {
+
+__global__ void __launch_bounds__(256) mark_blocks_kernel(const double2* __restrict__ M, int rows, int cols,
+                                                          unsigned char* __restrict__ flags, int fc) {
+  const int col = blockIdx.x * 256 + threadIdx.x, r16 = blockIdx.y;
+  const double2* m = M + (long long)blockIdx.z * rows * cols;
+  bool nz = false, bad = false;
+  if (col < cols) {
+#pragma unroll 4
+    for (int i = 0; i < KC; ++i) {
+      const int r = r16 * KC + i;
+      if (r >= rows) break;
+      const double2 v = __ldg(m + (long long)r * cols + col);
+      nz |= v.x != 0.0 || v.y != 0.0;
+      bad |= !isfinite(v.x) || !isfinite(v.y);
+    }
+  }
+  const unsigned n = __ballot_sync(0xffffffffu, nz), b = __ballot_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 15) == 0) {
+    const int c16 = col >> 4, sh = threadIdx.x & 16;
+    if (c16 < fc)
+      flags[((long long)blockIdx.z * gridDim.y + r16) * fc + c16] =
+          (((n >> sh) & 0xffffu) ? 1 : 0) | (((b >> sh) & 0xffffu) ? 2 : 0);
+  }
+}
+
+int mark_blocks(const double2* M, int batch, int rows, int cols, unsigned char* flags, cudaStream_t s) {
+  dim3 grid((unsigned)ceil_div(cols, 256), (unsigned)flag_dim(rows), (unsigned)batch);
+  if (grid.y > 65535 || grid.z > 65535) return fail(OI_ERANGE, "mark_blocks: %d x %d x %d too large", batch, rows, cols);
+  mark_blocks_kernel<<<grid, 256, 0, s>>>(M, rows, cols, flags, flag_dim(cols));
+  note_launch();
+  return check_launch("mark_blocks");
+}
+
+}  // namespace zg
+
 namespace eg {
 
-constexpr int BM = 32, BN = 32, BK = 16;   // GEMM tile
-constexpr int PMAX = 64;                   // block size limit of the one-CTA steps
+constexpr int PMAX = 64;                   // block size limit (one column tile, and the one-CTA steps)
+constexpr int EIG_START = 3;               // plain iterations before the first filter
+constexpr int EIG_DEGREE = 12;             // products with T between projections, at most
+constexpr double EIG_AMP = 1e8;            // a filter piece's amplification of lambda_0 over lambda_k
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 conjd(double2 a) { return make_double2(a.x, -a.y); }
 
-// C[z][m][n] = sum_{kk in chunk z} op(A)[i][kk] B[kk][j]; op(A) = A (A [m][lda]) or A^H (A [k][lda]).
-// With one chunk and acc = 1 the result is added to C.
-template <bool AH>
-__global__ void __launch_bounds__(256) zgemm_kernel(int m, int n, int k, const double2* __restrict__ A, long long lda,
-                                                    const double2* __restrict__ B, long long ldb, double2* C,
-                                                    long long ldc, int kchunk, int acc) {
-  __shared__ double2 As[BK][BM + 1];
-  __shared__ double2 Bs[BK][BN + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, z = blockIdx.z;
-  const int k0 = z * kchunk, k1 = min(k, k0 + kchunk);
-  double2 c00 = make_double2(0, 0), c01 = c00, c10 = c00, c11 = c00;
-  for (int kt = k0; kt < k1; kt += BK) {
-    for (int e = threadIdx.x; e < BM * BK; e += 256) {
-      int i, kk;
-      if (AH) {   // coalesced along i: A[kt + kk][m0 + i]
-        i = e % BM;
-        kk = e / BM;
-      } else {    // coalesced along kk: A[m0 + i][kt + kk]
-        kk = e % BK;
-        i = e / BK;
-      }
-      const int gi = m0 + i, gk = kt + kk;
-      double2 v = make_double2(0, 0);
-      if (gi < m && gk < k1) v = AH ? conjd(A[(long long)gk * lda + gi]) : A[(long long)gi * lda + gk];
-      As[kk][i] = v;
-    }
-    for (int e = threadIdx.x; e < BK * BN; e += 256) {
-      const int j = e % BN, kk = e / BN, gj = n0 + j, gk = kt + kk;
-      Bs[kk][j] = (gj < n && gk < k1) ? B[(long long)gk * ldb + gj] : make_double2(0, 0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      const double2 a0 = As[kk][2 * ty], a1 = As[kk][2 * ty + 1], b0 = Bs[kk][2 * tx], b1 = Bs[kk][2 * tx + 1];
-      cfma(c00, a0, b0);
-      cfma(c01, a0, b1);
-      cfma(c10, a1, b0);
-      cfma(c11, a1, b1);
-    }
-    __syncthreads();
-  }
-  const int i0 = m0 + 2 * ty, j0 = n0 + 2 * tx;
-  double2* Cz = C + (long long)z * m * ldc;
-  auto put = [&](int i, int j, double2 v) {
-    if (i < m && j < n) {
-      double2* p = Cz + (long long)i * ldc + j;
-      *p = acc ? cadd(*p, v) : v;
-    }
-  };
-  put(i0, j0, c00);
-  put(i0, j0 + 1, c01);
-  put(i0 + 1, j0, c10);
-  put(i0 + 1, j0 + 1, c11);
+// Tile of block i of n: from the middle outwards.  The middle rows of a TCC (low frequencies) have the most non-zero
+// blocks; started first, they do not end last.
+__device__ __forceinline__ int heavy_first(int i, int n) {
+  const int m = n / 2;
+  return i & 1 ? m - 1 - i / 2 : m + i / 2;
 }
 
-// out[e] (+)= sum_z parts[z][e], z = 0 .. nparts-1 in order.
-__global__ void reduce_parts_kernel(const double2* __restrict__ parts, int nparts, long long count, double2* out,
-                                    int acc) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= count) return;
-  double2 s = acc ? out[e] : make_double2(0, 0);
-  for (int z = 0; z < nparts; ++z) s = cadd(s, parts[(long long)z * count + e]);
-  out[e] = s;
+// parts[(bat * splits + z)][m][p] = the share z of op(A_bat) B_bat: 64 rows per block (blockIdx.x), share blockIdx.y,
+// batch blockIdx.z.  AH false: A = M [m][k], K over nseg segments of k (segment e at M + e * sm), B [nseg * k][p].
+// AH true: A = conj(M_bat)^T, M_bat [k][m].  Share z takes the chunks z, z + splits, ... so that zero blocks spread
+// over the shares.
+struct GemmArgs {
+  const double2* M;
+  long long sm;                  // elements between segments / batches of M
+  int m, k, nseg, p;
+  const double2* B;
+  double2* parts;
+  const unsigned char* flags;    // of M (zg::mark_blocks)
+  int fr, fc;
+};
+template <bool AH>
+__global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  pdl_trigger();
+  pdl_wait();
+  const int mt = heavy_first(blockIdx.x, gridDim.x), m0 = mt * zg::T, splits = gridDim.y, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int per = (a.k + zg::KC - 1) / zg::KC;
+  const double2* M = a.M + (AH ? blockIdx.z * a.sm : 0);
+  const unsigned char* fl = a.flags + (AH ? (long long)blockIdx.z * a.fr * a.fc : 0);
+  double2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
+  auto active = [&](int c) {
+    const int e = c / per, kc = c - e * per;
+    unsigned f = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      f |= AH ? fl[(long long)kc * a.fc + 4 * mt + u] : fl[((long long)e * a.fr + 4 * mt + u) * a.fc + kc];
+    return (f & 1u) != 0;
+  };
+  auto load = [&](int c, double2* As, double2* Bs) {
+    const int e = c / per, k0 = (c - e * per) * zg::KC;
+    if (AH)
+      zg::load_cols(As, M, a.m, m0, a.m, k0, a.k);
+    else
+      zg::load_rows(As, M + e * a.sm, a.k, m0, a.m, k0, a.k);
+    zg::load_cols(Bs, a.B + (long long)e * a.k * a.p, a.p, 0, a.p, k0, a.k);
+  };
+  zg::tile_loop<AH ? zg::CONJ_A : zg::NONE>(acc, smem, blockIdx.y, splits, per * a.nseg, active, load);
+  double2* out = a.parts + ((long long)blockIdx.z * splits + blockIdx.y) * a.m * a.p;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = m0 + ty + 16 * i, c = tx + 16 * j;
+      if (r < a.m && c < a.p) out[(long long)r * a.p + c] = acc[i][j];
+    }
+}
+
+// Row-block kernels: each block takes groups of RB rows (g, g + gridDim.x, ...) of n x p arrays.  gram: the block's
+// share of L^H Y (Hermitian: L = Y, or Y = T L), accumulated over its groups by the outputs (ty + 16 i, tx + 16 j),
+// i <= j, of each thread.
+template <int RB>
+__device__ __forceinline__ void gram_rows(double2 (&acc)[4][4], const double2* L, const double2* Y, int tx, int ty) {
+#pragma unroll 4
+  for (int r = 0; r < RB; ++r) {
+    double2 a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = L[r * PMAX + ty + 16 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) b[u] = Y[r * PMAX + tx + 16 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = u; v < 4; ++v) cfma_conj(acc[u][v], b[v], a[u]);
+  }
+}
+__device__ __forceinline__ void store_gram(const double2 (&acc)[4][4], double2* gparts, int tx, int ty) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = i; j < 4; ++j) gparts[(long long)blockIdx.x * PMAX * PMAX + (ty + 16 * i) * PMAX + tx + 16 * j] = acc[i][j];
+}
+
+// out = alpha sum_z parts[z] + beta b1 + gamma b0 (rows of n x p; batch blockIdx.y of n rows), and, with gparts, the
+// shares of left^H out (left null: out^H out).  out may be b0.
+struct FoldArgs {
+  const double2* parts;
+  int nparts, n, p;
+  double alpha, beta, gamma;
+  const double2 *b1, *b0, *left;
+  double2 *out, *gparts;
+};
+template <int RB>
+__global__ void __launch_bounds__(256) fold_kernel(FoldArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double2* ys = (double2*)smem;                  // [RB][64]
+  double2* ls = a.left ? ys + RB * PMAX : ys;    // left's rows, when given
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  pdl_trigger();
+  pdl_wait();
+  const long long np = (long long)a.n * a.p, boff = blockIdx.y * np;
+  double2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
+  for (int g = blockIdx.x; g * RB < a.n; g += gridDim.x) {
+    double2 v[RB / 4];
+#pragma unroll
+    for (int i = 0; i < RB / 4; ++i) v[i] = make_double2(0, 0);
+    const int c = tid & 63;
+    auto at = [&](int i) { return (long long)(g * RB + (tid >> 6) + 4 * i) * a.p + c; };
+    auto in = [&](int i) { return c < a.p && g * RB + (tid >> 6) + 4 * i < a.n; };
+    for (int z = 0; z < a.nparts; ++z) {
+      const double2* p = a.parts + boff * a.nparts + z * np;
+#pragma unroll
+      for (int i = 0; i < RB / 4; ++i)
+        if (in(i)) v[i] = cadd(v[i], p[at(i)]);
+    }
+#pragma unroll
+    for (int i = 0; i < RB / 4; ++i) {
+      double2 y = make_double2(a.alpha * v[i].x, a.alpha * v[i].y), l = make_double2(0, 0);
+      if (in(i)) {
+        const long long e = at(i);
+        if (a.b1) {
+          const double2 b = a.b1[e];
+          y.x = fma(a.beta, b.x, y.x);
+          y.y = fma(a.beta, b.y, y.y);
+        }
+        if (a.b0) {
+          const double2 b = a.b0[e];
+          y.x = fma(a.gamma, b.x, y.x);
+          y.y = fma(a.gamma, b.y, y.y);
+        }
+        a.out[boff + e] = y;
+        if (a.left) l = a.left[e];
+      }
+      ys[((tid >> 6) + 4 * i) * PMAX + c] = y;
+      if (a.left) ls[((tid >> 6) + 4 * i) * PMAX + c] = l;
+    }
+    if (a.gparts) {
+      __syncthreads();
+      gram_rows<RB>(acc, ls, ys, tx, ty);
+      __syncthreads();
+    }
+  }
+  if (a.gparts) store_gram(acc, a.gparts, tx, ty);
+}
+
+// G[r][c] = sum_b gparts[b][r][c] (p x p of the 64 x 64 shares), in a fixed order, for the stored 16 x 16 blocks, and
+// their mirror images.
+__global__ void __launch_bounds__(256) sum_gram_kernel(const double2* gparts, int nparts, int p, double2* G) {
+  __shared__ double2 sh[4][64];
+  pdl_trigger();
+  pdl_wait();
+  const int c = threadIdx.x & 63, q = threadIdx.x >> 6, r = blockIdx.x;
+  if ((c >> 4) < (r >> 4)) nparts = 0;
+  double2 s = make_double2(0, 0);
+#pragma unroll 8
+  for (int b = q; b < nparts; b += 4) s = cadd(s, gparts[(long long)b * PMAX * PMAX + r * PMAX + c]);
+  sh[q][c] = s;
+  __syncthreads();
+  if (q != 0 || c >= p || (c >> 4) < (r >> 4)) return;
+  s = cadd(cadd(sh[0][c], sh[1][c]), cadd(sh[2][c], sh[3][c]));
+  G[r * p + c] = s;
+  if ((c >> 4) > (r >> 4)) G[c * p + r] = conjd(s);
+}
+
+// One CTA: from the Gram matrix G of a block X, Rinv such that X Rinv has orthonormal columns:
+// S scales the columns (first pass: to unit length, diag(G)^-1/2; second pass: not at all, so that columns which the
+// first pass found dependent and left near zero stay there), shift is added to the diagonal against rank deficiency
+// (a pivot below it is raised to it), S G S + shift = L D L^H with L unit lower triangular, Rinv = S L^-H D^-1/2.
+// The elimination of the columns builds L^-1 in place: step j subtracts (A[a][j] / d_j) times row j from the rows
+// a > j, where columns c > j still hold the trailing matrix, columns c < j hold L^-1 and column j becomes -A[a][j] / d_j.
+// rdiag[c] = the diagonal of R = (X Rinv)^H X (the second pass multiplies the two passes' factors).
+// Bound: the chain of 64 dependent steps.  Each thread keeps its 2 x 4 entries (ty + 32 i, tx + 16 j) in registers; a
+// step is one barrier (row j and column j through a double-buffered line of shared memory, 1 / d_j by the entry's
+// owner).  64 x 64: CHOL_US us; with the matrix in shared memory, three barriers a step and a back substitution by one
+// thread per column it was 277 us.
+__global__ void __launch_bounds__(512) chol_inv_kernel(int p, const double2* G, double2* Rinv, double* rdiag,
+                                                       double shift, bool first) {
+  __shared__ double2 rowb[2][PMAX], colb[2][PMAX];
+  __shared__ double invb[2], sc[PMAX], D[PMAX];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  pdl_trigger();
+  pdl_wait();
+  if (tid < PMAX) {
+    const double g = tid < p ? G[tid * p + tid].x : 1.0;
+    sc[tid] = !first ? 1.0 : g > 0 ? 1.0 / sqrt(g) : 0.0;
+  }
+  __syncthreads();
+  double2 a[2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = ty + 32 * i, c = tx + 16 * j;
+      double2 v = make_double2(r == c ? 1.0 : 0.0, 0);
+      if (r < p && c < p) v = G[r * p + c];
+      const double s = sc[r] * sc[c];
+      a[i][j] = r == c ? make_double2(v.x * s + shift, 0.0) : make_double2(v.x * s, v.y * s);
+    }
+#pragma unroll
+  for (int jb = 0; jb < 4; ++jb) {
+#pragma unroll 1
+    for (int jj = 0; jj < 16; ++jj) {
+      const int j = 16 * jb + jj, buf = j & 1;
+      const bool col = tx == jj;   // this thread holds column j, as a[.][jb]
+      if (ty == (j & 31)) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rowb[buf][tx + 16 * k] = a[jb >> 1][k];
+        if (col) {
+          double d = a[jb >> 1][jb].x;
+          if (!(d > shift)) d = shift;
+          D[j] = d;
+          invb[buf] = 1.0 / d;
+        }
+      }
+      if (col) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) colb[buf][ty + 32 * i] = a[i][jb];
+      }
+      __syncthreads();
+      const double inv = -invb[buf];
+      double2 row[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) row[k] = rowb[buf][tx + 16 * k];
+      if (col) row[jb] = make_double2(1.0, 0.0);   // column j becomes the multiplier itself
+#pragma unroll
+      for (int i = jb >> 1; i < 2; ++i) {   // rows of the block before are done
+        const bool on = ty + 32 * i > j;
+        double2 m = colb[buf][ty + 32 * i];
+        m = on ? make_double2(m.x * inv, m.y * inv) : make_double2(0, 0);
+        if (on && col) a[i][jb] = make_double2(0, 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (i > (jb >> 1) || on) cfma(a[i][k], m, row[k]);
+        }
+      }
+    }
+  }
+  __syncthreads();   // D
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = ty + 32 * i, c = tx + 16 * j;   // L^-1[r][c] -> Rinv[c][r]
+      if (r >= p || c >= p) continue;
+      const double s = c <= r ? sc[c] / sqrt(D[r]) : 0.0;
+      const double2 v = r == c ? make_double2(1, 0) : a[i][j];
+      Rinv[c * p + r] = c <= r ? make_double2(v.x * s, -v.y * s) : make_double2(0, 0);
+    }
+  if (tid < p) {
+    const double d = sqrt(D[tid]);
+    rdiag[tid] = !first ? rdiag[tid] * d : sc[tid] > 0 ? d / sc[tid] : 0.0;
+  }
+}
+
+// Loads a group of RB rows of an n x p array (zero beyond) into [RB][PMAX].
+template <int RB>
+__device__ __forceinline__ void load_group(double2* s, const double2* src, int n, int p, int g) {
+#pragma unroll
+  for (int i = 0; i < RB / 4; ++i) {
+    const int e = threadIdx.x + 256 * i, r = e >> 6, c = e & 63;
+    s[e] = g * RB + r < n && c < p ? src[(long long)(g * RB + r) * p + c] : make_double2(0, 0);
+  }
+}
+__device__ __forceinline__ void load_square(double2* s, const double2* src, int p) {
+  for (int e = threadIdx.x; e < PMAX * PMAX; e += 256) {
+    const int r = e >> 6, c = e & 63;
+    s[e] = r < p && c < p ? src[r * p + c] : make_double2(0, 0);
+  }
+}
+// o[i][j] = sum_k xs[ty + 16 i][k] q[k][tx + 16 j], i < RB / 16
+template <int RB>
+__device__ __forceinline__ void times_square(double2 (&o)[RB / 16][4], const double2* xs, const double2* q, int tx, int ty) {
+#pragma unroll
+  for (int i = 0; i < RB / 16; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[i][j] = make_double2(0, 0);
+#pragma unroll 4
+  for (int k = 0; k < PMAX; ++k) {
+    double2 b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = q[k * PMAX + tx + 16 * j];
+#pragma unroll
+    for (int i = 0; i < RB / 16; ++i) {
+      const double2 x = xs[(ty + 16 * i) * PMAX + k];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cfma(o[i][j], x, b[j]);
+    }
+  }
+}
+
+// X <- X Rinv in place (groups of RB rows), and, with gparts, the shares of the result's Gram matrix.
+template <int RB>
+__global__ void __launch_bounds__(256) scale_kernel(int n, int p, double2* X, const double2* Rinv, double2* gparts) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double2* q = (double2*)smem;            // [64][64]
+  double2* xs = q + PMAX * PMAX;          // [RB][64]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  pdl_trigger();
+  pdl_wait();
+  load_square(q, Rinv, p);
+  double2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
+  for (int g = blockIdx.x; g * RB < n; g += gridDim.x) {
+    load_group<RB>(xs, X, n, p, g);
+    __syncthreads();
+    double2 o[RB / 16][4];
+    times_square<RB>(o, xs, q, tx, ty);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RB / 16; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int r = ty + 16 * i, c = tx + 16 * j;
+        xs[r * PMAX + c] = o[i][j];
+        if (g * RB + r < n && c < p) X[(long long)(g * RB + r) * p + c] = o[i][j];
+      }
+    __syncthreads();
+    if (gparts) gram_rows<RB>(acc, xs, xs, tx, ty);
+    __syncthreads();
+  }
+  if (gparts) store_gram(acc, gparts, tx, ty);
+}
+
+// X <- X Q, Z <- Z Q in place, and the shares rparts[block][64] of sum_rows |Z - w X|^2 per column.
+template <int RB>
+__global__ void __launch_bounds__(256) ritz_kernel(int n, int p, double2* X, double2* Z, const double2* Q, const double* w,
+                                                   double* rparts) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double2* q = (double2*)smem;            // [64][64]
+  double2* xs = q + PMAX * PMAX;          // [RB][64]
+  double2* zs = xs + RB * PMAX;           // [RB][64]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  pdl_trigger();
+  pdl_wait();
+  load_square(q, Q, p);
+  double res[4] = {0, 0, 0, 0}, wc[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) wc[j] = tx + 16 * j < p ? w[tx + 16 * j] : 0.0;
+  for (int g = blockIdx.x; g * RB < n; g += gridDim.x) {
+    load_group<RB>(xs, X, n, p, g);
+    load_group<RB>(zs, Z, n, p, g);
+    __syncthreads();
+    double2 ox[RB / 16][4], oz[RB / 16][4];
+    times_square<RB>(ox, xs, q, tx, ty);
+    times_square<RB>(oz, zs, q, tx, ty);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RB / 16; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int r = g * RB + ty + 16 * i, c = tx + 16 * j;
+        if (r < n && c < p) {
+          X[(long long)r * p + c] = ox[i][j];
+          Z[(long long)r * p + c] = oz[i][j];
+        }
+        const double dx = oz[i][j].x - wc[j] * ox[i][j].x, dy = oz[i][j].y - wc[j] * ox[i][j].y;
+        res[j] += dx * dx + dy * dy;
+      }
+  }
+  double* rs = (double*)xs;   // [16][64]
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) rs[ty * PMAX + tx + 16 * j] = res[j];
+  __syncthreads();
+  if (tid < PMAX) {
+    double s = 0;
+    for (int i = 0; i < 16; ++i) s += rs[i * PMAX + tid];
+    rparts[blockIdx.x * PMAX + tid] = s;
+  }
+}
+
+// res[c] = sqrt(sum_b rparts[b][c]).
+__global__ void __launch_bounds__(1024) residual_kernel(const double* rparts, int nparts, int p, double* res) {
+  __shared__ double sh[16][PMAX];
+  const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
+  pdl_trigger();
+  pdl_wait();
+  double s = 0;
+  for (int b = q; b < nparts; b += 16) s += rparts[b * PMAX + c];
+  sh[q][c] = s;
+  __syncthreads();
+  if (q == 0 && c < p) {
+    for (int i = 1; i < 16; ++i) s += sh[i][c];
+    res[c] = sqrt(s);
+  }
 }
 
 // Deterministic start block: entries uniform in [-1, 1] + i [-1, 1] from a 64-bit mix of their index.
@@ -109,189 +486,151 @@ __global__ void start_block_kernel(double2* X, long long count, unsigned long lo
   X[e] = make_double2((double)(a >> 11) * 0x1.0p-52 - 1.0, (double)(b >> 11) * 0x1.0p-52 - 1.0);
 }
 
-// One CTA: G (p x p Hermitian, row-major) = R^H R with R upper triangular (Cholesky, after adding
-// shift_rel * max_j G_jj to the diagonal against rank deficiency), then Rinv = R^-1.
-constexpr size_t CHOL_SMEM = sizeof(double2) * PMAX * (PMAX + 1) + 16;
-__global__ void __launch_bounds__(256) chol_inv_kernel(int p, const double2* __restrict__ Gin, double2* Rinv,
-                                                       double shift_rel) {
+// One CTA: eigendecomposition of a Hermitian p x p matrix (p <= 64; worked on as 64 x 64, zero beyond p) by cyclic
+// Jacobi sweeps in the round-robin order (32 disjoint rotations per step).  w: eigenvalues descending; Q: row-major,
+// column i the eigenvector of w[i].
+// A step is two phases of FP64 work on one SM: the two-sided update of A, one 2 x 2 block J_k^H A J_l per thread for
+// the 528 pairs (k, l) of one triangle (its mirror block is stored with it), and the update of V, during which one
+// warp derives the next step's rotations (algebraically, from square roots and divisions).  Pairs are dealt as
+// (k, k + d mod 32): neighbouring lanes touch neighbouring rows and columns, which with a row of 64 values falls on
+// different banks.  Sweeps end when the off-diagonal part is at rounding level, or below 1e-12 and no longer falling.
+// 64 x 64: JAC_US us a sweep, 2 to 7 sweeps; with separate column and row updates of the full matrix, trigonometric
+// rotations and serial bookkeeping by one thread a decomposition took 2.8 ms.
+struct Rot { double cs, sn, ex, ey; };
+constexpr int JN = PMAX, JH = PMAX / 2;
+constexpr size_t JACOBI_SMEM = 2 * sizeof(double2) * JN * JN;
+__global__ void __launch_bounds__(1024, 1) heev_jacobi_kernel(int p, const double2* Hin, double* w, double2* Q, int max_sweeps) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 (*G)[PMAX + 1] = (double2 (*)[PMAX + 1])smem_raw;
-  double& dmax = *(double*)(smem_raw + sizeof(double2) * PMAX * (PMAX + 1));
-  const int t = threadIdx.x;
-  for (int e = t; e < p * p; e += 256) G[e / p][e % p] = Gin[e];
-  __syncthreads();
-  if (t == 0) {
-    double m = 0;
-    for (int j = 0; j < p; ++j) m = fmax(m, G[j][j].x);
-    dmax = m;
+  double2* A = (double2*)smem_raw;
+  double2* V = A + JN * JN;
+  __shared__ Rot R[2][JH];
+  __shared__ int place[JN];
+  __shared__ double red[2][32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  pdl_trigger();
+  pdl_wait();
+  for (int e = t; e < JN * JN; e += 1024) {
+    const int r = e / JN, c = e % JN;
+    const bool in = r < p && c < p;
+    const double2 u = in ? Hin[r * p + c] : make_double2(0, 0), v = in ? Hin[c * p + r] : make_double2(0, 0);
+    A[e] = make_double2(0.5 * (u.x + v.x), 0.5 * (u.y - v.y));
+    V[e] = make_double2(r == c ? 1.0 : 0.0, 0.0);
   }
   __syncthreads();
-  if (t < p) G[t][t].x += shift_rel * dmax;
-  __syncthreads();
-  for (int j = 0; j < p; ++j) {   // row j of R overwrites row j of G (upper part)
-    if (t == 0) {
-      const double d = G[j][j].x;
-      G[j][j] = make_double2(sqrt(d > 1e-300 ? d : 1e-300), 0.0);
+  // the value in slot s at a step of the round robin: slot 0 stays, the others move one slot a step; pair k: slots k
+  // and 63 - k
+  auto elem = [](int s, int step) {
+    const int q = s - 1 - step;
+    return s == 0 ? 0 : 1 + (q < 0 ? q + JN - 1 : q);
+  };
+  auto rotate = [&](int k, int step, int buf) {
+    const int i = elem(k, step), j = elem(JN - 1 - k, step);
+    const double a = A[i * JN + i].x, b = A[j * JN + j].x;
+    const double2 c = A[i * JN + j];
+    const double g2 = c.x * c.x + c.y * c.y;
+    Rot r = {1.0, 0.0, 1.0, 0.0};
+    if (g2 > 1e-290) {   // (a smaller value is set to zero with its block)
+      const double rg = rsqrt(g2), tau = 0.5 * (a - b) * rg;
+      const double tn = copysign(1.0 / (fabs(tau) + sqrt(1.0 + tau * tau)), tau);
+      r.cs = rsqrt(1.0 + tn * tn);
+      r.sn = tn * r.cs;
+      r.ex = c.x * rg;
+      r.ey = -c.y * rg;   // conj(e^{i phi})
     }
-    __syncthreads();
-    const double r = G[j][j].x;
-    for (int c = j + 1 + t; c < p; c += 256) G[j][c] = make_double2(G[j][c].x / r, G[j][c].y / r);
-    __syncthreads();
-    const int w = p - j - 1;
-    for (int e = t; e < w * w; e += 256) {   // trailing update G[a][b] -= conj(R[j][a]) R[j][b], a <= b
-      const int a = j + 1 + e / w, b = j + 1 + e % w;
-      if (a <= b) {
-        const double2 ra = G[j][a], rb = G[j][b];
-        G[a][b].x -= ra.x * rb.x + ra.y * rb.y;
-        G[a][b].y -= ra.x * rb.y - ra.y * rb.x;
-      }
-    }
-    __syncthreads();
-  }
-  // Rinv: column c by back substitution, R Rinv[:, c] = e_c (upper triangular)
-  if (t < p) {
-    const int c = t;
-    double2 x[PMAX];
-    for (int i = p - 1; i >= 0; --i) {
-      double2 s = make_double2(i == c ? 1.0 : 0.0, 0.0);
-      if (i <= c) {
-        for (int l = i + 1; l <= c; ++l) {
-          const double2 rl = G[i][l];
-          s.x -= rl.x * x[l].x - rl.y * x[l].y;
-          s.y -= rl.x * x[l].y + rl.y * x[l].x;
-        }
-        const double r = G[i][i].x;
-        x[i] = make_double2(s.x / r, s.y / r);
-      } else {
-        x[i] = make_double2(0.0, 0.0);
-      }
-    }
-    for (int i = 0; i < p; ++i) Rinv[(long long)i * p + c] = x[i];
-  }
-}
-
-// One CTA: eigendecomposition of a Hermitian p x p matrix (p even, <= 64) by cyclic Jacobi sweeps in the
-// round-robin order (p/2 disjoint rotations per step).  w: eigenvalues descending; Q: row-major, column i the
-// eigenvector of w[i].
-constexpr size_t JACOBI_SMEM = 2 * sizeof(double2) * PMAX * (PMAX + 1);
-__global__ void __launch_bounds__(256) heev_jacobi_kernel(int p, const double2* __restrict__ Hin, double* w,
-                                                          double2* Q, int max_sweeps) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 (*A)[PMAX + 1] = (double2 (*)[PMAX + 1])smem_raw;
-  double2 (*V)[PMAX + 1] = (double2 (*)[PMAX + 1])(smem_raw + sizeof(double2) * PMAX * (PMAX + 1));
-  __shared__ double2 J[PMAX / 2][4];
-  __shared__ int pi[PMAX / 2], pj[PMAX / 2], order[PMAX], perm[PMAX];
-  __shared__ double off, tot;
-  const int t = threadIdx.x, h = p / 2;
-  for (int e = t; e < p * p; e += 256) {
-    const int r = e / p, c = e % p;
-    A[r][c] = Hin[e];
-    V[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
-  }
-  if (t < p) order[t] = t;
-  __syncthreads();
+    R[buf][k] = r;
+  };
+  if (warp == 0) rotate(t, 0, 0);
+  int buf = 0;
+  double last = 0;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-    if (t == 0) {
-      double o = 0, a = 0;
-      for (int r = 0; r < p; ++r)
-        for (int c = 0; c < p; ++c) {
-          const double v = A[r][c].x * A[r][c].x + A[r][c].y * A[r][c].y;
-          a += v;
-          if (r != c) o += v;
-        }
-      off = o;
-      tot = a;
+    double o = 0, d = 0;
+    for (int e = t; e < JN * JN; e += 1024) {
+      const double2 x = A[e];
+      const double v = x.x * x.x + x.y * x.y;
+      if (e / JN == e % JN) d += v; else o += v;
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      o += __shfl_xor_sync(0xffffffffu, o, s);
+      d += __shfl_xor_sync(0xffffffffu, d, s);
+    }
+    if (lane == 0) {
+      red[0][warp] = o;
+      red[1][warp] = d;
     }
     __syncthreads();
-    if (!(off > 1e-30 * tot)) break;
-    for (int step = 0; step < p - 1; ++step) {
-      if (t < h) {   // pair t of this step and its rotation (from the matrix before the step)
-        int i = order[t], j = order[p - 1 - t];
-        if (i > j) {
-          const int s = i;
-          i = j;
-          j = s;
+    o = 0;
+    d = 0;
+    for (int i = 0; i < 32; ++i) {   // the same sums in the same order in every thread
+      o += red[0][i];
+      d += red[1][i];
+    }
+    if (!(o > 1e-30 * (o + d)) || (sweep > 0 && o < 1e-24 * (o + d) && o > 0.25 * last)) break;
+    last = o;
+#pragma unroll 1
+    for (int step = 0; step < JN - 1; ++step, buf ^= 1) {
+      if (t < JH * (JH + 1) / 2) {
+        const int dd = t / JH, k = t % JH, l = (k + dd) % JH;
+        const Rot rk = R[buf][k], rl = R[buf][l];
+        const int ik = elem(k, step), jk = elem(JN - 1 - k, step), il = elem(l, step), jl = elem(JN - 1 - l, step);
+        double2 m[2][2] = {{A[ik * JN + il], A[ik * JN + jl]}, {A[jk * JN + il], A[jk * JN + jl]}};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {   // columns by J_l
+          const double2 a = m[u][0], b = cmul(m[u][1], make_double2(rl.ex, rl.ey));
+          m[u][0] = make_double2(rl.cs * a.x + rl.sn * b.x, rl.cs * a.y + rl.sn * b.y);
+          m[u][1] = make_double2(rl.cs * b.x - rl.sn * a.x, rl.cs * b.y - rl.sn * a.y);
         }
-        pi[t] = i;
-        pj[t] = j;
-        const double a = A[i][i].x, b = A[j][j].x;
-        const double2 c = A[i][j];
-        const double g = sqrt(c.x * c.x + c.y * c.y);
-        double2 j00 = make_double2(1, 0), j01 = make_double2(0, 0), j10 = make_double2(0, 0), j11 = make_double2(1, 0);
-        if (g > 0) {
-          const double ex = c.x / g, ey = -c.y / g;   // conj(e^{i phi})
-          const double th = 0.5 * atan2(2 * g, a - b), cs = cos(th), sn = sin(th);
-          j00 = make_double2(cs, 0);
-          j01 = make_double2(-sn, 0);
-          j10 = make_double2(ex * sn, ey * sn);
-          j11 = make_double2(ex * cs, ey * cs);
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {   // rows by J_k^H
+          const double2 a = m[0][v], b = cmul(m[1][v], make_double2(rk.ex, -rk.ey));
+          m[0][v] = make_double2(rk.cs * a.x + rk.sn * b.x, rk.cs * a.y + rk.sn * b.y);
+          m[1][v] = make_double2(rk.cs * b.x - rk.sn * a.x, rk.cs * b.y - rk.sn * a.y);
         }
-        J[t][0] = j00;
-        J[t][1] = j01;
-        J[t][2] = j10;
-        J[t][3] = j11;
+        if (dd == 0) {
+          A[ik * JN + ik] = make_double2(m[0][0].x, 0.0);
+          A[jk * JN + jk] = make_double2(m[1][1].x, 0.0);
+          A[ik * JN + jk] = A[jk * JN + ik] = make_double2(0.0, 0.0);
+        } else {
+          A[ik * JN + il] = m[0][0];
+          A[ik * JN + jl] = m[0][1];
+          A[jk * JN + il] = m[1][0];
+          A[jk * JN + jl] = m[1][1];
+          A[il * JN + ik] = conjd(m[0][0]);
+          A[jl * JN + ik] = conjd(m[0][1]);
+          A[il * JN + jk] = conjd(m[1][0]);
+          A[jl * JN + jk] = conjd(m[1][1]);
+        }
       }
       __syncthreads();
-      for (int e = t; e < p * h; e += 256) {   // columns: A <- A J, V <- V J
-        const int r = e / h, k = e % h, i = pi[k], j = pj[k];
-        const double2 j00 = J[k][0], j01 = J[k][1], j10 = J[k][2], j11 = J[k][3];
-        const double2 ai = A[r][i], aj = A[r][j], vi = V[r][i], vj = V[r][j];
-        A[r][i] = cadd(cmul(ai, j00), cmul(aj, j10));
-        A[r][j] = cadd(cmul(ai, j01), cmul(aj, j11));
-        V[r][i] = cadd(cmul(vi, j00), cmul(vj, j10));
-        V[r][j] = cadd(cmul(vi, j01), cmul(vj, j11));
-      }
-      __syncthreads();
-      for (int e = t; e < p * h; e += 256) {   // rows: A <- J^H A
-        const int c = e / h, k = e % h, i = pi[k], j = pj[k];
-        const double2 j00 = conjd(J[k][0]), j01 = conjd(J[k][1]), j10 = conjd(J[k][2]), j11 = conjd(J[k][3]);
-        const double2 ai = A[i][c], aj = A[j][c];
-        A[i][c] = cadd(cmul(j00, ai), cmul(j10, aj));
-        A[j][c] = cadd(cmul(j01, ai), cmul(j11, aj));
-      }
-      __syncthreads();
-      if (t == 0) {   // next round-robin order: keep order[0], rotate the rest
-        const int last = order[p - 1];
-        for (int s = p - 1; s > 1; --s) order[s] = order[s - 1];
-        order[1] = last;
+      if (warp == 0) {
+        rotate(t, step + 1 < JN - 1 ? step + 1 : 0, buf ^ 1);
+      } else {
+        const int i = elem(lane, step), j = elem(JN - 1 - lane, step);
+        const Rot q = R[buf][lane];
+        for (int r = warp - 1; r < JN; r += 31) {   // V <- V J
+          const double2 a = V[r * JN + i], b = cmul(V[r * JN + j], make_double2(q.ex, q.ey));
+          V[r * JN + i] = make_double2(q.cs * a.x + q.sn * b.x, q.cs * a.y + q.sn * b.y);
+          V[r * JN + j] = make_double2(q.cs * b.x - q.sn * a.x, q.cs * b.y - q.sn * a.y);
+        }
       }
       __syncthreads();
     }
   }
-  if (t == 0) {   // eigenvalues descending
-    for (int i = 0; i < p; ++i) perm[i] = i;
+  __syncthreads();
+  if (t < p) {   // eigenvalues descending: each value's place by counting (where one is NaN they keep their order)
+    const double x = A[t * JN + t].x;
+    bool bad = false;
+    int at = 0;
     for (int i = 0; i < p; ++i) {
-      int best = i;
-      for (int k = i + 1; k < p; ++k)
-        if (A[perm[k]][perm[k]].x > A[perm[best]][perm[best]].x) best = k;
-      const int s = perm[i];
-      perm[i] = perm[best];
-      perm[best] = s;
+      const double y = A[i * JN + i].x;
+      bad |= isnan(y);
+      at += y > x || (y == x && i < t);
     }
+    place[t] = bad ? t : at;
+    w[place[t]] = x;
   }
   __syncthreads();
-  if (t < p) w[t] = A[perm[t]][perm[t]].x;
-  for (int e = t; e < p * p; e += 256) Q[e] = V[e / p][perm[e % p]];
-}
-
-// res[j] = || Z[:, j] - w[j] X[:, j] ||, j < k (block per column).
-__global__ void residual_kernel(int n, int p, const double2* __restrict__ Z, const double2* __restrict__ X,
-                                const double* __restrict__ w, double* res) {
-  __shared__ double part[256];
-  const int j = blockIdx.x;
-  double s = 0;
-  for (int i = threadIdx.x; i < n; i += 256) {
-    const double2 z = Z[(long long)i * p + j], x = X[(long long)i * p + j];
-    const double dx = z.x - w[j] * x.x, dy = z.y - w[j] * x.y;
-    s += dx * dx + dy * dy;
-  }
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) res[j] = sqrt(part[0]);
+  for (int e = t; e < p * p; e += 1024) Q[(e / p) * p + place[e % p]] = V[(e / p) * JN + e % p];
 }
 
 // Output: vecs [n][k] = columns 0..k-1 of XQ (row-major n x p), vals[i] = max(w[i], 0).
@@ -303,40 +642,96 @@ __global__ void output_kernel(int n, int p, int k, const double2* __restrict__ X
 }
 
 // ------------------------------------------------------------------------------------------- host side
+constexpr int SMS = 148, GRAM_BLOCKS = 2 * SMS;
+
+// Shares of the K loop for `tiles` output tiles and `chunks` chunks of K: four blocks per SM (two are resident; tiles
+// differ in their non-zero blocks, and smaller shares even that out), at least four chunks each, at most 32 shares.
+static int shares(int tiles, int chunks) {
+  const int s = std::max(1, 4 * SMS / tiles);
+  return std::max(1, std::min(std::min(s, 32), chunks / 4));
+}
+
+struct Sizes {
+  long long np, pp, parts, flags;
+  int ne, s_;
+  Sizes(int n, int p, int ne_, int s) : ne(ne_), s_(s) {
+    np = (long long)n * p;
+    pp = (long long)p * p;
+    const int tn = ceil_div(n, zg::T);
+    if (ne > 0) {
+      const int ts = ceil_div(s, zg::T);
+      const long long back = (long long)shares(ts * ne, ceil_div(n, zg::KC)) * ne * s * p;
+      parts = std::max(back, shares(tn, ne * ceil_div(s, zg::KC)) * np);
+      flags = (long long)ne * zg::flag_dim(n) * zg::flag_dim(s);
+    } else {
+      parts = shares(tn, ceil_div(n, zg::KC)) * np;
+      flags = (long long)zg::flag_dim(n) * zg::flag_dim(n);
+    }
+    flags = (flags + 15) / 16 * 16;
+  }
+  long long wf() const { return (long long)ne * s_ * PMAX; }
+  long long complex_values() const { return 2 * np + wf() + 3 * pp + parts + (long long)GRAM_BLOCKS * PMAX * PMAX; }
+  long long bytes(int p) const { return 16 * complex_values() + 8 * ((long long)GRAM_BLOCKS * PMAX + 3 * p) + flags + 256; }
+};
+
 struct Solver {
   cudaStream_t s;
-  double2* parts;
-  long long parts_count;
+  int n, p, ne, seg;           // T: dense (ne = 0, seg = n) or ne pupil matrices [n][seg]
+  const double2* M;
+  const unsigned char* flags;
+  double2 *Wf, *parts, *gparts, *G, *Rinv;
+  double* rdiag;
   int status = OI_OK;
 
-  // C = op(A) B (+ C), split over K when the output has few tiles.
-  void gemm(bool ah, int m, int n, int k, const double2* A, long long lda, const double2* B, long long ldb, double2* C,
-            long long ldc, bool acc) {
-    if (status) return;
-    const int tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-    int splits = 1;
-    while (tiles * splits < 256 && k / (splits * 2) >= 4 * BK && (long long)(splits * 2) * m * n <= parts_count)
-      splits *= 2;
-    const int kchunk = ((k + splits - 1) / splits + BK - 1) / BK * BK;
-    splits = (k + kchunk - 1) / kchunk;
-    dim3 grid((unsigned)((n + BN - 1) / BN), (unsigned)((m + BM - 1) / BM), (unsigned)splits);
-    double2* out = splits > 1 ? parts : C;
-    const long long ldo = splits > 1 ? n : ldc;
-    if (ah)
-      zgemm_kernel<true><<<grid, 256, 0, s>>>(m, n, k, A, lda, B, ldb, out, ldo, kchunk, splits > 1 ? 0 : acc);
+  template <typename... KArgs, typename... Args>
+  void run(const char* what, void (*kern)(KArgs...), dim3 grid, int block, size_t smem, Args... args) {
+    if (status || (smem > 48 * 1024 && (status = ensure_smem((const void*)kern, smem, what)))) return;
+    (void)launch_pdl(kern, grid, dim3(block), smem, s, args...);
+    note_launch();
+    status = check_launch(what);
+  }
+  bool fine() const { return n <= 16 * SMS; }   // 16-row groups fill the SMs better; 32-row ones reuse more
+  int groups() const { return std::min(GRAM_BLOCKS, ceil_div(n, fine() ? 16 : 32)); }
+
+  void fold(const FoldArgs& f, int batch = 1) {
+    const int blocks = f.gparts ? groups() : ceil_div(f.n, 16);
+    const size_t row = sizeof(double2) * PMAX * (f.left ? 2 : 1);
+    if (!f.gparts || fine())
+      run("oi_eig_topk64/fold", fold_kernel<16>, dim3(blocks, batch), 256, 16 * row, f);
     else
-      zgemm_kernel<false><<<grid, 256, 0, s>>>(m, n, k, A, lda, B, ldb, out, ldo, kchunk, splits > 1 ? 0 : acc);
-    oi::note_launch();
-    if ((status = check_launch("oi_eig_topk64/gemm"))) return;
-    if (splits > 1) {
-      if (ldc != n) {
-        status = fail(OI_EINVAL, "oi_eig_topk64: split GEMM into a strided output");
-        return;
-      }
-      const long long cnt = (long long)m * n;
-      reduce_parts_kernel<<<(unsigned)ceil_div(cnt, 256), 256, 0, s>>>(parts, splits, cnt, C, acc ? 1 : 0);
-      oi::note_launch();
-      status = check_launch("oi_eig_topk64/reduce");
+      run("oi_eig_topk64/fold", fold_kernel<32>, dim3(blocks, batch), 256, 32 * row, f);
+  }
+  // out = alpha T in + beta b1 + gamma b0; gram: the shares of left^H out (left null: out^H out) into gparts.
+  void apply(const double2* in, double2* out, double alpha, double beta, const double2* b1, double gamma,
+             const double2* b0, bool gram, const double2* left) {
+    const double2* B = in;
+    const int tn = ceil_div(n, zg::T);
+    if (ne > 0) {
+      const int ts = ceil_div(seg, zg::T), sh = shares(ts * ne, ceil_div(n, zg::KC));
+      GemmArgs g{M, (long long)n * seg, seg, n, 1, p, in, parts, flags, zg::flag_dim(n), zg::flag_dim(seg)};
+      run("oi_eig_topk64/gemm", gemm_kernel<true>, dim3(ts, sh, ne), 256, zg::SMEM, g);   // Wf_e = h_e^H in
+      fold(FoldArgs{parts, sh, seg, p, 1.0, 0.0, 0.0, nullptr, nullptr, nullptr, Wf, nullptr}, ne);
+      B = Wf;
+    }
+    const int nseg = ne > 0 ? ne : 1, sh = shares(tn, nseg * ceil_div(seg, zg::KC));
+    GemmArgs g{M, (long long)n * seg, n, seg, nseg, p, B, parts, flags, zg::flag_dim(n), zg::flag_dim(seg)};
+    run("oi_eig_topk64/gemm", gemm_kernel<false>, dim3(tn, sh, 1), 256, zg::SMEM, g);
+    fold(FoldArgs{parts, sh, n, p, alpha, beta, gamma, b1, b0, left, out, gram ? gparts : nullptr});
+  }
+  void sum_gram() { run("oi_eig_topk64/gram", sum_gram_kernel, dim3(p), 256, 0, (const double2*)gparts, groups(), p, G); }
+  // X <- CholQR2(X); the Gram shares of X are in gparts.
+  void orth(double2* X) {
+    for (int pass = 0; pass < 2; ++pass) {
+      sum_gram();
+      run("oi_eig_topk64/chol", chol_inv_kernel, dim3(1), 512, 0, p, (const double2*)G, Rinv, rdiag,
+          pass == 0 ? 1e-13 : 1e-15, pass == 0);
+      double2* gp = pass == 0 ? gparts : nullptr;
+      if (fine())
+        run("oi_eig_topk64/scale", scale_kernel<16>, dim3(groups()), 256, sizeof(double2) * PMAX * (PMAX + 16), n, p, X,
+            (const double2*)Rinv, gp);
+      else
+        run("oi_eig_topk64/scale", scale_kernel<32>, dim3(groups()), 256, sizeof(double2) * PMAX * (PMAX + 32), n, p, X,
+            (const double2*)Rinv, gp);
     }
   }
 };
@@ -347,9 +742,7 @@ struct Solver {
 extern "C" int oi_eig_topk64_workspace(int n, int p, int ne, int s, long long* bytes) {
   using namespace oi;
   if (!bytes || n <= 0 || p <= 0) return fail(OI_EINVAL, "oi_eig_topk64_workspace: bad arguments");
-  const long long np = (long long)n * p, pp = (long long)p * p, sp = ne > 0 ? (long long)s * p : 0;
-  const long long parts = 256LL * pp > 8 * np ? 256LL * pp : 8 * np;
-  *bytes = 16 * (3 * np + sp + 4 * pp + parts) + 8 * (2 * (long long)p) + 256;
+  *bytes = eg::Sizes(n, p, std::max(ne, 0), std::max(s, 0)).bytes(p);
   return OI_OK;
 }
 
@@ -364,99 +757,121 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
     return fail(OI_EINVAL, "oi_eig_topk64: bad arguments");
   if (p > PMAX || p % 2 || k > p || p > n)
     return fail(OI_ERANGE, "oi_eig_topk64: need k <= p <= min(n, %d), p even (k=%d p=%d n=%d)", PMAX, k, p, n);
-  long long need = 0;
-  oi_eig_topk64_workspace(n, p, dense ? 0 : ne, s, &need);
+  if (dense) ne = 0, s = n;
+  const Sizes sz(n, p, ne, s);
+  const long long need = sz.bytes(p);
   if (work_bytes < need) return fail(OI_ERANGE, "oi_eig_topk64: %lld workspace bytes given, %lld needed", work_bytes, need);
-  if (int rc = ensure_smem((const void*)chol_inv_kernel, CHOL_SMEM, "oi_eig_topk64")) return rc;
-  if (int rc = ensure_smem((const void*)heev_jacobi_kernel, JACOBI_SMEM, "oi_eig_topk64")) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  const long long np = (long long)n * p, pp = (long long)p * p;
   double2* X = (double2*)(((uintptr_t)work + 255) & ~(uintptr_t)255);
-  double2* Y = X + np;
-  double2* Z = Y + np;
-  double2* Wf = Z + np;                                // factored form: h_e^H X, [s][p]
-  double2* G = Wf + (dense ? 0 : (long long)s * p);
-  double2* Rinv = G + pp;
-  double2* Q = Rinv + pp;
-  double2* Hm = Q + pp;
-  double2* parts = Hm + pp;
-  const long long parts_count = 256LL * pp > 8 * np ? 256LL * pp : 8 * np;
-  double* w = (double*)(parts + parts_count);
+  double2* Z = X + sz.np;
+  double2* Wf = Z + sz.np;
+  double2* G = Wf + sz.wf();
+  double2* Rinv = G + sz.pp;
+  double2* Q = Rinv + sz.pp;
+  double2* parts = Q + sz.pp;
+  double2* gparts = parts + sz.parts;
+  double* rparts = (double*)(gparts + (long long)GRAM_BLOCKS * PMAX * PMAX);
+  double* w = rparts + (long long)GRAM_BLOCKS * PMAX;   // [p], then the residuals [p] and the diagonal of R [p]
   double* res = w + p;
-  Solver sv{st, parts, parts_count};
-  const double2* T = (const double2*)tcc;
-  const double2* hh = (const double2*)h;
+  double* rdiag = res + p;
+  unsigned char* flags = (unsigned char*)(rdiag + p);
+  const double2* M = (const double2*)(dense ? tcc : h);
+  if (int rc = zg::mark_blocks(M, dense ? 1 : ne, n, s, flags, st)) return rc;
+  Solver sv{st, n, p, ne, s, M, flags, Wf, parts, gparts, G, Rinv, rdiag};
 
-  auto apply = [&](const double2* in, double2* out) {   // out = T in
-    if (dense) {
-      sv.gemm(false, n, p, n, T, n, in, p, out, p, false);
-    } else {
-      for (int e = 0; e < ne; ++e) {
-        const double2* he = hh + (long long)e * n * s;
-        sv.gemm(true, s, p, n, he, s, in, p, Wf, p, false);   // h_e^H in
-        sv.gemm(false, n, p, s, he, s, Wf, p, out, p, e > 0);  // out (+)= h_e (h_e^H in)
-      }
-    }
-  };
-  auto orth = [&](const double2* in, double2* out) {   // out = CholQR2(in), through Z (in and out distinct)
-    for (int pass = 0; pass < 2 && !sv.status; ++pass) {
-      const double2* src = pass == 0 ? in : Z;
-      double2* dst = pass == 0 ? Z : out;
-      sv.gemm(true, p, p, n, src, p, src, p, G, p, false);   // Gram matrix
-      if (sv.status) return;
-      chol_inv_kernel<<<1, 256, CHOL_SMEM, st>>>(p, G, Rinv, pass == 0 ? 1e-13 : 1e-15);
-      oi::note_launch();
-      if ((sv.status = check_launch("oi_eig_topk64/chol"))) return;
-      sv.gemm(false, n, p, p, src, p, Rinv, p, dst, p, false);
-    }
-  };
-
-  start_block_kernel<<<(unsigned)ceil_div(np, 256), 256, 0, st>>>(Y, np, 0x5eed0f71ull + (unsigned long long)n);
-  oi::note_launch();
+  start_block_kernel<<<(unsigned)ceil_div(sz.np, 256), 256, 0, st>>>(Z, sz.np, 0x5eed0f71ull + (unsigned long long)n);
+  note_launch();
   if (int rc = check_launch("oi_eig_topk64/start")) return rc;
-  orth(Y, X);
-  int it = 0;
+  int it = 0, stalls = 0;   // products with T so far (a projection's own is not counted)
+  double last = -1;
   bool converged = false;
-  std::vector<double> hres(k), hw(p);
-  const int check = 4;
-  while (!sv.status && it < max_iter) {
-    apply(X, Y);
-    orth(Y, X);
-    ++it;
-    if (it % check == 0 || it == max_iter) {
-      apply(X, Z);                                                    // Rayleigh-Ritz
-      sv.gemm(true, p, p, n, X, p, Z, p, Hm, p, false);
-      if (sv.status) break;
-      heev_jacobi_kernel<<<1, 256, JACOBI_SMEM, st>>>(p, Hm, w, Q, 40);
-      oi::note_launch();
-      if ((sv.status = check_launch("oi_eig_topk64/jacobi"))) break;
-      sv.gemm(false, n, p, p, X, p, Q, p, Y, p, false);               // Y = X Q (Ritz vectors)
-      sv.gemm(false, n, p, p, Z, p, Q, p, X, p, false);               // X = Z Q = T X Q
-      if (sv.status) break;
-      residual_kernel<<<(unsigned)k, 256, 0, st>>>(n, p, X, Y, w, res);
-      oi::note_launch();
-      if ((sv.status = check_launch("oi_eig_topk64/residual"))) break;
-      if (cudaMemcpyAsync(hres.data(), res, 8 * k, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaMemcpyAsync(hw.data(), w, 8 * p, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess) {
-        sv.status = fail(OI_ECUDA, "oi_eig_topk64: %s", cudaGetErrorString(cudaGetLastError()));
-        break;
-      }
-      double worst = 0;
-      for (int i = 0; i < k; ++i) worst = std::fmax(worst, hres[i]);
-      const double scale = std::fabs(hw[0]) > 0 ? std::fabs(hw[0]) : 1.0;
-      cudaMemcpyAsync(X, Y, 16 * np, cudaMemcpyDeviceToDevice, st);   // continue from the Ritz vectors
-      if (worst <= tol * scale) {
-        converged = true;
-        break;
-      }
+  std::vector<double> host(2 * (size_t)p);
+  auto fetch = [&](const double* src, size_t count) {
+    if (!sv.status && (cudaMemcpyAsync(host.data(), src, 8 * count, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                       cudaStreamSynchronize(st) != cudaSuccess))
+      sv.status = fail(OI_ECUDA, "oi_eig_topk64: %s", cudaGetErrorString(cudaGetLastError()));
+    return sv.status == OI_OK;
+  };
+  auto plain = [&](int count) {   // X = CholQR2(T X)
+    for (int i = 0; i < count && it < max_iter; ++i, ++it) {
+      sv.apply(X, X, 1.0, 0.0, nullptr, 0.0, nullptr, true, nullptr);
+      sv.orth(X);
     }
+  };
+  // X = CholQR2(f(T) X) with f small on [0, b], for values w0 >= wk wanted and the residual `worst` (over w0)
+  auto filter = [&](double w0, double wk, double b, double worst) {
+    const double x = 2 * wk / b - 1, x0 = 2 * w0 / b - 1;
+    if (!(x > 1.05)) return plain(4);
+    const double rho = x + std::sqrt(x * x - 1), rho0 = x0 + std::sqrt(x0 * x0 - 1);
+    const double want = std::ceil(std::log(100.0 * worst / tol) / std::log(rho));
+    int total = (int)std::max(1.0, std::min((double)std::min(EIG_DEGREE, max_iter - it), want));
+    const double piece = std::log(EIG_AMP) / std::max(std::log(rho0 / rho), 1e-9);
+    const int degree = (int)std::max(1.0, std::min((double)total, piece));
+    const double c = 0.5 * b, e = 0.5 * b;
+    while (total > 0 && !sv.status) {
+      const int d = std::min(degree, total);
+      total -= d;
+      it += d;
+      // Y_j = T_j((T - c) / e) X / T_j((w0 - c) / e) by the scaled three-term recurrence, Y_0 in X, Y_1 in Z
+      const double s1 = e / (w0 - c);
+      sv.apply(X, Z, s1 / e, -c * s1 / e, X, 0.0, nullptr, d == 1, nullptr);
+      double sig = s1;
+      for (int j = 2; j <= d; ++j) {
+        const double s2 = 1.0 / (2.0 / s1 - sig);
+        sv.apply(Z, X, 2 * s2 / e, -2 * s2 * c / e, Z, -sig * s2, X, j == d, nullptr);
+        sig = s2;
+        std::swap(X, Z);
+      }
+      std::swap(X, Z);   // the newest is in X
+      sv.orth(X);
+    }
+  };
+
+  std::swap(X, Z);   // the random block is the first X
+  plain(EIG_START);
+  if (it < max_iter && fetch(rdiag, p)) {
+    for (int i = 0; i < p; ++i)
+      if (!(host[i] > 0)) host[i] = 0;
+    std::sort(host.begin(), host.begin() + p, [](double a, double b) { return a > b; });
+    const double w0 = host[0], wk = host[k - 1], wp = host[p - 1];
+    // the error left after the plain iterations; a TCC that is not a number, or of a rank below k, goes on to the
+    // projection as it is
+    if (w0 > 0 && wk > 1e-8 * w0)
+      filter(w0, wk, std::max(1.05 * wp, 1e-8 * w0), std::min(1.0, std::pow(wp / wk, EIG_START)) * wk / w0);
+  }
+  while (!sv.status) {
+    // Rayleigh-Ritz: Z = T X, H = X^H Z
+    sv.apply(X, Z, 1.0, 0.0, nullptr, 0.0, nullptr, true, X);
+    sv.sum_gram();
+    sv.run("oi_eig_topk64/jacobi", heev_jacobi_kernel, dim3(1), 1024, JACOBI_SMEM, p, (const double2*)G, w, Q, 40);
+    if (sv.fine())
+      sv.run("oi_eig_topk64/ritz", ritz_kernel<16>, dim3(sv.groups()), 256, sizeof(double2) * PMAX * (PMAX + 32), n, p, X, Z,
+             (const double2*)Q, (const double*)w, rparts);
+    else
+      sv.run("oi_eig_topk64/ritz", ritz_kernel<32>, dim3(sv.groups()), 256, sizeof(double2) * PMAX * (PMAX + 64), n, p, X, Z,
+             (const double2*)Q, (const double*)w, rparts);
+    sv.run("oi_eig_topk64/residual", residual_kernel, dim3(1), 1024, 0, (const double*)rparts, sv.groups(), p, res);
+    if (!fetch(w, 2 * (size_t)p)) break;
+    double worst = 0;   // (fmax passes NaN by: a TCC that is not a number ends here, with NaN pairs)
+    for (int i = 0; i < k; ++i) worst = std::fmax(worst, host[p + i]);
+    const double w0 = std::fabs(host[0]) > 0 ? std::fabs(host[0]) : 1.0;
+    if (worst <= tol * w0) {
+      converged = true;
+      break;
+    }
+    if (it >= max_iter) break;
+    if (last >= 0 && worst > 0.25 * last) ++stalls;
+    last = worst;
+    if (stalls)
+      plain(4);
+    else
+      filter(w0, host[k - 1], std::max(1.05 * host[p - 1], 1e-8 * w0), worst / w0);
   }
   if (sv.status) return sv.status;
   if (iters) *iters = converged ? it : -it;
   // X holds the Ritz vectors (columns by descending w)
   output_kernel<<<(unsigned)ceil_div((long long)n * k > p ? (long long)n * k : p, 256), 256, 0, st>>>(
       n, p, k, X, w, (double2*)vecs, vals);
-  oi::note_launch();
+  note_launch();
   return check_launch("oi_eig_topk64/output");
 }
