@@ -353,13 +353,13 @@ OI_API int oi_tcc_pupils64_pol(const float* ff, int lf, const float* gg, int lg,
 
 /*
  * The k leading eigenpairs of the TCC in FP64 (DecomposeTCC_SOCS.py:7-9, where the reference runs a full
- * torch.svd of its complex64 TCC): block subspace iteration on p vectors with Cholesky-QR orthonormalisation and
- * Rayleigh-Ritz every 4 iterations (one-CTA Jacobi on the p x p projection), until the leading k residuals
- * ||T u - lambda u|| are below tol * lambda_0 or max_iter iterations have run.  The TCC is given densely (tcc:
+ * torch.svd of its complex64 TCC): Chebyshev-filtered subspace iteration on p vectors with Cholesky-QR
+ * orthonormalisation and Rayleigh-Ritz (one-CTA Jacobi on the p x p projection), until the leading k residuals
+ * ||T u - lambda u|| are below tol * lambda_0 or max_iter products with T (besides the projections') have run.  The TCC is given densely (tcc:
  * complex128 [n][n], h NULL) or as its pupil factor (h: complex128 [ne][n][s] with TCC = sum_e h_e h_e^H,
  * tcc NULL; the TCC is not formed).  k <= p <= min(n, 64), p even.  Output: vecs complex128 [n][k] (row-major,
  * column i the eigenvector of vals[i]), vals double [k] descending, clamped at zero (device pointers); *iters
- * (host) the iterations run, negative when tol was not reached.  work: oi_eig_topk64_workspace bytes.  Unlike
+ * (host) the products run, negative when tol was not reached.  work: oi_eig_topk64_workspace bytes.  Unlike
  * the imaging entry points this one synchronises its stream (it reads the residuals to decide when to stop).
  */
 OI_API int oi_eig_topk64_workspace(int n, int p, int ne, int s, long long* bytes);

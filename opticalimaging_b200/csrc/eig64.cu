@@ -100,15 +100,12 @@ __global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   pdl_trigger();
   pdl_wait();
-  const int mt = heavy_first(blockIdx.x, gridDim.x), m0 = mt * zg::T, splits = gridDim.y, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int mt = heavy_first(blockIdx.x, gridDim.x), m0 = mt * zg::T, splits = gridDim.y;
   const int per = (a.k + zg::KC - 1) / zg::KC;
   const double2* M = a.M + (AH ? blockIdx.z * a.sm : 0);
   const unsigned char* fl = a.flags + (AH ? (long long)blockIdx.z * a.fr * a.fc : 0);
-  double2 acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
+  zg::TileAcc acc;
+  acc.clear();
   auto active = [&](int c) {
     const int e = c / per, kc = c - e * per;
     unsigned f = 0;
@@ -127,38 +124,25 @@ __global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs a) {
   };
   zg::tile_loop<AH ? zg::CONJ_A : zg::NONE>(acc, smem, blockIdx.y, splits, per * a.nseg, active, load);
   double2* out = a.parts + ((long long)blockIdx.z * splits + blockIdx.y) * a.m * a.p;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int r = m0 + ty + 16 * i, c = tx + 16 * j;
-      if (r < a.m && c < a.p) out[(long long)r * a.p + c] = acc[i][j];
-    }
+  acc.each([&](int i, int j, double2 v) {
+    const int r = m0 + zg::tile_row() + i, c = zg::tile_col() + j;
+    if (r < a.m && c < a.p) out[(long long)r * a.p + c] = v;
+  });
 }
 
-// Row-block kernels: each block takes groups of RB rows (g, g + gridDim.x, ...) of n x p arrays.  gram: the block's
-// share of L^H Y (Hermitian: L = Y, or Y = T L), accumulated over its groups by the outputs (ty + 16 i, tx + 16 j),
-// i <= j, of each thread.
+// Row-block kernels: each block takes groups of RB rows (g, g + gridDim.x, ...) of n x p arrays, held in shared memory
+// with rows of PL values.  gram: the block's share of L^H Y (Hermitian: L = Y, or Y = T L), accumulated over its
+// groups; its 16 x 16 blocks on and above the diagonal are stored.
+constexpr int PL = zg::LD;
 template <int RB>
-__device__ __forceinline__ void gram_rows(double2 (&acc)[4][4], const double2* L, const double2* Y, int tx, int ty) {
-#pragma unroll 4
-  for (int r = 0; r < RB; ++r) {
-    double2 a[4], b[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = L[r * PMAX + ty + 16 * u];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) b[u] = Y[r * PMAX + tx + 16 * u];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = u; v < 4; ++v) cfma_conj(acc[u][v], b[v], a[u]);
-  }
+__device__ __forceinline__ void gram_rows(zg::TileAcc& acc, const double2* L, const double2* Y) {
+  zg::warp_mma<zg::CONJ_A, RB>(acc, L + zg::tile_row(), 1, PL, Y + zg::tile_col(), PL);
 }
-__device__ __forceinline__ void store_gram(const double2 (&acc)[4][4], double2* gparts, int tx, int ty) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = i; j < 4; ++j) gparts[(long long)blockIdx.x * PMAX * PMAX + (ty + 16 * i) * PMAX + tx + 16 * j] = acc[i][j];
+__device__ __forceinline__ void store_gram(const zg::TileAcc& acc, double2* gparts) {
+  acc.each([&](int i, int j, double2 v) {
+    const int r = zg::tile_row() + i, c = zg::tile_col() + j;
+    if ((c >> 4) >= (r >> 4)) gparts[(long long)blockIdx.x * PMAX * PMAX + r * PMAX + c] = v;
+  });
 }
 
 // out = alpha sum_z parts[z] + beta b1 + gamma b0 (rows of n x p; batch blockIdx.y of n rows), and, with gparts, the
@@ -173,17 +157,14 @@ struct FoldArgs {
 template <int RB>
 __global__ void __launch_bounds__(256) fold_kernel(FoldArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double2* ys = (double2*)smem;                  // [RB][64]
-  double2* ls = a.left ? ys + RB * PMAX : ys;    // left's rows, when given
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  double2* ys = (double2*)smem;                // [RB][PL]
+  double2* ls = a.left ? ys + RB * PL : ys;    // left's rows, when given
+  const int tid = threadIdx.x;
   pdl_trigger();
   pdl_wait();
   const long long np = (long long)a.n * a.p, boff = blockIdx.y * np;
-  double2 acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
+  zg::TileAcc acc;
+  acc.clear();
   for (int g = blockIdx.x; g * RB < a.n; g += gridDim.x) {
     double2 v[RB / 4];
 #pragma unroll
@@ -215,16 +196,16 @@ __global__ void __launch_bounds__(256) fold_kernel(FoldArgs a) {
         a.out[boff + e] = y;
         if (a.left) l = a.left[e];
       }
-      ys[((tid >> 6) + 4 * i) * PMAX + c] = y;
-      if (a.left) ls[((tid >> 6) + 4 * i) * PMAX + c] = l;
+      ys[((tid >> 6) + 4 * i) * PL + c] = y;
+      if (a.left) ls[((tid >> 6) + 4 * i) * PL + c] = l;
     }
     if (a.gparts) {
       __syncthreads();
-      gram_rows<RB>(acc, ls, ys, tx, ty);
+      gram_rows<RB>(acc, ls, ys);
       __syncthreads();
     }
   }
-  if (a.gparts) store_gram(acc, a.gparts, tx, ty);
+  if (a.gparts) store_gram(acc, a.gparts);
 }
 
 // G[r][c] = sum_b gparts[b][r][c] (p x p of the 64 x 64 shares), in a fixed order, for the stored 16 x 16 blocks, and
@@ -255,7 +236,7 @@ __global__ void __launch_bounds__(256) sum_gram_kernel(const double2* gparts, in
 // rdiag[c] = the diagonal of R = (X Rinv)^H X (the second pass multiplies the two passes' factors).
 // Bound: the chain of 64 dependent steps.  Each thread keeps its 2 x 4 entries (ty + 32 i, tx + 16 j) in registers; a
 // step is one barrier (row j and column j through a double-buffered line of shared memory, 1 / d_j by the entry's
-// owner).  64 x 64: CHOL_US us; with the matrix in shared memory, three barriers a step and a back substitution by one
+// owner).  64 x 64: 39 us; with the matrix in shared memory, three barriers a step and a back substitution by one
 // thread per column it was 277 us.
 __global__ void __launch_bounds__(512) chol_inv_kernel(int p, const double2* G, double2* Rinv, double* rdiag,
                                                        double shift, bool first) {
@@ -336,76 +317,59 @@ __global__ void __launch_bounds__(512) chol_inv_kernel(int p, const double2* G, 
   }
 }
 
-// Loads a group of RB rows of an n x p array (zero beyond) into [RB][PMAX].
+// Loads a group of RB rows of an n x p array (zero beyond) into [RB][PL], and a p x p matrix into [64][PL].
 template <int RB>
 __device__ __forceinline__ void load_group(double2* s, const double2* src, int n, int p, int g) {
 #pragma unroll
   for (int i = 0; i < RB / 4; ++i) {
     const int e = threadIdx.x + 256 * i, r = e >> 6, c = e & 63;
-    s[e] = g * RB + r < n && c < p ? src[(long long)(g * RB + r) * p + c] : make_double2(0, 0);
+    s[r * PL + c] = g * RB + r < n && c < p ? src[(long long)(g * RB + r) * p + c] : make_double2(0, 0);
   }
 }
 __device__ __forceinline__ void load_square(double2* s, const double2* src, int p) {
+#pragma unroll 4
   for (int e = threadIdx.x; e < PMAX * PMAX; e += 256) {
     const int r = e >> 6, c = e & 63;
-    s[e] = r < p && c < p ? src[r * p + c] : make_double2(0, 0);
+    s[r * PL + c] = r < p && c < p ? src[r * p + c] : make_double2(0, 0);
   }
 }
-// o[i][j] = sum_k xs[ty + 16 i][k] q[k][tx + 16 j], i < RB / 16
+// xs q for a group: RB x 64 by 8 warps, 16 rows x 8 NI columns each (NI = RB / 16)
+template <int RB> using GroupAcc = zg::Acc<2, RB / 16>;
+template <int RB> __device__ __forceinline__ int group_row() { return RB == 32 ? 16 * (threadIdx.x >> 7) : 0; }
+template <int RB> __device__ __forceinline__ int group_col() { return (RB / 2) * ((threadIdx.x >> 5) & (128 / RB - 1)); }
 template <int RB>
-__device__ __forceinline__ void times_square(double2 (&o)[RB / 16][4], const double2* xs, const double2* q, int tx, int ty) {
-#pragma unroll
-  for (int i = 0; i < RB / 16; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) o[i][j] = make_double2(0, 0);
-#pragma unroll 4
-  for (int k = 0; k < PMAX; ++k) {
-    double2 b[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = q[k * PMAX + tx + 16 * j];
-#pragma unroll
-    for (int i = 0; i < RB / 16; ++i) {
-      const double2 x = xs[(ty + 16 * i) * PMAX + k];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cfma(o[i][j], x, b[j]);
-    }
-  }
+__device__ __forceinline__ void times_square(GroupAcc<RB>& o, const double2* xs, const double2* q) {
+  o.clear();
+  zg::warp_mma<zg::NONE, PMAX>(o, xs + group_row<RB>() * PL, PL, 1, q + group_col<RB>(), PL);
 }
 
 // X <- X Rinv in place (groups of RB rows), and, with gparts, the shares of the result's Gram matrix.
 template <int RB>
 __global__ void __launch_bounds__(256) scale_kernel(int n, int p, double2* X, const double2* Rinv, double2* gparts) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double2* q = (double2*)smem;            // [64][64]
-  double2* xs = q + PMAX * PMAX;          // [RB][64]
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  double2* q = (double2*)smem;          // [64][PL]
+  double2* xs = q + PMAX * PL;          // [RB][PL]
   pdl_trigger();
   pdl_wait();
   load_square(q, Rinv, p);
-  double2 acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
+  zg::TileAcc acc;
+  acc.clear();
   for (int g = blockIdx.x; g * RB < n; g += gridDim.x) {
     load_group<RB>(xs, X, n, p, g);
     __syncthreads();
-    double2 o[RB / 16][4];
-    times_square<RB>(o, xs, q, tx, ty);
+    GroupAcc<RB> o;
+    times_square<RB>(o, xs, q);
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < RB / 16; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = ty + 16 * i, c = tx + 16 * j;
-        xs[r * PMAX + c] = o[i][j];
-        if (g * RB + r < n && c < p) X[(long long)(g * RB + r) * p + c] = o[i][j];
-      }
+    o.each([&](int i, int j, double2 v) {
+      const int r = group_row<RB>() + i, c = group_col<RB>() + j;
+      xs[r * PL + c] = v;
+      if (g * RB + r < n && c < p) X[(long long)(g * RB + r) * p + c] = v;
+    });
     __syncthreads();
-    if (gparts) gram_rows<RB>(acc, xs, xs, tx, ty);
+    if (gparts) gram_rows<RB>(acc, xs, xs);
     __syncthreads();
   }
-  if (gparts) store_gram(acc, gparts, tx, ty);
+  if (gparts) store_gram(acc, gparts);
 }
 
 // X <- X Q, Z <- Z Q in place, and the shares rparts[block][64] of sum_rows |Z - w X|^2 per column.
@@ -413,47 +377,46 @@ template <int RB>
 __global__ void __launch_bounds__(256) ritz_kernel(int n, int p, double2* X, double2* Z, const double2* Q, const double* w,
                                                    double* rparts) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double2* q = (double2*)smem;            // [64][64]
-  double2* xs = q + PMAX * PMAX;          // [RB][64]
-  double2* zs = xs + RB * PMAX;           // [RB][64]
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  double2* q = (double2*)smem;          // [64][PL]
+  double2* xs = q + PMAX * PL;          // [RB][PL]
+  double2* zs = xs + RB * PL;           // [RB][PL]
+  const int tid = threadIdx.x;
   pdl_trigger();
   pdl_wait();
   load_square(q, Q, p);
-  double res[4] = {0, 0, 0, 0}, wc[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) wc[j] = tx + 16 * j < p ? w[tx + 16 * j] : 0.0;
+  double res = 0;   // column tid / 4, rows tid % 4 + 4 i
+  const int col = tid >> 2;
+  const double wc = col < p ? w[col] : 0.0;
   for (int g = blockIdx.x; g * RB < n; g += gridDim.x) {
     load_group<RB>(xs, X, n, p, g);
     load_group<RB>(zs, Z, n, p, g);
     __syncthreads();
-    double2 ox[RB / 16][4], oz[RB / 16][4];
-    times_square<RB>(ox, xs, q, tx, ty);
-    times_square<RB>(oz, zs, q, tx, ty);
+    GroupAcc<RB> ox, oz;
+    times_square<RB>(ox, xs, q);
+    times_square<RB>(oz, zs, q);
+    __syncthreads();
+    ox.each([&](int i, int j, double2 v) { xs[(group_row<RB>() + i) * PL + group_col<RB>() + j] = v; });
+    oz.each([&](int i, int j, double2 v) { zs[(group_row<RB>() + i) * PL + group_col<RB>() + j] = v; });
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < RB / 16; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = g * RB + ty + 16 * i, c = tx + 16 * j;
-        if (r < n && c < p) {
-          X[(long long)r * p + c] = ox[i][j];
-          Z[(long long)r * p + c] = oz[i][j];
-        }
-        const double dx = oz[i][j].x - wc[j] * ox[i][j].x, dy = oz[i][j].y - wc[j] * ox[i][j].y;
-        res[j] += dx * dx + dy * dy;
+    for (int i = 0; i < RB / 4; ++i) {
+      const int e = tid + 256 * i, r = e >> 6, c = e & 63;
+      if (g * RB + r < n && c < p) {
+        X[(long long)(g * RB + r) * p + c] = xs[r * PL + c];
+        Z[(long long)(g * RB + r) * p + c] = zs[r * PL + c];
       }
-  }
-  double* rs = (double*)xs;   // [16][64]
-  __syncthreads();
+    }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) rs[ty * PMAX + tx + 16 * j] = res[j];
-  __syncthreads();
-  if (tid < PMAX) {
-    double s = 0;
-    for (int i = 0; i < 16; ++i) s += rs[i * PMAX + tid];
-    rparts[blockIdx.x * PMAX + tid] = s;
+    for (int i = 0; i < RB / 4; ++i) {
+      const double2 x = xs[((tid & 3) + 4 * i) * PL + col], z = zs[((tid & 3) + 4 * i) * PL + col];
+      const double dx = z.x - wc * x.x, dy = z.y - wc * x.y;
+      res += dx * dx + dy * dy;
+    }
+    __syncthreads();
   }
+  res += __shfl_xor_sync(0xffffffffu, res, 1);
+  res += __shfl_xor_sync(0xffffffffu, res, 2);
+  if ((tid & 3) == 0) rparts[blockIdx.x * PMAX + col] = res;
 }
 
 // res[c] = sqrt(sum_b rparts[b][c]).
@@ -494,7 +457,7 @@ __global__ void start_block_kernel(double2* X, long long count, unsigned long lo
 // warp derives the next step's rotations (algebraically, from square roots and divisions).  Pairs are dealt as
 // (k, k + d mod 32): neighbouring lanes touch neighbouring rows and columns, which with a row of 64 values falls on
 // different banks.  Sweeps end when the off-diagonal part is at rounding level, or below 1e-12 and no longer falling.
-// 64 x 64: JAC_US us a sweep, 2 to 7 sweeps; with separate column and row updates of the full matrix, trigonometric
+// 64 x 64: 145 us a sweep, 2 to 7 sweeps; with separate column and row updates of the full matrix, trigonometric
 // rotations and serial bookkeeping by one thread a decomposition took 2.8 ms.
 struct Rot { double cs, sn, ex, ey; };
 constexpr int JN = PMAX, JH = PMAX / 2;
@@ -695,7 +658,7 @@ struct Solver {
 
   void fold(const FoldArgs& f, int batch = 1) {
     const int blocks = f.gparts ? groups() : ceil_div(f.n, 16);
-    const size_t row = sizeof(double2) * PMAX * (f.left ? 2 : 1);
+    const size_t row = sizeof(double2) * PL * (f.left ? 2 : 1);
     if (!f.gparts || fine())
       run("oi_eig_topk64/fold", fold_kernel<16>, dim3(blocks, batch), 256, 16 * row, f);
     else
@@ -719,18 +682,19 @@ struct Solver {
     fold(FoldArgs{parts, sh, n, p, alpha, beta, gamma, b1, b0, left, out, gram ? gparts : nullptr});
   }
   void sum_gram() { run("oi_eig_topk64/gram", sum_gram_kernel, dim3(p), 256, 0, (const double2*)gparts, groups(), p, G); }
-  // X <- CholQR2(X); the Gram shares of X are in gparts.
-  void orth(double2* X) {
-    for (int pass = 0; pass < 2; ++pass) {
+  // X R = X by Cholesky QR, the Gram shares of X in gparts: one pass keeps the columns independent, a second one
+  // (wanted before a projection) makes them orthonormal to rounding.
+  void orth(double2* X, int passes) {
+    for (int pass = 0; pass < passes; ++pass) {
       sum_gram();
       run("oi_eig_topk64/chol", chol_inv_kernel, dim3(1), 512, 0, p, (const double2*)G, Rinv, rdiag,
           pass == 0 ? 1e-13 : 1e-15, pass == 0);
-      double2* gp = pass == 0 ? gparts : nullptr;
+      double2* gp = pass + 1 < passes ? gparts : nullptr;
       if (fine())
-        run("oi_eig_topk64/scale", scale_kernel<16>, dim3(groups()), 256, sizeof(double2) * PMAX * (PMAX + 16), n, p, X,
+        run("oi_eig_topk64/scale", scale_kernel<16>, dim3(groups()), 256, sizeof(double2) * PL * (PMAX + 16), n, p, X,
             (const double2*)Rinv, gp);
       else
-        run("oi_eig_topk64/scale", scale_kernel<32>, dim3(groups()), 256, sizeof(double2) * PMAX * (PMAX + 32), n, p, X,
+        run("oi_eig_topk64/scale", scale_kernel<32>, dim3(groups()), 256, sizeof(double2) * PL * (PMAX + 32), n, p, X,
             (const double2*)Rinv, gp);
     }
   }
@@ -792,16 +756,16 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
       sv.status = fail(OI_ECUDA, "oi_eig_topk64: %s", cudaGetErrorString(cudaGetLastError()));
     return sv.status == OI_OK;
   };
-  auto plain = [&](int count) {   // X = CholQR2(T X)
+  auto plain = [&](int count, int last_passes) {   // X R = T X
     for (int i = 0; i < count && it < max_iter; ++i, ++it) {
       sv.apply(X, X, 1.0, 0.0, nullptr, 0.0, nullptr, true, nullptr);
-      sv.orth(X);
+      sv.orth(X, i + 1 < count && it + 1 < max_iter ? 1 : last_passes);
     }
   };
-  // X = CholQR2(f(T) X) with f small on [0, b], for values w0 >= wk wanted and the residual `worst` (over w0)
+  // X R = f(T) X with f small on [0, b], for values w0 >= wk wanted and the residual `worst` (over w0)
   auto filter = [&](double w0, double wk, double b, double worst) {
     const double x = 2 * wk / b - 1, x0 = 2 * w0 / b - 1;
-    if (!(x > 1.05)) return plain(4);
+    if (!(x > 1.05)) return plain(4, 2);
     const double rho = x + std::sqrt(x * x - 1), rho0 = x0 + std::sqrt(x0 * x0 - 1);
     const double want = std::ceil(std::log(100.0 * worst / tol) / std::log(rho));
     int total = (int)std::max(1.0, std::min((double)std::min(EIG_DEGREE, max_iter - it), want));
@@ -823,12 +787,13 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
         std::swap(X, Z);
       }
       std::swap(X, Z);   // the newest is in X
-      sv.orth(X);
+      sv.orth(X, total > 0 ? 1 : 2);
     }
   };
 
   std::swap(X, Z);   // the random block is the first X
-  plain(EIG_START);
+  plain(EIG_START, 1);
+  bool ready = false;   // X is orthonormal to rounding
   if (it < max_iter && fetch(rdiag, p)) {
     for (int i = 0; i < p; ++i)
       if (!(host[i] > 0)) host[i] = 0;
@@ -836,8 +801,13 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
     const double w0 = host[0], wk = host[k - 1], wp = host[p - 1];
     // the error left after the plain iterations; a TCC that is not a number, or of a rank below k, goes on to the
     // projection as it is
-    if (w0 > 0 && wk > 1e-8 * w0)
+    ready = w0 > 0 && wk > 1e-8 * w0;
+    if (ready)
       filter(w0, wk, std::max(1.05 * wp, 1e-8 * w0), std::min(1.0, std::pow(wp / wk, EIG_START)) * wk / w0);
+  }
+  if (!ready) {
+    sv.fold(FoldArgs{nullptr, 0, n, p, 0.0, 1.0, 0.0, X, nullptr, nullptr, X, gparts});
+    sv.orth(X, 2);
   }
   while (!sv.status) {
     // Rayleigh-Ritz: Z = T X, H = X^H Z
@@ -845,10 +815,10 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
     sv.sum_gram();
     sv.run("oi_eig_topk64/jacobi", heev_jacobi_kernel, dim3(1), 1024, JACOBI_SMEM, p, (const double2*)G, w, Q, 40);
     if (sv.fine())
-      sv.run("oi_eig_topk64/ritz", ritz_kernel<16>, dim3(sv.groups()), 256, sizeof(double2) * PMAX * (PMAX + 32), n, p, X, Z,
+      sv.run("oi_eig_topk64/ritz", ritz_kernel<16>, dim3(sv.groups()), 256, sizeof(double2) * PL * (PMAX + 32), n, p, X, Z,
              (const double2*)Q, (const double*)w, rparts);
     else
-      sv.run("oi_eig_topk64/ritz", ritz_kernel<32>, dim3(sv.groups()), 256, sizeof(double2) * PMAX * (PMAX + 64), n, p, X, Z,
+      sv.run("oi_eig_topk64/ritz", ritz_kernel<32>, dim3(sv.groups()), 256, sizeof(double2) * PL * (PMAX + 64), n, p, X, Z,
              (const double2*)Q, (const double*)w, rparts);
     sv.run("oi_eig_topk64/residual", residual_kernel, dim3(1), 1024, 0, (const double*)rparts, sv.groups(), p, res);
     if (!fetch(w, 2 * (size_t)p)) break;
@@ -863,7 +833,7 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
     if (last >= 0 && worst > 0.25 * last) ++stalls;
     last = worst;
     if (stalls)
-      plain(4);
+      plain(4, 2);
     else
       filter(w0, host[k - 1], std::max(1.05 * host[p - 1], 1e-8 * w0), worst / w0);
   }

@@ -2,10 +2,11 @@
 // tile by 256 threads, K in chunks of 16 through a ring of shared-memory stages filled by 16-byte asynchronous
 // copies (one complex value each, so either operand can be transposed on the way in).
 //
-// Bound: FP64 issue (64 DFMA per SM and cycle).  Each thread owns the 4 x 4 outputs (ty + 16 i, tx + 16 j): per k a
-// warp reads 4 + 4 values as 12 conflict-free shared-memory wavefronts against 64 DFMA (128 issue cycles).  With the
-// outputs 4 ty + i, 4 tx + j the column reads are 64 bytes apart, an 8-way bank conflict, and the TCC assembly ran at
-// a third of the FP64 rate.
+// Bound: FP64 issue (64 multiply-adds per SM and cycle).  The products run on the FP64 matrix instruction
+// (mma.sync m8n8k4): each of the 8 warps owns 32 x 16 outputs, and per four k a warp reads 4 + 2 shared-memory values a
+// lane for 32 matrix instructions (8192 multiply-adds).  As scalar FMAs on 4 x 4 outputs a thread, the same work needs
+// 32 such reads, and shared memory is as busy as the FP64 pipe: T X at 3481 x 3481 x 64, about 60 % of it zero blocks,
+// 218 -> 169 us.
 #pragma once
 #include "oi_common.cuh"
 #include <cstdint>
@@ -14,7 +15,7 @@ namespace oi {
 namespace zg {
 
 constexpr int T = 64, KC = 16;             // output tile, K chunk
-constexpr int LD = T + 1;                  // stage row (odd: transposing copies touch every bank)
+constexpr int LD = T + 2;                  // stage row: 2 (mod 8), so that a fragment's 4 x 2 values fall on 8 banks
 constexpr int STAGES = 3;
 constexpr int STAGE_Z = 2 * KC * LD;       // complex values per stage: A and B
 constexpr int LIST = 1024;                 // chunks looked at together
@@ -29,23 +30,72 @@ __device__ __forceinline__ void cp16(double2* dst, const double2* src, bool on) 
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// acc (+)= a b, conj(a) b or a conj(b)
-enum Conj { NONE, CONJ_A, CONJ_B };
-template <int C> __device__ __forceinline__ void mac(double2& acc, double2 a, double2 b) {
-  if (C == NONE) cfma(acc, a, b);
-  if (C == CONJ_A) cfma_conj(acc, b, a);
-  if (C == CONJ_B) cfma_conj(acc, a, b);
+// Output tile of a warp, 8 MI x 8 NI complex values: lane l holds rows l / 4 + 8 i, columns 2 (l % 4) + {0, 1} + 8 j.
+template <int MI, int NI> struct Acc {
+  double re[MI][NI][2], im[MI][NI][2];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NI; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+  }
+  // f(row, column, value) of this lane's values
+  template <typename F> __device__ __forceinline__ void each(F f) const {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NI; ++j)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          f((lane >> 2) + 8 * i, 2 * (lane & 3) + u + 8 * j, make_double2(re[i][j][u], im[i][j][u]));
+  }
+};
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
 }
 
+// acc += a b, conj(a) b or a conj(b) over KN (a multiple of 4) values of k: a(i, k) = A[i * am + k * ak], row i of the
+// warp's tile, b(k, j) = B[k * bk + j].
+enum Conj { NONE, CONJ_A, CONJ_B };
+template <int C, int KN, int MI, int NI>
+__device__ __forceinline__ void warp_mma(Acc<MI, NI>& acc, const double2* A, int am, int ak, const double2* B, int bk) {
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int k = 0; k < KN; k += 4) {
+    double2 a[MI], b[NI];
+#pragma unroll
+    for (int i = 0; i < MI; ++i) a[i] = A[(r + 8 * i) * am + (k + q) * ak];
+#pragma unroll
+    for (int j = 0; j < NI; ++j) b[j] = B[(k + q) * bk + r + 8 * j];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NI; ++j) {
+        dmma(acc.re[i][j], a[i].x, b[j].x);
+        dmma(acc.re[i][j], C == NONE ? -a[i].y : a[i].y, b[j].y);
+        dmma(acc.im[i][j], C == CONJ_B ? -a[i].x : a[i].x, b[j].y);
+        dmma(acc.im[i][j], C == CONJ_A ? -a[i].y : a[i].y, b[j].x);
+      }
+  }
+}
+
+using TileAcc = Acc<4, 2>;   // 64 x 64 by 8 warps: warp w at rows 32 (w / 4), columns 16 (w % 4)
+__device__ __forceinline__ int tile_row() { return 32 * (threadIdx.x >> 7); }
+__device__ __forceinline__ int tile_col() { return 16 * ((threadIdx.x >> 5) & 3); }
+
 // Runs the K loop of one tile.  active(c): whether chunk c (first + i * step, c < chunks) contributes; load(c, As, Bs)
-// issues the copies of chunk c into As[KC][LD], Bs[KC][LD] (k-major).  acc[i][j] is output (ty + 16 i, tx + 16 j).
+// issues the copies of chunk c into As[KC][LD], Bs[KC][LD] (k-major).
 template <int C, typename Active, typename Load>
-__device__ __forceinline__ void tile_loop(double2 (&acc)[4][4], unsigned char* smem, int first, int step, int chunks,
+__device__ __forceinline__ void tile_loop(TileAcc& acc, unsigned char* smem, int first, int step, int chunks,
                                           Active active, Load load) {
   double2* ring = (double2*)smem;
   unsigned short* list = (unsigned short*)(ring + STAGES * STAGE_Z);
   int* wsum = (int*)(list + LIST);   // [8] per-warp counts
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int base = 0; first + base * step < chunks; base += LIST) {
     int count = 0;
     __syncthreads();   // the previous window's list and stages are consumed
@@ -80,18 +130,7 @@ __device__ __forceinline__ void tile_loop(double2 (&acc)[4][4], unsigned char* s
       fetch(i + STAGES - 1);
       const double2* As = ring + (i % STAGES) * STAGE_Z;
       const double2* Bs = As + KC * LD;
-#pragma unroll 4
-      for (int k = 0; k < KC; ++k) {
-        double2 a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = As[k * LD + ty + 16 * u];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) b[u] = Bs[k * LD + tx + 16 * u];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) mac<C>(acc[u][v], a[u], b[v]);
-      }
+      warp_mma<C, KC>(acc, As + tile_row(), 1, LD, Bs + tile_col(), LD);
     }
     cp_wait<0>();
   }
