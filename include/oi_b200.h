@@ -371,6 +371,14 @@ OI_API int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int s, i
  */
 OI_API int oi_tcc_assemble64(const void* h, int ne, int fg, int nsrc, void* tcc, void* stream);
 
+/*
+ * oi_tcc_assemble64 with a workspace (oi_tcc_assemble64_marked_workspace bytes, device) for marks of h's non-zero
+ * blocks: blocks that add nothing are left out (a pupil sample outside the shifted disc is zero).  Same result.
+ */
+OI_API int oi_tcc_assemble64_marked_workspace(int ne, int fg, int nsrc, long long* bytes);
+OI_API int oi_tcc_assemble64_marked(const void* h, int ne, int fg, int nsrc, void* tcc, void* work,
+                                    long long work_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -26,6 +26,8 @@ _SIGS = {
     'oi_abbe_pupils_pol': [_vp, _vp, _i, _i, _vp, _vp, _vp, _i, _d, _vp, _i, _vp, _i, _vp, _d, _d, _d, _d, _vp,
                            _vp, _vp],
     'oi_tcc_assemble64': [_vp, _i, _i, _i, _vp, _vp],
+    'oi_tcc_assemble64_marked_workspace': [_i, _i, _i, _vp],
+    'oi_tcc_assemble64_marked': [_vp, _i, _i, _i, _vp, _vp, _ll, _vp],
     'oi_fft_supported': [_i, _i],
     'oi_band_spectrum_fft': [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp, _vp],
     'oi_coarse_to_image_fft': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp,

@@ -461,10 +461,19 @@ def tcc_pupil_matrix(source, xypitch, projector, focus, numerics):
 def CalculateTCCMatrix(source, xypitch, projector, focus, numerics):
     """TCC [FG, FG] complex128 on the device and FG_ValidSize [len g, len f] (CalculateTCCMatrix.py:9-56)."""
     h, fg = tcc_pupil_matrix(source, xypitch, projector, focus, numerics)
-    n = h.shape[1]
+    return _assemble_tcc(h), fg
+
+
+def _assemble_tcc(h):
+    """sum_e h_e h_e^H [FG, FG] complex128 from h [ne, FG, S] on the device."""
+    ne, n, s = h.shape
     tcc = torch.empty((n, n), dtype=torch.complex128, device=h.device)
-    N.call('oi_tcc_assemble64', N.ptr(h), h.shape[0], n, h.shape[2], N.ptr(tcc), N.stream_handle(h.device))
-    return tcc, fg
+    nbytes = ctypes.c_longlong(0)
+    N.call('oi_tcc_assemble64_marked_workspace', ne, n, s, ctypes.byref(nbytes))
+    work = torch.empty(nbytes.value, dtype=torch.uint8, device=h.device)
+    N.call('oi_tcc_assemble64_marked', N.ptr(h), ne, n, s, N.ptr(tcc), N.ptr(work), nbytes.value,
+           N.stream_handle(h.device))
+    return tcc
 
 
 def GetTCCMatrix(sourceData, shiftedPupil):
@@ -472,11 +481,7 @@ def GetTCCMatrix(sourceData, shiftedPupil):
     dev = require_cuda()
     w = sourceData.Value.reshape(-1).to(torch.float64)
     p = torch.as_tensor(shiftedPupil).to(dev, torch.complex128)
-    h = (p * torch.sqrt(w.to(dev) / torch.sum(w).to(dev))).contiguous().unsqueeze(0)
-    n = h.shape[1]
-    tcc = torch.empty((n, n), dtype=torch.complex128, device=dev)
-    N.call('oi_tcc_assemble64', N.ptr(h), 1, n, h.shape[2], N.ptr(tcc), N.stream_handle(dev))
-    return tcc
+    return _assemble_tcc((p * torch.sqrt(w.to(dev) / torch.sum(w).to(dev))).contiguous().unsqueeze(0))
 
 
 def _socs_count(numerics, evals, size):
@@ -565,9 +570,7 @@ def socs_kernels_from_pupils(h, FG_ValidSize, Nfg, numerics) -> SocsKernels:
     Kernels equal socs_kernels_from_tcc's up to a phase per kernel (images are unchanged)."""
     ne, fg, s = h.shape
     if ne * s >= fg:
-        tcc = torch.empty((fg, fg), dtype=torch.complex128, device=h.device)
-        N.call('oi_tcc_assemble64', N.ptr(h), ne, fg, s, N.ptr(tcc), N.stream_handle(h.device))
-        return socs_kernels_from_tcc(tcc, FG_ValidSize, Nfg, numerics)
+        return socs_kernels_from_tcc(_assemble_tcc(h), FG_ValidSize, Nfg, numerics)
     nf, ng = Nfg
     lg, lf = FG_ValidSize
     if lf > ng or lg > nf:
