@@ -782,7 +782,8 @@ extern "C" int oi_coarse_to_image_fft(float* coarse, int nparts, int count, int 
     else if (mr == 128) rc = launch_coarse_spec_fft<4, 2>(coarse, nparts, count, br, bc, tr, tc, ih, s);
     else rc = launch_coarse_spec_fft<2, 4>(coarse, nparts, count, br, bc, tr, tc, ih, s);
   } else {
-    rc = coarse_spectrum(coarse, count, mr, mc, br, bc, gc, gr, scratch_ihat, s, nparts);
+    rc = coarse_spectrum(coarse, count, mr, mc, br, bc, gc, gr, scratch_ihat, s, nparts, scratch_v,
+                         (long long)count * bc * ny * (long long)sizeof(float2));
   }
   if (rc) return rc;
   const float2* ih = (const float2*)scratch_ihat;

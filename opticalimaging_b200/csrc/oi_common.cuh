@@ -80,8 +80,9 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // Adds partial sums 1..nparts-1 (each n floats, one after another) into the first, in place.
 int fold_parts(float* coarse, int nparts, long long n, cudaStream_t s);
 
-// The coarse intensity may be split in `nparts` partial sums, each count*mr*mc floats, added in order.
+// The coarse intensity may be split in `nparts` partial sums, each count*mr*mc floats, added in order.  room: device
+// memory the caller does not need until the stage is done (it can be faster with count*mr*bc complex values of it).
 int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, const void* gc, const void* gr,
-                    void* ihat, cudaStream_t s, int nparts);
+                    void* ihat, cudaStream_t s, int nparts, void* room, long long room_bytes);
 
 }  // namespace oi

@@ -9,7 +9,7 @@
 // only qc >= 0 is kept (qc > 0 doubled) and the x synthesis is a real dot product:
 //   V[y][qc]   = sum_qr Ihat(qr, qc) exp(-2 pi i qr y/Ny)
 //   out[y][x]  = sum_qc Re(V[y][qc] exp(-2 pi i qc x/Nx))                                 (synth kernel)
-#include "oi_common.cuh"
+#include "dft_gemm.cuh"
 
 namespace oi {
 
@@ -53,61 +53,130 @@ __global__ void __launch_bounds__(256) coarse_spec_kernel(const float* __restric
   }
 }
 
-constexpr int SY_TY = 8;  // output rows per synth block
+// The same spectrum as two tile products (dft_gemm.cuh), U = coarse * gc and ihat = gr^T U, when the caller has room for
+// U: the partial sums are added as the first product's operand is read.  Four 128 x 128 coarse images of 59 x 59 bands:
+// 239 us (16 blocks, one output per thread at a time) -> 20 us, and the separate addition of the parts (4 us) goes.
+struct SpecRows {
+  using A = float;
+  static constexpr bool A_K = true;
+  const float* coarse;
+  int nparts;
+  long long pstride;
+  int mc, bc;
+  const float2* gc;
+  float2* u;
+  __device__ __forceinline__ float a(int, int R, int sc) const {
+    const float* p = coarse + (long long)R * mc + sc;
+    float v = __ldg(p);
+    for (int i = 1; i < nparts; ++i) v += __ldg(p + i * pstride);
+    return v;
+  }
+  __device__ __forceinline__ float2 b(int, int sc, int qc) const { return __ldg(gc + (long long)sc * bc + qc); }
+  __device__ __forceinline__ void put(int, int R, int qc, float2 v) const { u[(long long)R * bc + qc] = v; }
+};
+struct SpecCols {
+  using A = float2;
+  static constexpr bool A_K = false;
+  const float2* u;
+  int mr, nq, bc;
+  const float2* gr;
+  float norm;
+  float2* ihat;
+  __device__ __forceinline__ float2 a(int, int jr, int sr) const { return __ldg(gr + (long long)sr * nq + jr); }
+  __device__ __forceinline__ float2 b(int img, int sr, int qc) const { return u[((long long)img * mr + sr) * bc + qc]; }
+  __device__ __forceinline__ void put(int img, int jr, int qc, float2 v) const {
+    const float s = qc == 0 ? norm : 2.f * norm;
+    ihat[((long long)img * nq + jr) * bc + qc] = make_float2(v.x * s, v.y * s);
+  }
+};
 
-// grid (ceil(ny/8), count).
-template <int NV>
-__global__ void __launch_bounds__(256) synth_kernel(const float2* __restrict__ ihat, int br, int bc,
-                                                    const float2* __restrict__ sy, const float2* __restrict__ sx,
-                                                    int ny, int nx, float* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* vs = (float2*)smem_raw;  // [SY_TY][bc]
-  const int tid = threadIdx.x;
-  const int y0 = blockIdx.x * SY_TY;
-  const long long img = blockIdx.y;
-  const int nq = 2 * br - 1;
-  const float2* ih = ihat + img * (long long)nq * bc;
-  // V[r][qc] = sum_jr sy[y0+r][jr] ihat[jr][qc]
-  for (int e = tid; e < SY_TY * bc; e += 256) {
-    int r = e / bc, qc = e - r * bc, y = y0 + r;
-    float2 acc = make_float2(0.f, 0.f);
-    if (y < ny) {
-      const float2* srow = sy + (long long)y * nq;
-      for (int jr = 0; jr < nq; ++jr) cfma(acc, __ldg(srow + jr), __ldg(ih + (long long)jr * bc + qc));
+// RB output rows per block (grid ceil(ny / RB), count): V of those rows into shared memory by 16-frequency steps, then
+// out = Re(V sx) with one or two columns and all RB rows per thread; V is read as pairs of frequencies, one broadcast
+// 16-byte load per row for 4 or 8 multiply-adds.  Bound: FP32 issue.  Four 1000 x 750 images, 59 columns: 61 -> 45 us.
+template <int RB, int XV>
+__device__ __forceinline__ void synth_columns(const float4* vs, int pairs, const float2* __restrict__ sx, int bc, int nx,
+                                              int x0, float* o, int rows) {
+  float acc[RB][XV];
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int u = 0; u < XV; ++u) acc[r][u] = 0.f;
+  const int x = x0 + threadIdx.x;
+#pragma unroll 2
+  for (int q = 0; q < pairs; ++q) {
+    float2 t0[XV], t1[XV];
+#pragma unroll
+    for (int u = 0; u < XV; ++u) {
+      const bool in = x + 256 * u < nx;
+      const float2* p = sx + (long long)(2 * q) * nx + x + 256 * u;
+      t0[u] = in ? __ldg(p) : make_float2(0.f, 0.f);
+      t1[u] = in && 2 * q + 1 < bc ? __ldg(p + nx) : make_float2(0.f, 0.f);
     }
-    vs[e] = acc;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      const float4 v = vs[r * pairs + q];
+#pragma unroll
+      for (int u = 0; u < XV; ++u) {
+        acc[r][u] = fmaf(v.x, t0[u].x, fmaf(-v.y, t0[u].y, acc[r][u]));
+        acc[r][u] = fmaf(v.z, t1[u].x, fmaf(-v.w, t1[u].y, acc[r][u]));
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int u = 0; u < XV; ++u)
+      if (r < rows && x + 256 * u < nx) o[(long long)r * nx + x + 256 * u] = acc[r][u];
+}
+
+template <int RB>
+__global__ void __launch_bounds__(256, 2) synth_kernel(const float2* __restrict__ ihat, int br, int bc,
+                                                       const float2* __restrict__ sy, const float2* __restrict__ sx,
+                                                       int ny, int nx, float* __restrict__ out) {
+  constexpr int CG = 256 / RB, NQ = RB / 4, KS = 16;   // column groups of a row, outputs per thread, frequencies per step
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* vs = (float2*)smem_raw;   // [RB][2 * pairs]
+  __shared__ float2 ys[KS][RB + 1], hs[KS][64];
+  const int tid = threadIdx.x, y0 = blockIdx.x * RB, rows = min(RB, ny - y0), nq = 2 * br - 1, pairs = (bc + 1) / 2;
+  const long long img = blockIdx.y;
+  const float2* ih = ihat + img * (long long)nq * bc;
+  const int r = tid / CG, cq = tid % CG;
+  for (int q0 = 0; q0 < 2 * pairs; q0 += 64) {
+    float2 acc[NQ];
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) acc[j] = make_float2(0.f, 0.f);
+    for (int k0 = 0; k0 < nq; k0 += KS) {
+      __syncthreads();
+      for (int e = tid; e < KS * RB; e += 256) {
+        const int k = e % KS, rr = e / KS;
+        ys[k][rr] = rr < rows && k0 + k < nq ? __ldg(sy + (long long)(y0 + rr) * nq + k0 + k) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < KS * 64 / 256; ++i) {
+        const int e = tid + 256 * i, q = e % 64, k = e / 64;
+        hs[k][q] = k0 + k < nq && q0 + q < bc ? __ldg(ih + (long long)(k0 + k) * bc + q0 + q) : make_float2(0.f, 0.f);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        const float2 y = ys[k][r];
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) cfma(acc[j], y, hs[k][cq + CG * j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      const int q = q0 + cq + CG * j;
+      if (q < 2 * pairs) vs[r * 2 * pairs + q] = acc[j];
+    }
   }
   __syncthreads();
-  // out[y][x] = sum_qc (V.re * sx.re - V.im * sx.im)
-  float acc[SY_TY][NV];
-#pragma unroll
-  for (int r = 0; r < SY_TY; ++r)
-#pragma unroll
-    for (int v = 0; v < NV; ++v) acc[r][v] = 0.f;
-  for (int qc = 0; qc < bc; ++qc) {
-    float2 t[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      int x = tid + 256 * v;
-      t[v] = x < nx ? __ldg(sx + (long long)qc * nx + x) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int r = 0; r < SY_TY; ++r) {
-      float2 vv = vs[r * bc + qc];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) acc[r][v] = fmaf(vv.x, t[v].x, fmaf(-vv.y, t[v].y, acc[r][v]));
-    }
-  }
-  float* o = out + img * (long long)ny * nx;
-#pragma unroll
-  for (int r = 0; r < SY_TY; ++r) {
-    int y = y0 + r;
-    if (y >= ny) continue;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      int x = tid + 256 * v;
-      if (x < nx) o[(long long)y * nx + x] = acc[r][v];
-    }
+  float* o = out + (img * ny + y0) * (long long)nx;
+  for (int x0 = 0; x0 < nx; x0 += 512) {
+    if (nx - x0 > 256)
+      synth_columns<RB, 2>((const float4*)vs, pairs, sx, bc, nx, x0, o, rows);
+    else
+      synth_columns<RB, 1>((const float4*)vs, pairs, sx, bc, nx, x0, o, rows);
   }
 }
 
@@ -135,10 +204,19 @@ int fold_parts(float* coarse, int nparts, long long n, cudaStream_t s) {
 }
 
 int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, const void* gc, const void* gr,
-                    void* ihat, cudaStream_t s, int nparts) {
+                    void* ihat, cudaStream_t s, int nparts, void* room, long long room_bytes) {
   if (mr < 2 * br - 1 || mc < 2 * bc - 1)
     return fail(OI_EINVAL, "coarse grid %dx%d too small for band %dx%d", mr, mc, br, bc);
   if (mr > 1024 || count > 65535) return fail(OI_ERANGE, "coarse grid mr=%d or count=%d out of range", mr, count);
+  if ((long long)count * mr * bc * (long long)sizeof(float2) <= room_bytes) {
+    float2* u = (float2*)room;
+    const int nq = 2 * br - 1;
+    int rc = dg::gemm<64, 64, 4, 4>(SpecRows{coarse, nparts, (long long)count * mr * mc, mc, bc, (const float2*)gc, u}, 1,
+                                    count * mr, bc, mc, s, "coarse spectrum/rows");
+    if (rc) return rc;
+    return dg::gemm<32, 32, 2, 2>(SpecCols{u, mr, nq, bc, (const float2*)gr, 1.0f / ((float)mr * (float)mc), (float2*)ihat},
+                                  count, nq, bc, mr, s, "coarse spectrum/columns");
+  }
   int rc = fold_parts(coarse, nparts, (long long)count * mr * mc, s);
   if (rc) return rc;
   nparts = 1;
@@ -154,12 +232,24 @@ int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, co
   return check_launch("coarse spectrum");
 }
 
-template <int NV>
-static void launch_synth(const float2* ihat, int count, int br, int bc, const float2* sy, const float2* sx, int ny,
-                         int nx, float* out, cudaStream_t s) {
-  dim3 grid((unsigned)ceil_div(ny, SY_TY), (unsigned)count);
-  synth_kernel<NV><<<grid, 256, sizeof(float2) * SY_TY * bc, s>>>(ihat, br, bc, sy, sx, ny, nx, out);
+template <int RB>
+static void launch_synth_rb(const float2* ihat, int count, int br, int bc, const float2* sy, const float2* sx, int ny,
+                            int nx, float* out, cudaStream_t s) {
+  dim3 grid((unsigned)ceil_div(ny, RB), (unsigned)count);
+  synth_kernel<RB><<<grid, 256, sizeof(float2) * RB * 2 * ((bc + 1) / 2), s>>>(ihat, br, bc, sy, sx, ny, nx, out);
   oi::note_launch();
+}
+// More rows per block reuse the sx values more; fewer fill the SMs when there are few rows (and 16 rows of more than 256
+// frequencies pass the shared memory that needs no opt-in).
+static void launch_synth(const float2* ihat, int count, int br, int bc, const float2* sy, const float2* sx, int ny, int nx,
+                         float* out, cudaStream_t s) {
+  auto enough = [&](int rb) { return (long long)ceil_div(ny, rb) * count >= 148; };
+  if (enough(16) && bc <= 256)
+    launch_synth_rb<16>(ihat, count, br, bc, sy, sx, ny, nx, out, s);
+  else if (enough(8))
+    launch_synth_rb<8>(ihat, count, br, bc, sy, sx, ny, nx, out, s);
+  else
+    launch_synth_rb<4>(ihat, count, br, bc, sy, sx, ny, nx, out, s);
 }
 
 }  // namespace oi
@@ -176,19 +266,11 @@ extern "C" int oi_coarse_to_image(float* coarse, int nparts, int count, int mr, 
   if (mr > 1024 || bc > 512 || nx > 2048 || count > 65535)
     return fail(OI_ERANGE, "oi_coarse_to_image: sizes out of range (mr=%d bc=%d nx=%d)", mr, bc, nx);
   cudaStream_t s = (cudaStream_t)stream;
-  int rc = coarse_spectrum(coarse, count, mr, mc, br, bc, gc, gr, scratch, s, nparts);
+  // U lives in `out` until the synthesis writes it
+  int rc = coarse_spectrum(coarse, count, mr, mc, br, bc, gc, gr, scratch, s, nparts, out,
+                           (long long)count * ny * nx * (long long)sizeof(float));
   if (rc) return rc;
-  const float2* ih = (const float2*)scratch;
-  switch ((nx + 255) / 256) {
-    case 1: launch_synth<1>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    case 2: launch_synth<2>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    case 3: case 4:
-      launch_synth<4>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    case 5: case 6: case 7: case 8:
-      launch_synth<8>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    default:
-      return fail(OI_ERANGE, "oi_coarse_to_image: nx=%d above 2048 not supported", nx);
-  }
+  launch_synth((const float2*)scratch, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s);
   return check_launch("oi_coarse_to_image/synth");
 }
 
@@ -200,14 +282,6 @@ extern "C" int oi_spectrum_to_image(const void* ihat, int count, int br, int bc,
   if (bc > 512 || nx > 2048 || count > 65535)
     return fail(OI_ERANGE, "oi_spectrum_to_image: sizes out of range (bc=%d nx=%d)", bc, nx);
   cudaStream_t s = (cudaStream_t)stream;
-  const float2* ih = (const float2*)ihat;
-  switch ((nx + 255) / 256) {
-    case 1: launch_synth<1>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    case 2: launch_synth<2>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    case 3: case 4:
-      launch_synth<4>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-    default:
-      launch_synth<8>(ih, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s); break;
-  }
+  launch_synth((const float2*)ihat, count, br, bc, (const float2*)sy, (const float2*)sx, ny, nx, out, s);
   return check_launch("oi_spectrum_to_image");
 }
