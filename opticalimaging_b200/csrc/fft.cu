@@ -286,45 +286,47 @@ __global__ void __launch_bounds__(COLS_T, 6) fft_cols_fwd_kernel(const float2* _
 // --------------------------------------------------------------------------- inverse, shared part
 // Thread n1 of a group: z[k2] = W_N^{-k2 n1} sum_{k1} coef(k2 + 32 k1) W_N1^{-k1 n1} over the non-zero
 // coefficients, which sit at frequencies q in [-qmax, qmax] (index q mod N); coef(q) = cq[q + qmax].
-template <int N1>
+// H = 2, 4: |q| < 32 H, the inputs of k2 are q = k2 + 32 k1, -H <= k1 < H: 2 H predicated terms with their twiddles
+// in registers and no runtime loops, so the 32 independent k2 chains interleave.  H = 0: any qmax.
+template <int N1, int H>
 __device__ __forceinline__ void inverse_gather(float2 (&z)[32], const float2* cq, int qmax, const float2* t2,
                                                const float2* t1, int n1) {
   constexpr int N = 32 * N1;
-  if (qmax < 64) {
-    // |q| <= 63: the only non-zero inputs of k2 are q = k2, k2 + 32 (k1 = 0, 1) and q = k2 - 32, k2 - 64
-    // (k1 = N1 - 1, N1 - 2).  Four predicated terms with their twiddles in registers: no runtime loops, so
-    // the 32 independent k2 chains interleave.
-    const float2 w1 = sgn<-1>(t1[1 * N1 + n1]);            // W_N1^{-n1}
-    const float2 wm1 = sgn<-1>(t1[(N1 - 1) * N1 + n1]);    // W_N1^{-(N1-1) n1}
-    const float2 wm2 = sgn<-1>(t1[(N1 - 2) * N1 + n1]);    // W_N1^{-(N1-2) n1}
-    const float2* c0 = cq + qmax;                          // c0[q] = coefficient of frequency q
+  if constexpr (H > 0) {
+    float2 w[2 * H];   // W_N1^{-k1 n1}, k1 = -H .. H - 1
+#pragma unroll
+    for (int i = 0; i < 2 * H; ++i) w[i] = sgn<-1>(t1[((i - H) & (N1 - 1)) * N1 + n1]);
+    const float2* c0 = cq + qmax;   // c0[q] = coefficient of frequency q
 #pragma unroll
     for (int k2 = 0; k2 < 32; ++k2) {
       float2 acc = k2 <= qmax ? c0[k2] : make_float2(0.f, 0.f);
-      if (k2 + 32 <= qmax) cfma(acc, c0[k2 + 32], w1);
-      if (k2 - 32 >= -qmax) cfma(acc, c0[k2 - 32], wm1);
-      if (k2 - 64 >= -qmax) cfma(acc, c0[k2 - 64], wm2);
+#pragma unroll
+      for (int i = 0; i < 2 * H; ++i) {
+        const int q = k2 + 32 * (i - H);
+        if (i != H && q <= qmax && q >= -qmax) cfma(acc, c0[q], w[i]);
+      }
       z[k2] = cmul(acc, sgn<-1>(t2[k2 * N1 + n1]));
     }
-    fft32<-1>(z);
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int k2 = 0; k2 < 32; ++k2) {
-    float2 acc = make_float2(0.f, 0.f);
-    for (int k1 = 0; k2 + 32 * k1 <= qmax; ++k1)  // q = k2 + 32 k1 >= 0
-      cfma(acc, cq[k2 + 32 * k1 + qmax], sgn<-1>(t1[k1 * N1 + n1]));
-    for (int k1 = N1 - 1; k1 > 0 && k2 + 32 * k1 >= N - qmax; --k1)  // q = k2 + 32 k1 - N < 0
-      cfma(acc, cq[k2 + 32 * k1 - N + qmax], sgn<-1>(t1[k1 * N1 + n1]));
-    z[k2] = cmul(acc, sgn<-1>(t2[k2 * N1 + n1]));
+    for (int k2 = 0; k2 < 32; ++k2) {
+      float2 acc = make_float2(0.f, 0.f);
+      for (int k1 = 0; k2 + 32 * k1 <= qmax; ++k1)  // q = k2 + 32 k1 >= 0
+        cfma(acc, cq[k2 + 32 * k1 + qmax], sgn<-1>(t1[k1 * N1 + n1]));
+      for (int k1 = N1 - 1; k1 > 0 && k2 + 32 * k1 >= N - qmax; --k1)  // q = k2 + 32 k1 - N < 0
+        cfma(acc, cq[k2 + 32 * k1 - N + qmax], sgn<-1>(t1[k1 * N1 + n1]));
+      z[k2] = cmul(acc, sgn<-1>(t2[k2 * N1 + n1]));
+    }
   }
   fft32<-1>(z);
 }
+// The H of a band of b frequencies per side (qmax = b - 1).  For N1 = 8 (N = 256) 32 H must stay below N / 2 + 1.
+__host__ __device__ constexpr int gather_blocks(int b) { return b <= 64 ? 2 : b <= 128 ? 4 : 0; }
 
 // ------------------------------------------------------------------------------ inverse, columns
 // ihat[i][jr][qc] (qr = jr - (br-1)) -> v[i][qc][y] = sum_qr ihat exp(-2 pi i qr y / ny)
-template <int N1>
-__global__ void __launch_bounds__(256, 3) fft_cols_inv_kernel(const float2* __restrict__ ihat, long long ncols, int br,
+template <int N1, int H>
+__global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_cols_inv_kernel(const float2* __restrict__ ihat, long long ncols, int br,
                                                            int bc, const float2* __restrict__ wn_g,
                                                            float2* __restrict__ v) {
   constexpr int N = 32 * N1, G = 256 / N1;
@@ -349,7 +351,7 @@ __global__ void __launch_bounds__(256, 3) fft_cols_inv_kernel(const float2* __re
   __syncthreads();
   const long long col = col0 + g;
   float2 z[32];
-  inverse_gather<N1>(z, cs + g * nq, br - 1, t2, t1, n1);
+  inverse_gather<N1, H>(z, cs + g * nq, br - 1, t2, t1, n1);
   if (col >= ncols) return;
   float2* dst = v + col * N;
 #pragma unroll
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(G * N1) cols_inv_tiles_kernel(const float2* __
   }
   __syncthreads();
   float2 z[32];
-  inverse_gather<N1>(z, cs + g * nq, br - 1, t2, t1, n1);
+  inverse_gather<N1, 2>(z, cs + g * nq, br - 1, t2, t1, n1);   // 2 br - 1 <= 128
   // z[k] is row n1 + N1 bitrev5(k): even k give the first half of the rows, odd k the second.  The rows are
   // transposed through shared memory one half at a time (half the buffer: more blocks per SM, one wave).
 #pragma unroll
@@ -444,8 +446,8 @@ static int cols_inv_tiles(const float2* ihat, int count, int br, int bc, int ny,
 
 // --------------------------------------------------------------------------------- inverse, rows
 // v[i][qc][y] (qc = 0..bc-1, qc > 0 doubled) -> out[i][y][x] = sum_qc Re(v exp(-2 pi i qc x / nx))
-template <int N1>
-__global__ void __launch_bounds__(256, 3) fft_rows_inv_kernel(const float2* __restrict__ v, long long nrows, int ny,
+template <int N1, int H>
+__global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_inv_kernel(const float2* __restrict__ v, long long nrows, int ny,
                                                            int bc, const float2* __restrict__ wn_g,
                                                            float* __restrict__ out) {
   constexpr int N = 32 * N1, G = 256 / N1;
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(256, 3) fft_rows_inv_kernel(const float2* __re
   __syncthreads();
   const long long r0 = rblk + 2 * g;
   float2 z[32];
-  inverse_gather<N1>(z, cs + g * nq, bc - 1, t2, t1, n1);
+  inverse_gather<N1, H>(z, cs + g * nq, bc - 1, t2, t1, n1);
   if (r0 >= nrows) return;
   float* o0 = out + r0 * N;
   float* o1 = o0 + N;
@@ -494,6 +496,125 @@ __global__ void __launch_bounds__(256, 3) fft_rows_inv_kernel(const float2* __re
     o0[x] = z[i].x;
     if (second) o1[x] = z[i].y;
   }
+}
+
+// ------------------------------------------------------- coarse intensity -> image columns, two passes
+// Rows: U[i][qc][sr] = sum_sc (sum_p coarse[p][i][sr][sc]) exp(+2 pi i qc sc / mc), 0 <= qc < bc, mc = 32 N1C: PAIRS row
+// pairs per block (one complex transform each), the partial sums added as the rows load, U written transposed.
+// Columns: the mr-point transform of U's column (mr = 32 N1R), its 2 br - 1 bins scaled by 1 / (mr mc), qc > 0 doubled,
+// and the ny-point inverse transform of those (ny = 32 N1) back into the same column: v[i][qc][y].
+// Bound: latency; the point of the split is blocks.  One image used to be two blocks for the whole coarse spectrum:
+// 8 images of 128 x 128, 12 parts, 59 x 59 band, 1024 rows: 20.1 (spectrum) + 8.5 (columns) us -> 5.3 + 9.5;
+// 4 of 256 x 256, 37 parts, 117 x 117 band, 2048 rows: 58 + 9.4 + 39.6 -> 7.0 + 9.7.
+constexpr int COARSE_T = 128;
+
+template <int N1C, int PAIRS>
+__global__ void __launch_bounds__(COARSE_T) coarse_rows_kernel(const float* __restrict__ coarse, int nparts,
+                                                               long long pstride, int mr, int bc,
+                                                               const float2* __restrict__ wc, int ny,
+                                                               float2* __restrict__ u) {
+  constexpr int MC = 32 * N1C, PER = 2 * PAIRS * MC / 4 / COARSE_T > 0 ? 2 * PAIRS * MC / 4 / COARSE_T : 1;
+  constexpr int LOADERS = 2 * PAIRS * MC / 4 / PER;   // threads that load (all, except for few short rows)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* img = (float*)smem_raw;                      // [2 PAIRS][MC]
+  float2* ys = (float2*)smem_raw + PAIRS * MC;        // [PAIRS][32][N1C + 1]
+  const int tid = threadIdx.x, r0 = blockIdx.x * 2 * PAIRS;
+  const long long i = blockIdx.y;
+  if (tid < LOADERS) {
+    const float4* src = (const float4*)(coarse + (i * mr + r0) * MC) + tid;
+    float4 acc[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) acc[k] = __ldg(src + LOADERS * k);
+#pragma unroll 4
+    for (int p = 1; p < nparts; ++p) {
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+        const float4 x = __ldg(src + p * (pstride / 4) + LOADERS * k);
+        acc[k].x += x.x;
+        acc[k].y += x.y;
+        acc[k].z += x.z;
+        acc[k].w += x.w;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) ((float4*)img)[tid + LOADERS * k] = acc[k];
+  }
+  __syncthreads();
+  if (tid < PAIRS * N1C) {
+    const int p = tid / N1C, n1 = tid % N1C;
+    float2 z[32];
+#pragma unroll
+    for (int n2 = 0; n2 < 32; ++n2) z[n2] = make_float2(img[2 * p * MC + n1 + N1C * n2], img[(2 * p + 1) * MC + n1 + N1C * n2]);
+    fft32<+1>(z);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const int k2 = bitrev5(k);
+      ys[(p * 32 + k2) * (N1C + 1) + n1] = cmul(z[k], __ldg(wc + ((k2 * n1) & (MC - 1))));
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < PAIRS * bc; e += COARSE_T) {
+    const int p = e % PAIRS, qc = e / PAIRS;
+    const float2* y = ys + p * 32 * (N1C + 1);
+    float2 zp = make_float2(0.f, 0.f), zm = zp;   // bins qc and -qc
+#pragma unroll
+    for (int n1 = 0; n1 < N1C; ++n1) {
+      const float2 w = __ldg(wc + ((32 * (qc >> 5) * n1) & (MC - 1)));
+      const int m = -qc & (MC - 1);
+      cfma(zp, y[(qc & 31) * (N1C + 1) + n1], w);
+      cfma(zm, y[(m & 31) * (N1C + 1) + n1], __ldg(wc + ((32 * (m >> 5) * n1) & (MC - 1))));
+    }
+    float2* o = u + (i * bc + qc) * (long long)ny + r0 + 2 * p;
+    o[0] = make_float2(0.5f * (zp.x + zm.x), 0.5f * (zp.y - zm.y));
+    o[1] = make_float2(0.5f * (zp.y + zm.y), -0.5f * (zp.x - zm.x));
+  }
+}
+
+template <int N1R, int N1, int H>
+__global__ void __launch_bounds__(COARSE_T) coarse_cols_kernel(long long ncols, int br, int bc, const float2* __restrict__ wr,
+                                                               const float2* __restrict__ wn_g, float norm, float2* v) {
+  constexpr int MR = 32 * N1R, N = 32 * N1, G = COARSE_T / N1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nq = 2 * br - 1;
+  float2* us = (float2*)smem_raw;           // [G][MR]
+  float2* ys = us + G * MR;                 // [G][32][N1R + 1]
+  float2* cs = ys + G * 32 * (N1R + 1);     // [G][nq]
+  const int tid = threadIdx.x;
+  const long long col0 = (long long)blockIdx.x * G;
+  for (int e = tid; e < G * MR; e += COARSE_T) {
+    const int g = e / MR;
+    us[e] = col0 + g < ncols ? v[(col0 + g) * N + e % MR] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  float2 z[32];
+  if (tid < G * N1R) {
+    const int g = tid / N1R, n1 = tid % N1R;
+#pragma unroll
+    for (int n2 = 0; n2 < 32; ++n2) z[n2] = us[g * MR + n1 + N1R * n2];
+    fft32<+1>(z);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const int k2 = bitrev5(k);
+      ys[(g * 32 + k2) * (N1R + 1) + n1] = cmul(z[k], __ldg(wr + ((k2 * n1) & (MR - 1))));
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < G * nq; e += COARSE_T) {
+    const int g = e / nq, jr = e - g * nq, k = (jr - (br - 1)) & (MR - 1);
+    const float2* y = ys + (g * 32 + (k & 31)) * (N1R + 1);
+    float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int n1 = 0; n1 < N1R; ++n1) cfma(a, y[n1], __ldg(wr + ((32 * (k >> 5) * n1) & (MR - 1))));
+    const float s = (col0 + g) % bc == 0 ? norm : 2.f * norm;
+    cs[e] = make_float2(a.x * s, a.y * s);
+  }
+  __syncthreads();
+  const int g = tid / N1, n1 = tid % N1;
+  if (col0 + g >= ncols) return;
+  inverse_gather<N1, H>(z, cs + g * nq, br - 1, wn_g, wn_g + 32 * N1, n1);
+  float2* dst = v + (col0 + g) * N;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) dst[n1 + N1 * bitrev5(i)] = z[i];
 }
 
 // --------------------------------------------------------------- coarse intensity -> its spectrum
@@ -654,28 +775,85 @@ static int cols_fwd(const float2* t, int batch, int bc, const float2* wn_y, int 
   return check_launch("oi_band_spectrum_fft/cols");
 }
 
-template <int N1>
-static int cols_inv(const float2* ihat, int count, int br, int bc, const float2* wn_y, float2* v, cudaStream_t s) {
+template <int N1, int H>
+static int cols_inv_h(const float2* ihat, int count, int br, int bc, const float2* wn_y, float2* v, cudaStream_t s) {
   constexpr int G = 256 / N1;
   size_t smem = sizeof(float2) * (G * (2 * br - 1));
-  int rc = set_smem(fft_cols_inv_kernel<N1>, smem, "oi_coarse_to_image_fft/cols");
+  int rc = set_smem(fft_cols_inv_kernel<N1, H>, smem, "oi_coarse_to_image_fft/cols");
   if (rc) return rc;
   const long long ncols = (long long)count * bc;
-  fft_cols_inv_kernel<N1><<<(unsigned)ceil_div(ncols, G), 256, smem, s>>>(ihat, ncols, br, bc, wn_y, v);
+  fft_cols_inv_kernel<N1, H><<<(unsigned)ceil_div(ncols, G), 256, smem, s>>>(ihat, ncols, br, bc, wn_y, v);
   oi::note_launch();
   return check_launch("oi_coarse_to_image_fft/cols");
 }
-
 template <int N1>
-static int rows_inv(const float2* v, int count, int ny, int bc, const float2* wn_x, float* out, cudaStream_t s) {
+static int cols_inv(const float2* ihat, int count, int br, int bc, const float2* wn_y, float2* v, cudaStream_t s) {
+  switch (gather_blocks(br)) {
+    case 2: return cols_inv_h<N1, 2>(ihat, count, br, bc, wn_y, v, s);
+    case 4: return cols_inv_h<N1, 4>(ihat, count, br, bc, wn_y, v, s);
+  }
+  return cols_inv_h<N1, 0>(ihat, count, br, bc, wn_y, v, s);
+}
+
+template <int N1, int H>
+static int rows_inv_h(const float2* v, int count, int ny, int bc, const float2* wn_x, float* out, cudaStream_t s) {
   constexpr int G = 256 / N1;
   size_t smem = sizeof(float2) * (bc * (2 * G + 1) + G * (2 * bc - 1));
-  int rc = set_smem(fft_rows_inv_kernel<N1>, smem, "oi_coarse_to_image_fft/rows");
+  int rc = set_smem(fft_rows_inv_kernel<N1, H>, smem, "oi_coarse_to_image_fft/rows");
   if (rc) return rc;
   const long long nrows = (long long)count * ny;
-  fft_rows_inv_kernel<N1><<<(unsigned)ceil_div(nrows, 2 * G), 256, smem, s>>>(v, nrows, ny, bc, wn_x, out);
+  fft_rows_inv_kernel<N1, H><<<(unsigned)ceil_div(nrows, 2 * G), 256, smem, s>>>(v, nrows, ny, bc, wn_x, out);
   oi::note_launch();
   return check_launch("oi_coarse_to_image_fft/rows");
+}
+template <int N1>
+static int rows_inv(const float2* v, int count, int ny, int bc, const float2* wn_x, float* out, cudaStream_t s) {
+  switch (gather_blocks(bc)) {
+    case 2: return rows_inv_h<N1, 2>(v, count, ny, bc, wn_x, out, s);
+    case 4: return rows_inv_h<N1, 4>(v, count, ny, bc, wn_x, out, s);
+  }
+  return rows_inv_h<N1, 0>(v, count, ny, bc, wn_x, out, s);
+}
+
+// Coarse intensity (nparts partial sums of [count][32 N1R][32 N1C]) -> v, the first two passes of the synthesis; v holds
+// count * bc columns of ny >= 32 N1R complex values and carries U between the two (same column, its first 32 N1R values).
+template <int N1C>
+static int coarse_rows(const float* coarse, int nparts, int count, int mr, int bc, const float2* wc, int ny, float2* v,
+                       cudaStream_t s) {
+  constexpr int MC = 32 * N1C;
+  auto run = [&](auto kern, int pairs) {
+    const size_t smem = sizeof(float2) * ((size_t)pairs * MC + pairs * 32 * (N1C + 1));
+    if (int rc = set_smem(kern, smem, "coarse rows fft")) return rc;
+    kern<<<dim3((unsigned)(mr / (2 * pairs)), (unsigned)count), COARSE_T, smem, s>>>(
+        coarse, nparts, (long long)count * mr * MC, mr, bc, wc, ny, v);
+    oi::note_launch();
+    return check_launch("coarse rows fft");
+  };
+  // 16 rows per block write whole 128-byte lines; 8 or 4 rows while that leaves SMs (148) without a block
+  if ((long long)count * mr / 16 >= 148) return run(coarse_rows_kernel<N1C, 8>, 8);
+  if ((long long)count * mr / 8 >= 148) return run(coarse_rows_kernel<N1C, 4>, 4);
+  return run(coarse_rows_kernel<N1C, 2>, 2);
+}
+template <int N1R, int N1, int H>
+static int coarse_cols_h(int count, int br, int bc, const float2* wr, const float2* wn_y, float2* v, float norm, cudaStream_t s) {
+  constexpr int G = COARSE_T / N1, MR = 32 * N1R;
+  const size_t smem = sizeof(float2) * ((size_t)G * MR + G * 32 * (N1R + 1) + G * (2 * br - 1));
+  auto kern = coarse_cols_kernel<N1R, N1, H>;
+  if (int rc = set_smem(kern, smem, "coarse columns fft")) return rc;
+  kern<<<(unsigned)ceil_div((long long)count * bc, G), COARSE_T, smem, s>>>((long long)count * bc, br, bc, wr, wn_y, norm, v);
+  oi::note_launch();
+  return check_launch("coarse columns fft");
+}
+template <int N1R>
+static int coarse_cols(int count, int br, int bc, const float2* wr, const float2* wn_y, int ny1, float2* v, float norm,
+                       cudaStream_t s) {
+  constexpr int H = N1R == 8 ? 4 : 2;   // 2 br - 1 <= 32 N1R
+  switch (ny1) {
+    case 8: return coarse_cols_h<N1R, 8, H>(count, br, bc, wr, wn_y, v, norm, s);
+    case 16: return coarse_cols_h<N1R, 16, H>(count, br, bc, wr, wn_y, v, norm, s);
+    case 32: return coarse_cols_h<N1R, 32, H>(count, br, bc, wr, wn_y, v, norm, s);
+  }
+  return coarse_cols_h<N1R, 64, H>(count, br, bc, wr, wn_y, v, norm, s);
 }
 
 static int n1_of(int n) {
@@ -774,20 +952,31 @@ extern "C" int oi_coarse_to_image_fft(float* coarse, int nparts, int count, int 
   if (2 * br - 1 > ny || 2 * bc - 1 > nx) return fail(OI_ERANGE, "oi_coarse_to_image_fft: band too wide for grid");
   cudaStream_t s = (cudaStream_t)stream;
   int rc;
-  if (wm_r && wm_c && (mr == 64 || mr == 128) && (mc == 64 || mc == 128) && bc <= 64) {
-    float2* ih = (float2*)scratch_ihat;
+  float2* v = (float2*)scratch_v;
+  auto small = [](int m) { return m == 64 || m == 128 || m == 256; };
+  if (wm_r && wm_c && small(mr) && small(mc) && mr <= ny && 2 * br - 1 <= mr && 2 * bc - 1 <= mc && count <= 65535) {
     const float2 *tr = (const float2*)wm_r, *tc = (const float2*)wm_c;
-    if (mr == 128 && mc == 128) rc = launch_coarse_spec_fft<4, 4>(coarse, nparts, count, br, bc, tr, tc, ih, s);
-    else if (mr == 64 && mc == 64) rc = launch_coarse_spec_fft<2, 2>(coarse, nparts, count, br, bc, tr, tc, ih, s);
-    else if (mr == 128) rc = launch_coarse_spec_fft<4, 2>(coarse, nparts, count, br, bc, tr, tc, ih, s);
-    else rc = launch_coarse_spec_fft<2, 4>(coarse, nparts, count, br, bc, tr, tc, ih, s);
-  } else {
-    rc = coarse_spectrum(coarse, count, mr, mc, br, bc, gc, gr, scratch_ihat, s, nparts, scratch_v,
-                         (long long)count * bc * ny * (long long)sizeof(float2));
+    rc = mc == 64    ? coarse_rows<2>(coarse, nparts, count, mr, bc, tc, ny, v, s)
+         : mc == 128 ? coarse_rows<4>(coarse, nparts, count, mr, bc, tc, ny, v, s)
+                     : coarse_rows<8>(coarse, nparts, count, mr, bc, tc, ny, v, s);
+    if (rc) return rc;
+    const float norm = 1.0f / ((float)mr * (float)mc);
+    const float2* wy = (const float2*)wn_y;
+    rc = mr == 64    ? coarse_cols<2>(count, br, bc, tr, wy, ny1, v, norm, s)
+         : mr == 128 ? coarse_cols<4>(count, br, bc, tr, wy, ny1, v, norm, s)
+                     : coarse_cols<8>(count, br, bc, tr, wy, ny1, v, norm, s);
+    if (rc) return rc;
+    switch (nx1) {
+      case 8: return rows_inv<8>(v, count, ny, bc, (const float2*)wn_x, out, s);
+      case 16: return rows_inv<16>(v, count, ny, bc, (const float2*)wn_x, out, s);
+      case 32: return rows_inv<32>(v, count, ny, bc, (const float2*)wn_x, out, s);
+      default: return rows_inv<64>(v, count, ny, bc, (const float2*)wn_x, out, s);
+    }
   }
+  rc = coarse_spectrum(coarse, count, mr, mc, br, bc, gc, gr, scratch_ihat, s, nparts, scratch_v,
+                       (long long)count * bc * ny * (long long)sizeof(float2));
   if (rc) return rc;
   const float2* ih = (const float2*)scratch_ihat;
-  float2* v = (float2*)scratch_v;
   switch (ny1) {
     case 8: rc = cols_inv<8>(ih, count, br, bc, (const float2*)wn_y, v, s); break;
     case 16: rc = cols_inv<16>(ih, count, br, bc, (const float2*)wn_y, v, s); break;

@@ -114,7 +114,8 @@ class Plan:
             self.wn_y = fft_tables(ny, device)
         self.coarse_fft = self.mr in (64, 128) and self.mc in (64, 128)
         self.coarse256 = (self.mr, self.mc) == (256, 256)     # the tensor-memory accumulator kernel
-        if self.coarse_fft or self.coarse256:                 # the coarse-grid FFT tables
+        self.coarse_small = self.mr in (64, 128, 256) and self.mc in (64, 128, 256)
+        if self.coarse_small:                                 # the coarse-grid FFT tables
             self.wm_r = t(1, self.mr, 1, 0, self.mr, +1)
             self.wm_c = t(1, self.mc, 1, 0, self.mc, +1)
 
@@ -175,7 +176,8 @@ class Plan:
         return t
 
     def big_coarse_fft(self, form) -> bool:
-        """Coarse grids above 128 (bands over 64) on FFT output grids: the coarse spectrum by the FFT band pass."""
+        """Coarse grids above 128 (bands over 64) on FFT output grids: the coarse spectrum by FFTs (the FFT band pass, or,
+        for 256 per axis, the synthesis's own row and column passes)."""
         lib = N.load()
         return (form != 'dft' and self.fft and not self.coarse_fft and lib.oi_fft_supported(self.mr, self.mc) == 1
                 and 2 * (self.band.bc - 1) < self.mc and 2 * self.band.br - 1 <= self.mr)
@@ -334,7 +336,7 @@ def coherent_image(band: torch.Tensor, pupils: torch.Tensor, weights: torch.Tens
         tiles = torch.empty(batch * nz * plan.ny * 512, dtype=torch.uint8, device=dev)
         N.call('oi_coarse_to_image_tcs', N.ptr(coarse), nsplit, batch * nz, b.br, b.bc, N.ptr(plan.synth_consts()),
                N.ptr(plan.rows_consts(1)), plan.ny, plan.nx, N.ptr(tiles), N.ptr(out), s)
-    elif plan.big_coarse_fft(form):
+    elif plan.big_coarse_fft(form) and not plan.coarse_small:
         # the coarse intensity's Hermitian half-spectrum by the FFT band pass, then the FFT synthesis
         count = batch * nz
         wn_r, wn_c = plan.coarse_fft_tables()
@@ -346,7 +348,7 @@ def coherent_image(band: torch.Tensor, pupils: torch.Tensor, weights: torch.Tens
                plan.ny, plan.nx, N.ptr(v), N.ptr(out), s)
     elif plan.use_fft(form):
         v = torch.empty(batch * nz * b.bc * plan.ny, dtype=torch.complex64, device=dev)
-        wm_r, wm_c = (plan.wm_r, plan.wm_c) if plan.coarse_fft else (None, None)
+        wm_r, wm_c = (plan.wm_r, plan.wm_c) if plan.coarse_small else (None, None)
         N.call('oi_coarse_to_image_fft', N.ptr(coarse), nsplit, batch * nz, plan.mr, plan.mc, b.br, b.bc,
                N.ptr(plan.gc), N.ptr(plan.gr), N.ptr(wm_r), N.ptr(wm_c), N.ptr(plan.wn_y), N.ptr(plan.wn_x),
                plan.ny, plan.nx, N.ptr(ihat), N.ptr(v), N.ptr(out), s)
