@@ -5,6 +5,7 @@
 // For one (image b, plane z, subset of fields), each field A = P[z][k] .* band[b][c] (Br x Bc, on the band)
 // is taken to the Mr x Mc coarse grid by a 2-D inverse transform
 //   E[sr][sc] = sum_{ir,ic} A[ir][ic] exp(-2 pi i ((m0r+ir) sr/Mr + (m0c+ic) sc/Mc))
+// (up to the phase of the band's offset, which |E|^2 does not see)
 // done as Br pruned row FFTs (Mc points, only Bc inputs non-zero) into shared memory, then Mc pruned column
 // FFTs (Mr points, only Br inputs non-zero).  Each thread owns one column task (sc, n1) for the whole field
 // loop and accumulates w |E|^2 of its 32 outputs in registers, so E never leaves the SM.  Every FFT is the
@@ -19,7 +20,6 @@
 namespace oi {
 
 using cg::brev5;
-using cg::gather_ifft;
 using cg::ifft32;
 
 struct CoherentFftArgs {
@@ -37,52 +37,65 @@ struct CoherentFftArgs {
 };
 
 // grid (nsplit, nz, batch); block = mc * N1R threads (column tasks); mr = 32 N1R, mc = 32 N1C.
+// Bound: FP32 and shared-memory issue, and latency where a block has one field.  With the band at frequency 0 (fft_common)
+// a gather term is one load and one complex FMA (64 a transform of 128 points); with the band in place it was 128 tests,
+// and twiddles read by computed index: one field a block, 96 blocks, 128 x 128: 17.0 -> 11.3 us.
 template <int N1R, int N1C>
 __global__ void __launch_bounds__(32 * N1C * N1R) coherent_fft_kernel(CoherentFftArgs a) {
-  constexpr int MR = 32 * N1R, MC = 32 * N1C, T = MC * N1R;
+  using R = cg::Axis<N1R>;
+  using C = cg::Axis<N1C>;
+  constexpr int T = C::M * N1R, WARPS = T / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* wr = (float2*)smem_raw;   // [MR]
-  float2* wc = wr + MR;             // [MC]
-  float2* as = wc + MC;             // [br][bc]
-  float2* e1 = as + a.br * a.bc;    // [br][MC + 1] (padded against bank conflicts)
-  const int tid = threadIdx.x;
-  const int split = blockIdx.x, z = blockIdx.y;
+  float2* twr = (float2*)smem_raw;         // [32][N1R]
+  float2* twc = twr + 32 * N1R;            // [32][N1C]
+  float2* as = twc + 32 * N1C;             // [R::B][C::BAND_LD]  the field on the band, columns zero beyond bc
+  float2* e1 = as + R::B * C::BAND_LD;     // [R::B][C::FIELD_LD] its rows transformed, rows zero beyond br
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int split = blockIdx.x, z = blockIdx.y, br = a.br, bc = a.bc;
   const long long b = blockIdx.z;
-  for (int j = tid; j < MR; j += T) wr[j] = a.wr[j];
-  for (int j = tid; j < MC; j += T) wc[j] = a.wc[j];
-  const int sc = tid % MC, n1r = tid / MC;  // column task of this thread
+  cg::build_twiddles<N1R>(twr, a.wr, tid, T);
+  cg::build_twiddles<N1C>(twc, a.wc, tid, T);
+  for (int j = br * C::FIELD_LD + tid; j < R::B * C::FIELD_LD; j += T) e1[j] = make_float2(0.f, 0.f);
+  const int sc = tid % C::M, n1r = tid / C::M;  // column task of this thread
   float acc[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) acc[i] = 0.f;
   const int nfield = a.nk * a.nch;
-  const long long plane = (long long)a.br * a.bc;
+  const long long plane = (long long)br * bc;
   const float2* pup = a.pupil + b * a.pupil_batch_stride + (long long)z * a.nk * plane;
   for (int f = split; f < nfield; f += a.nsplit) {
     const int k = f / a.nch, c = f % a.nch;
     const float w = __ldg(a.weight + (long long)z * a.nk + k);
     const float2* pk = pup + (long long)k * plane;
     const float2* hc = a.band + b * a.band_img_stride + (long long)c * plane;
-    __syncthreads();  // previous field's readers are done with as / e1; tables are loaded
-    for (long long e = tid; e < plane; e += T) as[e] = cmul(__ldg(pk + e), __ldg(hc + e));
-    __syncthreads();
-    // row pass: br rows x N1C tasks, Mc-point transforms of the bc band columns
-    for (int task = tid; task < a.br * N1C; task += T) {
-      const int ir = task / N1C, n1 = task % N1C;
-      float2 zr[32];
-      gather_ifft<N1C>(zr, as + ir * a.bc, 1, a.m0c, a.bc, wc, n1);
+    // (the previous field's rows are read; its columns are read before the barrier after the row pass)
+#pragma unroll 2
+    for (int ir = warp; ir < br; ir += WARPS) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) e1[ir * (MC + 1) + n1 + N1C * brev5(i)] = zr[i];
+      for (int u = 0; u < C::B / 32; ++u) {
+        const int ic = lane + 32 * u;
+        as[ir * C::BAND_LD + ic] = ic < bc ? cmul(__ldg(pk + ir * bc + ic), __ldg(hc + ir * bc + ic)) : make_float2(0.f, 0.f);
+      }
     }
     __syncthreads();
-    // column pass: thread (sc, n1r), Mr-point transform of the br band rows of column sc
+    // row pass: br rows x N1C tasks
+    for (int task = tid; task < br * N1C; task += T) {
+      const int ir = task / N1C, n1 = task % N1C;
+      float2 zr[32];
+      cg::band_ifft<N1C>(zr, as + ir * C::BAND_LD, 1, twc, n1);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) e1[ir * C::FIELD_LD + n1 + N1C * brev5(i)] = zr[i];
+    }
+    __syncthreads();
+    // column pass: thread (sc, n1r)
     float2 zc[32];
-    gather_ifft<N1R>(zc, e1 + sc, MC + 1, a.m0r, a.br, wr, n1r);
+    cg::band_ifft<N1R>(zc, e1 + sc, C::FIELD_LD, twr, n1r);
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = fmaf(w, fmaf(zc[i].x, zc[i].x, zc[i].y * zc[i].y), acc[i]);
   }
-  float* out = a.coarse + split * a.split_stride + ((b * a.nz + z) * (long long)MR) * MC;
+  float* out = a.coarse + split * a.split_stride + ((b * a.nz + z) * (long long)R::M) * C::M;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) out[(n1r + N1R * brev5(i)) * MC + sc] = acc[i];
+  for (int i = 0; i < 32; ++i) out[(n1r + N1R * brev5(i)) * C::M + sc] = acc[i];
 }
 
 // ---- 256 x 256 coarse grid (bands of 65..128 per axis): the |E|^2 accumulator in tensor memory.
@@ -227,8 +240,10 @@ static int launch_cfft256(const CoherentFftArgs& a, int batch, cudaStream_t s) {
 
 template <int N1R, int N1C>
 static int launch_cfft(const CoherentFftArgs& a, int batch, cudaStream_t s) {
-  constexpr int MR = 32 * N1R, MC = 32 * N1C, T = MC * N1R;
-  size_t smem = sizeof(float2) * ((size_t)MR + MC + (size_t)a.br * a.bc + (size_t)a.br * (MC + 1));
+  using R = cg::Axis<N1R>;
+  using C = cg::Axis<N1C>;
+  constexpr int T = C::M * N1R;
+  const size_t smem = sizeof(float2) * (32 * (N1R + N1C) + (size_t)R::B * (C::BAND_LD + C::FIELD_LD));
   auto kern = coherent_fft_kernel<N1R, N1C>;
   {
     int rc_smem = ensure_smem((const void*)kern, smem, "oi_coherent_coarse_fft");

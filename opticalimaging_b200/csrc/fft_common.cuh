@@ -20,8 +20,9 @@ __host__ __device__ constexpr int brev5(int i) {
   return ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2) | ((i & 16) >> 4);
 }
 
-// 32-point DFT with exp(-2 pi i k n / 32) in registers, decimation in frequency: v[i] = X[brev5(i)].
-__device__ __forceinline__ void ifft32(float2 (&v)[32]) {
+// 32-point DFT with exp(SIGN 2 pi i k n / 32) in registers, decimation in frequency: v[i] = X[brev5(i)].
+template <int SIGN>
+__device__ __forceinline__ void dft32(float2 (&v)[32]) {
 #pragma unroll
   for (int len = 32; len >= 2; len >>= 1) {
     const int half = len >> 1, step = 32 / len;
@@ -36,14 +37,49 @@ __device__ __forceinline__ void ifft32(float2 (&v)[32]) {
         if (t == 0) {
           v[blk + j + half] = d;
         } else if (t == 8) {
-          v[blk + j + half] = make_float2(d.y, -d.x);  // * (-i)
+          v[blk + j + half] = SIGN > 0 ? make_float2(-d.y, d.x) : make_float2(d.y, -d.x);  // * (+-i)
         } else {
-          const float c = c32(t), s = -s32(t);
+          const float c = c32(t), s = SIGN * s32(t);
           v[blk + j + half] = make_float2(d.x * c - d.y * s, d.x * s + d.y * c);
         }
       }
     }
   }
+}
+__device__ __forceinline__ void ifft32(float2 (&v)[32]) { dft32<-1>(v); }
+
+// The coarse grids' geometry (M = 32 N1, 64 or 128 points per axis).  A band of b frequencies fits when 2 b - 1 <= M,
+// so b <= B = 16 N1; its offset only turns the phase of the field, E[s] = exp(-2 pi i m0 s / M) E0[s] with E0 the
+// transform of the band placed at frequency 0, and neither |E|^2 nor the adjoint's products see that phase.  With the
+// band at 0 and zeros up to B, the four-step gather of an output is N1 / 2 terms with no bounds to check.
+template <int N1> struct Axis {
+  static constexpr int M = 32 * N1, B = 16 * N1;
+  static constexpr int BAND_LD = B + 2;     // row of a band array: eight rows' values fall on eight bank pairs
+  static constexpr int FIELD_LD = M + N1;   // row of a row-transformed array: as many rows as a half warp holds
+};
+
+// tw[t][n1] = exp(-2 pi i t n1 / M), 32 x N1, from w[j] = exp(+2 pi i j / M).
+template <int N1>
+__device__ __forceinline__ void build_twiddles(float2* tw, const float2* w, int tid, int nthreads) {
+  for (int e = tid; e < 32 * N1; e += nthreads) {
+    const float2 t = __ldg(w + (((e / N1) * (e % N1)) & (32 * N1 - 1)));
+    tw[e] = make_float2(t.x, -t.y);
+  }
+}
+
+// Thread n1 of N1: z[i] = X[n1 + N1 brev5(i)], X[s] = sum_{j < 16 N1} src[j * stride] exp(-2 pi i j s / M).
+template <int N1>
+__device__ __forceinline__ void band_ifft(float2 (&z)[32], const float2* src, int stride, const float2* tw, int n1) {
+  static_assert(N1 == 2 || N1 == 4, "coarse grids of 64 or 128");
+  // W_4^{-n1}: 1, -i, -1, i
+  const float2 w1 = make_float2(n1 == 0 ? 1.f : n1 == 2 ? -1.f : 0.f, n1 == 1 ? -1.f : n1 == 3 ? 1.f : 0.f);
+#pragma unroll
+  for (int t = 0; t < 32; ++t) {
+    float2 acc = src[t * stride];
+    if (N1 == 4) cfma(acc, src[(t + 32) * stride], w1);
+    z[t] = t == 0 ? acc : cmul(acc, tw[t * N1 + n1]);
+  }
+  ifft32(z);
 }
 
 // Inverse four-step for an M = 32 N1 point transform of a band-limited input: thread n1 forms

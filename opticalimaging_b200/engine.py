@@ -16,6 +16,7 @@ grid FFT evaluation index for index.
 from __future__ import annotations
 
 import collections
+import functools
 import math
 import threading
 from dataclasses import dataclass
@@ -241,10 +242,15 @@ def field_split(nfields: int, blocks: int, sms: int | None = None) -> int:
 
 
 def field_split_sm(nfields: int, blocks: int, sms: int | None = None) -> int:
-    """Field split for a kernel of one block per SM (the 256 x 256 coarse grid): the d minimising
+    """Field split for a kernel of one block per SM (the FFT coherent sums and the adjoint): the d minimising
     waves(d) * (fields per block + 1/2), the half standing for a block's fixed start and partial-sum write;
-    ties go to the smaller d (fewer partial sums)."""
-    sms = sm_count() if sms is None else sms
+    ties go to the smaller d (fewer partial sums).  64 images of 12 fields: 2 blocks an image, 6 fields each, in one
+    wave; as many waves as fields allow (field_split) took 12 blocks of one field in 5.2 waves."""
+    return _field_split_sm(nfields, blocks, sm_count() if sms is None else sms)
+
+
+@functools.lru_cache(maxsize=1024)
+def _field_split_sm(nfields: int, blocks: int, sms: int) -> int:
     best, best_cost = 1, None
     for d in range(1, nfields + 1):
         cost = -(-blocks * d // sms) * (-(-nfields // d) + 0.5)
@@ -316,7 +322,7 @@ def coherent_image(band: torch.Tensor, pupils: torch.Tensor, weights: torch.Tens
                int(pupil_batch_stride), N.ptr(weights), nz, nk, N.ptr(plan.tc_constants()), ctas, nsplit,
                N.ptr(coarse), s)
     elif plan.use_coarse_fft(form) or plan.use_coarse256(form):
-        nsplit = (field_split_sm(nk * nch, batch * nz) if plan.coarse256 else field_split(nk * nch, batch * nz))
+        nsplit = field_split_sm(nk * nch, batch * nz)
         coarse = torch.empty((nsplit, batch, nz, plan.mr, plan.mc), dtype=torch.float32, device=dev)
         N.call('oi_coherent_coarse_fft', N.ptr(band), batch, nch, b.m0r, b.br, b.m0c, b.bc, N.ptr(pupils),
                int(pupil_batch_stride), N.ptr(weights), nz, nk, plan.mr, plan.mc, N.ptr(plan.wm_r),
@@ -505,8 +511,7 @@ class CoherentModel:
         b, p = self.band, self.plan
         nz = self.planes
         form = self.form if form is None else form
-        split = (field_split(self.count * nch, batch * nz) if p.use_coarse_fft(None)
-                 else field_split_sm(self.count * nch, batch * nz) if p.use_coarse256(form)
+        split = (field_split_sm(self.count * nch, batch * nz) if p.use_coarse_fft(None) or p.use_coarse256(form)
                  else field_split(self.count * nch, batch * nz * ((p.mr + 15) // 16)))
         if form == 'bf16x3':
             split = tc_parts_bound(batch * nz, self.count * nch)
