@@ -332,6 +332,20 @@ OI_API int oi_coherent_adjoint(const void* band, int batch, int nch, int m0r, in
                                int mc, const void* wr, const void* wc, int nsplit, void* wout, float* field_dot,
                                void* stream);
 
+/* The field dots of oi_coherent_adjoint alone (field_dot as there). */
+OI_API int oi_coherent_field_dots(const void* band, int batch, int nch, int m0r, int br, int m0c, int bc,
+                                  const void* pupil, const float* weight, int nz, int nk, const float* gcoarse, int mr, int mc,
+                                  const void* wr, const void* wc, int nsplit, float* field_dot, void* stream);
+
+/*
+ * The Hermitian half-spectrum of Re sum_m W(m) exp(-2 pi i m.y/N): W the sum of nparts x nz bands (w complex64
+ * [nparts][batch][nz][br][bc], as oi_coherent_adjoint writes them for one channel), half complex64
+ * [batch][2R+1][C+1], R and C the band's largest |frequency| per axis,
+ *   half[b][qr + R][qc] = scale (qc ? 2 : 1) (W(q) + conj W(-q)) / 2      -- an input of oi_spectrum_to_image(_fft).
+ */
+OI_API int oi_hermitian_half(const void* w, int nparts, int batch, int nz, int m0r, int br, int m0c, int bc, float scale,
+                             void* half, void* stream);
+
 /*
  * Shifted pupil matrix of the TCC (CalculateTCCMatrix.py:17-51), FP64, scaled for a Gram product:
  *   h[e][p][j] = sqrt(index_image * v[j] / weight_sum) * valid * obliquity * exp(2 pi i W) * defocus * transfer_e

@@ -36,6 +36,8 @@ _SIGS = {
     'oi_spectrum_to_image_fft': [_vp, _i, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp],
     'oi_coherent_adjoint': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _vp,
                             _vp],
+    'oi_coherent_field_dots': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _vp],
+    'oi_hermitian_half': [_vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
     'oi_band_spectrum_noalloc': [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp],
     'oi_coherent_coarse_fft': [_vp, _i, _i, _i, _i, _i, _i, _vp, _ll, _vp, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp],
     'oi_coherent_tc_layout': [_ll, _i, _vp, _vp],

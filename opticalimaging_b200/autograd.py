@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 
 from . import _native as N
-from .engine import Band, CoherentModel, Plan, band_spectrum, field_split
+from .engine import Band, CoherentModel, Plan, band_spectrum, coherent_image, field_split_sm
 
 
 def _half_spectrum_to_image(ihat: torch.Tensor, br: int, bc: int, ny: int, nx: int) -> torch.Tensor:
@@ -52,42 +52,79 @@ def adjoint_plan(model: CoherentModel) -> Plan:
 def coarse_gradient(model: CoherentModel, g: torch.Tensor) -> torch.Tensor:
     """The band-limited coarse copy g^c [B, Z, Mr, Mc] of g = dL/dI [B, Z, ny, nx]:
     g^c(s) = 1/(Mr Mc) sum_{|qr|<br, |qc|<bc} ghat(q) exp(-2 pi i q.s/M), ghat(q) = sum_r g(r) exp(+2 pi i q.r/N)."""
+    plan = adjoint_plan(model)
+    return _coarse_gradient(model, g, 1.0 / (plan.mr * plan.mc))
+
+
+def _coarse_gradient(model: CoherentModel, g: torch.Tensor, scale: float) -> torch.Tensor:
+    """scale * sum_q ghat(q) exp(-2 pi i q.s/M) on the adjoint's coarse grid."""
     b, plan = model.band, adjoint_plan(model)
     B, Z = g.shape[0], g.shape[1]
+    ny, nx = model.ny, model.nx
     ib = Band(-(b.br - 1), 2 * b.br - 1, 0, b.bc)                     # image band, Hermitian half in x
-    gplan = Plan.get(model.ny, model.nx, ib, model.device)
-    gh = band_spectrum(g.reshape(B * Z, model.ny, model.nx).contiguous(), N.FIELD_REAL_F32, gplan,
-                       scale=float(model.ny * model.nx))[:, 0]          # [B*Z, 2br-1, bc], ghat(q)
-    gh = gh * (1.0 / (plan.mr * plan.mc))
-    gh[:, :, 1:] *= 2.0
+    gplan = Plan.get(ny, nx, ib, model.device)
+    g = g.reshape(B * Z, ny, nx).contiguous()
+    if gplan.fft:   # the half-spectrum with qc > 0 doubled, 1 / (ny nx) folded out of the last scale
+        t = torch.empty(B * Z * ny * b.bc, dtype=torch.complex64, device=model.device)
+        gh = torch.empty((B * Z, 2 * b.br - 1, b.bc), dtype=torch.complex64, device=model.device)
+        N.call('oi_coarse_half_spectrum_fft', N.ptr(g), 1, B * Z, ny, nx, b.br, b.bc, N.ptr(gplan.wn_x),
+               N.ptr(gplan.wn_y), N.ptr(t), N.ptr(gh), N.stream_handle(model.device))
+        if scale * ny * nx != 1.0:
+            gh = gh * (scale * ny * nx)
+    else:
+        gh = band_spectrum(g, N.FIELD_REAL_F32, gplan, scale=scale * ny * nx)[:, 0]   # [B*Z, 2br-1, bc]
+        gh[:, :, 1:] *= 2.0
     return _half_spectrum_to_image(gh, b.br, b.bc, plan.mr, plan.mc).view(B, Z, plan.mr, plan.mc)
+
+
+def _adjoint_shares(model: CoherentModel, band: torch.Tensor, gc: torch.Tensor, pupils, weights):
+    """W in shares [nsplit, B, Z, nch, br, bc] over the fields `pupils` [Z, K, br, bc] weighted by `weights`."""
+    b, plan = model.band, adjoint_plan(model)
+    B, nch = band.shape[0], band.shape[1]
+    Z, K = pupils.shape[0], pupils.shape[1]
+    nsplit = field_split_sm(K * nch, B * Z)
+    wout = torch.empty((nsplit, B, Z, nch, b.br, b.bc), dtype=torch.complex64, device=model.device)
+    N.call('oi_coherent_adjoint', N.ptr(band), B, nch, b.m0r, b.br, b.m0c, b.bc, N.ptr(pupils), N.ptr(weights), Z, K,
+           N.ptr(gc), plan.mr, plan.mc, N.ptr(plan.wm_r), N.ptr(plan.wm_c), nsplit, N.ptr(wout), None,
+           N.stream_handle(model.device))
+    return wout
+
+
+def _field_dots(model: CoherentModel, band: torch.Tensor, gc: torch.Tensor) -> torch.Tensor:
+    """<g, |E_f|^2> of every field f of the model: [B, Z, K*nch]."""
+    b, plan = model.band, adjoint_plan(model)
+    B, nch = band.shape[0], band.shape[1]
+    Z, K = model.planes, model.count
+    nsplit = field_split_sm(K * nch, B * Z)
+    gc = gc.contiguous()
+    dots = torch.empty((B, Z, K * nch), dtype=torch.float32, device=model.device)
+    N.call('oi_coherent_field_dots', N.ptr(band), B, nch, b.m0r, b.br, b.m0c, b.bc, N.ptr(model.pupils),
+           N.ptr(model.weights), Z, K, N.ptr(gc), plan.mr, plan.mc, N.ptr(plan.wm_r), N.ptr(plan.wm_c), nsplit, N.ptr(dots),
+           N.stream_handle(model.device))
+    return dots
 
 
 def coherent_adjoint(model: CoherentModel, band: torch.Tensor, gc: torch.Tensor, field_dots: bool = False):
     """W [B, nch, br, bc] (summed over planes) and, optionally, field dots [B, Z, K*nch]."""
-    b, plan = model.band, adjoint_plan(model)
-    B, nch = band.shape[0], band.shape[1]
-    Z, K = model.planes, model.count
-    nsplit = field_split(K * nch, B * Z)
-    wout = torch.empty((nsplit, B, Z, nch, b.br, b.bc), dtype=torch.complex64, device=model.device)
-    dots = torch.empty((B, Z, K * nch), dtype=torch.float32, device=model.device) if field_dots else None
-    N.call('oi_coherent_adjoint', N.ptr(band), B, nch, b.m0r, b.br, b.m0c, b.bc, N.ptr(model.pupils),
-           N.ptr(model.weights), Z, K, N.ptr(gc.contiguous()), plan.mr, plan.mc, N.ptr(plan.wm_r),
-           N.ptr(plan.wm_c), nsplit, N.ptr(wout), N.ptr(dots), N.stream_handle(model.device))
-    return wout.sum(dim=(0, 2)), dots
+    gc = gc.contiguous()
+    w = _adjoint_shares(model, band, gc, model.pupils, model.weights).sum(dim=(0, 2))
+    return w, (_field_dots(model, band, gc) if field_dots else None)
 
 
 def mask_gradient_from_w(model: CoherentModel, w: torch.Tensor) -> torch.Tensor:
     """dL/dt [B, ny, nx] = 2/(ny nx) Re sum_{m in band} W(m) exp(-2 pi i m.y/N) for W [B, br, bc]."""
+    return _mask_gradient(model, w.contiguous()[None, :, None], 2.0 / (model.ny * model.nx))
+
+
+def _mask_gradient(model: CoherentModel, shares: torch.Tensor, scale: float) -> torch.Tensor:
+    """scale Re sum_m W(m) exp(-2 pi i m.y/N) [B, ny, nx], W the sum of shares [n, B, Z, br, bc] over n and Z."""
     b = model.band
-    B = w.shape[0]
+    n, B, Z = shares.shape[0], shares.shape[1], shares.shape[2]
     R = max(abs(b.m0r), abs(b.m0r + b.br - 1))
     C = max(abs(b.m0c), abs(b.m0c + b.bc - 1))
-    full = torch.zeros((B, 2 * R + 1, 2 * C + 1), dtype=torch.complex64, device=w.device)
-    full[:, b.m0r + R: b.m0r + R + b.br, b.m0c + C: b.m0c + C + b.bc] = w
-    herm = 0.5 * (full + torch.conj(torch.flip(full, dims=(1, 2))))       # H(q) = (W(q) + conj W(-q)) / 2
-    half = herm[:, :, C:] * (2.0 / (model.ny * model.nx))
-    half[:, :, 1:] *= 2.0
+    half = torch.empty((B, 2 * R + 1, C + 1), dtype=torch.complex64, device=shares.device)
+    N.call('oi_hermitian_half', N.ptr(shares), n, B, Z, b.m0r, b.br, b.m0c, b.bc, float(scale), N.ptr(half),
+           N.stream_handle(model.device))
     return _half_spectrum_to_image(half, R + 1, C + 1, model.ny, model.nx)
 
 
@@ -95,19 +132,27 @@ class _CoherentImage(torch.autograd.Function):
     @staticmethod
     def forward(ctx, mask, model):
         ctx.model = model
-        ctx.save_for_backward(mask)
         with torch.no_grad():
-            return CoherentModel.image(model, mask.detach().contiguous())   # [B, Z, ny, nx] for every model
+            m = mask.detach().contiguous()
+            band = band_spectrum(m, N.FIELD_REAL_F32, model.plan, form=model.form)
+            image = coherent_image(band, *model.fields_for(N.FIELD_REAL_F32), model.plan, form=model.form)
+        # the backward pass starts from the FP32 band spectrum: the forward's own, unless that ran in split form
+        ctx.save_for_backward(mask, band if model.form in (None, 'fft') else None)
+        return image                                                        # [B, Z, ny, nx] for every model
 
     @staticmethod
     def backward(ctx, g):
-        (mask,) = ctx.saved_tensors
+        mask, band = ctx.saved_tensors
         model = ctx.model
         with torch.no_grad():
-            band = band_spectrum(mask.detach().contiguous(), N.FIELD_REAL_F32, model.plan)
-            gc = coarse_gradient(model, g.to(torch.float32).contiguous())
-            w, _ = coherent_adjoint(model, band, gc)
-            grad = mask_gradient_from_w(model, w[:, 0])
+            if band is None:
+                band = band_spectrum(mask.detach().contiguous(), N.FIELD_REAL_F32, model.plan)
+            # g^c without its 1 / (ny nx) -> the factor (ny nx) / (Mr Mc) moves to the last scale; a real mask's
+            # gradient is the same through the packed fields, which give the same image for every real mask
+            plan = adjoint_plan(model)
+            gc = _coarse_gradient(model, g.to(torch.float32), 1.0 / (model.ny * model.nx))
+            w = _adjoint_shares(model, band, gc, *model.fields_for(N.FIELD_REAL_F32))
+            grad = _mask_gradient(model, w[:, :, :, 0], 2.0 / (plan.mr * plan.mc))
         return grad.view_as(mask), None
 
 
@@ -127,7 +172,7 @@ def source_weight_gradient(model: CoherentModel, mask: torch.Tensor, g: torch.Te
     with torch.no_grad():
         band = band_spectrum(mask.contiguous(), N.FIELD_REAL_F32, model.plan)
         gc = coarse_gradient(model, g.to(torch.float32).contiguous())
-        _, dots = coherent_adjoint(model, band, gc, field_dots=True)    # [B, Z, P*S*E]
+        dots = _field_dots(model, band, gc)                             # [B, Z, P*S*E]
         S = values.numel()
         P = getattr(model, 'pol_states', 1)                              # incoherent polarisation states
         E = model.count // (S * P)

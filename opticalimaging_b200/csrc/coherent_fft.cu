@@ -37,9 +37,9 @@ struct CoherentFftArgs {
 };
 
 // grid (nsplit, nz, batch); block = mc * N1R threads (column tasks); mr = 32 N1R, mc = 32 N1C.
-// Bound: FP32 and shared-memory issue, and latency where a block has one field.  With the band at frequency 0 (fft_common)
-// a gather term is one load and one complex FMA (64 a transform of 128 points); with the band in place it was 128 tests,
-// and twiddles read by computed index: one field a block, 96 blocks, 128 x 128: 17.0 -> 11.3 us.
+// Bound: FP32 and shared-memory issue, and latency where a block has one field.  With the band wrapped (fft_common) a
+// gather term is one load and one complex FMA (64 a transform of 128 points); gathered from a band array it was 128
+// tests, and twiddles read by computed index: one field a block, 96 blocks, 128 x 128: 17.0 -> 11.3 us.
 template <int N1R, int N1C>
 __global__ void __launch_bounds__(32 * N1C * N1R) coherent_fft_kernel(CoherentFftArgs a) {
   using R = cg::Axis<N1R>;
@@ -48,14 +48,16 @@ __global__ void __launch_bounds__(32 * N1C * N1R) coherent_fft_kernel(CoherentFf
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* twr = (float2*)smem_raw;         // [32][N1R]
   float2* twc = twr + 32 * N1R;            // [32][N1C]
-  float2* as = twc + 32 * N1C;             // [R::B][C::BAND_LD]  the field on the band, columns zero beyond bc
-  float2* e1 = as + R::B * C::BAND_LD;     // [R::B][C::FIELD_LD] its rows transformed, rows zero beyond br
+  float2* as = twc + 32 * N1C;             // [R::B][C::BAND_LD]  the field on the band, columns at their places, else zero
+  float2* e1 = as + R::B * C::BAND_LD;     // [R::B][C::FIELD_LD] its rows transformed, rows at their places, else zero
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x, z = blockIdx.y, br = a.br, bc = a.bc;
   const long long b = blockIdx.z;
   cg::build_twiddles<N1R>(twr, a.wr, tid, T);
   cg::build_twiddles<N1C>(twc, a.wc, tid, T);
-  for (int j = br * C::FIELD_LD + tid; j < R::B * C::FIELD_LD; j += T) e1[j] = make_float2(0.f, 0.f);
+  for (int j = tid; j < R::B * (C::BAND_LD + C::FIELD_LD); j += T) as[j] = make_float2(0.f, 0.f);
+  const int pr = R::place0(a.m0r, br), pc = C::place0(a.m0c, bc);
+  __syncthreads();
   const int sc = tid % C::M, n1r = tid / C::M;  // column task of this thread
   float acc[32];
 #pragma unroll
@@ -74,7 +76,7 @@ __global__ void __launch_bounds__(32 * N1C * N1R) coherent_fft_kernel(CoherentFf
 #pragma unroll
       for (int u = 0; u < C::B / 32; ++u) {
         const int ic = lane + 32 * u;
-        as[ir * C::BAND_LD + ic] = ic < bc ? cmul(__ldg(pk + ir * bc + ic), __ldg(hc + ir * bc + ic)) : make_float2(0.f, 0.f);
+        if (ic < bc) as[ir * C::BAND_LD + ((pc + ic) & (C::B - 1))] = cmul(__ldg(pk + ir * bc + ic), __ldg(hc + ir * bc + ic));
       }
     }
     __syncthreads();
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(32 * N1C * N1R) coherent_fft_kernel(CoherentFf
       float2 zr[32];
       cg::band_ifft<N1C>(zr, as + ir * C::BAND_LD, 1, twc, n1);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) e1[ir * C::FIELD_LD + n1 + N1C * brev5(i)] = zr[i];
+      for (int i = 0; i < 32; ++i) e1[((pr + ir) & (R::B - 1)) * C::FIELD_LD + n1 + N1C * brev5(i)] = zr[i];
     }
     __syncthreads();
     // column pass: thread (sc, n1r)

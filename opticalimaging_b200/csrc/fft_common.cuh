@@ -1,5 +1,5 @@
-// Device helpers shared by the coarse-grid kernels (coherent_fft.cu, coherent_tc.cu, adjoint.cu): the 32-point
-// transform in registers and the inverse four-step gather of a band-limited input.
+// Device helpers shared by the coarse-grid kernels (coherent_fft.cu, adjoint.cu): the 32-point transform in registers and
+// the inverse four-step gather of a band-limited input.
 #pragma once
 #include "oi_common.cuh"
 
@@ -49,60 +49,40 @@ __device__ __forceinline__ void dft32(float2 (&v)[32]) {
 __device__ __forceinline__ void ifft32(float2 (&v)[32]) { dft32<-1>(v); }
 
 // The coarse grids' geometry (M = 32 N1, 64 or 128 points per axis).  A band of b frequencies fits when 2 b - 1 <= M,
-// so b <= B = 16 N1; its offset only turns the phase of the field, E[s] = exp(-2 pi i m0 s / M) E0[s] with E0 the
-// transform of the band placed at frequency 0, and neither |E|^2 nor the adjoint's products see that phase.  With the
-// band at 0 and zeros up to B, the four-step gather of an output is N1 / 2 terms with no bounds to check.
+// so b <= B = 16 N1.  A band inside [-B/2, B/2) is kept wrapped, frequency m at place m mod B; any other is shifted
+// there first: that only turns the phase of the field, which neither |E|^2 nor the adjoint's products see.
+// A gather term then needs no bounds, and frequency 0, the largest by far, meets no rounded twiddle.
 template <int N1> struct Axis {
   static constexpr int M = 32 * N1, B = 16 * N1;
   static constexpr int BAND_LD = B + 2;     // row of a band array: eight rows' values fall on eight bank pairs
   static constexpr int FIELD_LD = M + N1;   // row of a row-transformed array: as many rows as a half warp holds
+  // where band index 0 (frequency m0) goes: index i of b is at (place0 + i) mod B
+  __host__ __device__ static int place0(int m0, int b) { return (m0 >= -B / 2 && m0 + b <= B / 2 ? m0 : -B / 2) & (B - 1); }
 };
 
-// tw[t][n1] = exp(-2 pi i t n1 / M), 32 x N1, from w[j] = exp(+2 pi i j / M).
+// tw[t][n1] = exp(-2 pi i m n1 / M), 32 x N1, from w[j] = exp(+2 pi i j / M): m = t, or for B = 32 the frequency at place t.
 template <int N1>
 __device__ __forceinline__ void build_twiddles(float2* tw, const float2* w, int tid, int nthreads) {
+  constexpr int M = 32 * N1;
   for (int e = tid; e < 32 * N1; e += nthreads) {
-    const float2 t = __ldg(w + (((e / N1) * (e % N1)) & (32 * N1 - 1)));
-    tw[e] = make_float2(t.x, -t.y);
+    const int t = e / N1, m = N1 == 2 && t >= 16 ? t - 32 : t;
+    const float2 v = __ldg(w + ((m * (e % N1)) & (M - 1)));
+    tw[e] = make_float2(v.x, -v.y);
   }
 }
 
-// Thread n1 of N1: z[i] = X[n1 + N1 brev5(i)], X[s] = sum_{j < 16 N1} src[j * stride] exp(-2 pi i j s / M).
+// Thread n1 of N1: z[i] = X[n1 + N1 brev5(i)], X[s] = sum_p src[p * stride] exp(-2 pi i m(p) s / M), p < B, m(p) = p below
+// B / 2, else p - B.
 template <int N1>
 __device__ __forceinline__ void band_ifft(float2 (&z)[32], const float2* src, int stride, const float2* tw, int n1) {
   static_assert(N1 == 2 || N1 == 4, "coarse grids of 64 or 128");
-  // W_4^{-n1}: 1, -i, -1, i
-  const float2 w1 = make_float2(n1 == 0 ? 1.f : n1 == 2 ? -1.f : 0.f, n1 == 1 ? -1.f : n1 == 3 ? 1.f : 0.f);
+  // the place t + 32 holds frequency t - 32: exp(+2 pi i 32 n1 / 128) = 1, i, -1, -i
+  const float2 w1 = make_float2(n1 == 0 ? 1.f : n1 == 2 ? -1.f : 0.f, n1 == 1 ? 1.f : n1 == 3 ? -1.f : 0.f);
 #pragma unroll
   for (int t = 0; t < 32; ++t) {
     float2 acc = src[t * stride];
     if (N1 == 4) cfma(acc, src[(t + 32) * stride], w1);
     z[t] = t == 0 ? acc : cmul(acc, tw[t * N1 + n1]);
-  }
-  ifft32(z);
-}
-
-// Inverse four-step for an M = 32 N1 point transform of a band-limited input: thread n1 forms
-//   z[k2] = W_M^{-k2 n1} sum_k1 x[k2 + 32 k1] W_N1^{-k1 n1},  x[k] = src[((k - m0) mod M) * stride] if < b else 0,
-// then the 32-point transform; on return z[i] = X[n1 + N1 brev5(i)], X[s] = sum_m x_m exp(-2 pi i m s / M).
-// w: exp(+2 pi i j / M), j < M.
-template <int N1>
-__device__ __forceinline__ void gather_ifft(float2 (&z)[32], const float2* src, int stride, int m0, int b,
-                                            const float2* w, int n1) {
-  constexpr int M = 32 * N1;
-#pragma unroll
-  for (int k2 = 0; k2 < 32; ++k2) {
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) {
-      const int idx = (k2 + 32 * k1 - m0) & (M - 1);
-      if (idx < b) {
-        const float2 tw = w[(32 * k1 * n1) & (M - 1)];
-        cfma(acc, src[idx * stride], make_float2(tw.x, -tw.y));
-      }
-    }
-    const float2 tw = w[(k2 * n1) & (M - 1)];
-    z[k2] = cmul(acc, make_float2(tw.x, -tw.y));
   }
   ifft32(z);
 }
