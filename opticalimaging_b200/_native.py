@@ -105,7 +105,7 @@ def exported_symbols():
 
 def call(name, *args):
     """Call entry point `name`; raise NativeError with the library's message on a non-zero status."""
-    lib = load()
+    lib = _lib or load()
     rc = getattr(lib, name)(*args)
     if rc < 0:
         msg = lib.oi_last_error().decode(errors='replace')
@@ -113,12 +113,14 @@ def call(name, *args):
 
 
 def ptr(t):
-    """Device pointer of a tensor (None -> NULL)."""
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    """Device pointer of a tensor as an integer (None -> NULL)."""
+    return None if t is None else t.data_ptr()
 
 
 def stream_handle(device=None):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The current CUDA stream of a device (the current one for None) as an integer handle."""
+    index = None if device is None else torch.device(device).index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def host_doubles(values):

@@ -197,7 +197,7 @@ class Plan:
 
     @classmethod
     def get(cls, ny, nx, band: Band, device, coarse=None) -> 'Plan':
-        key = (ny, nx, band, str(device), coarse)
+        key = (ny, nx, band, device, coarse)
         with cls._lock:
             p = cls._cache.get(key)
             if p is None:
@@ -216,7 +216,7 @@ _SM_COUNTS: dict = {}
 def sm_count() -> int:
     """Streaming multiprocessors of the current device (148 on a B200): the grids of the one-block-per-SM
     kernels and the field splits below are sized by it, as the native layouts are."""
-    if not torch.cuda.is_available():
+    if not (torch.cuda.is_initialized() or torch.cuda.is_available()):
         return B200_SMS
     d = torch.cuda.current_device()
     n = _SM_COUNTS.get(d)
@@ -336,7 +336,7 @@ def coherent_image(band: torch.Tensor, pupils: torch.Tensor, weights: torch.Tens
     _mark(marks, 'coherent_coarse')
     if out is None:
         out = torch.empty((batch, nz, plan.ny, plan.nx), dtype=torch.float32, device=dev)
-    ihat = torch.empty(batch * nz * (2 * b.br - 1) * b.bc, dtype=torch.complex64, device=dev)
+    nhat, nv = batch * nz * (2 * b.br - 1) * b.bc, batch * nz * b.bc * plan.ny
     if form == 'bf16x3' and plan.tc_rows(form):
         # coarse spectrum and column synthesis as two tensor-core GEMMs straight into the row pass's operand tiles
         tiles = torch.empty(batch * nz * plan.ny * 512, dtype=torch.uint8, device=dev)
@@ -347,18 +347,21 @@ def coherent_image(band: torch.Tensor, pupils: torch.Tensor, weights: torch.Tens
         count = batch * nz
         wn_r, wn_c = plan.coarse_fft_tables()
         t = torch.empty(count * plan.mr * b.bc, dtype=torch.complex64, device=dev)
+        ihat = torch.empty(nhat, dtype=torch.complex64, device=dev)
         N.call('oi_coarse_half_spectrum_fft', N.ptr(coarse), nsplit, count, plan.mr, plan.mc, b.br, b.bc, N.ptr(wn_c),
                N.ptr(wn_r), N.ptr(t), N.ptr(ihat), s)
-        v = torch.empty(count * b.bc * plan.ny, dtype=torch.complex64, device=dev)
+        v = torch.empty(nv, dtype=torch.complex64, device=dev)
         N.call('oi_spectrum_to_image_fft', N.ptr(ihat), count, b.br, b.bc, N.ptr(plan.wn_y), N.ptr(plan.wn_x),
                plan.ny, plan.nx, N.ptr(v), N.ptr(out), s)
     elif plan.use_fft(form):
-        v = torch.empty(batch * nz * b.bc * plan.ny, dtype=torch.complex64, device=dev)
+        # one allocation: v, then ihat (a multiple of 512 bytes on, as ny is at least 256)
+        v = torch.empty(nv + nhat, dtype=torch.complex64, device=dev)
         wm_r, wm_c = (plan.wm_r, plan.wm_c) if plan.coarse_small else (None, None)
         N.call('oi_coarse_to_image_fft', N.ptr(coarse), nsplit, batch * nz, plan.mr, plan.mc, b.br, b.bc,
                N.ptr(plan.gc), N.ptr(plan.gr), N.ptr(wm_r), N.ptr(wm_c), N.ptr(plan.wn_y), N.ptr(plan.wn_x),
-               plan.ny, plan.nx, N.ptr(ihat), N.ptr(v), N.ptr(out), s)
+               plan.ny, plan.nx, N.ptr(v) + 8 * nv, N.ptr(v), N.ptr(out), s)
     else:
+        ihat = torch.empty(nhat, dtype=torch.complex64, device=dev)
         N.call('oi_coarse_to_image', N.ptr(coarse), nsplit, batch * nz, plan.mr, plan.mc, b.br, b.bc,
                N.ptr(plan.gc), N.ptr(plan.gr), N.ptr(plan.sy), N.ptr(plan.sx), plan.ny, plan.nx, N.ptr(ihat),
                N.ptr(out), s)
