@@ -332,6 +332,29 @@ OI_API int oi_coherent_adjoint(const void* band, int batch, int nch, int m0r, in
                                int mc, const void* wr, const void* wc, int nsplit, void* wout, float* field_dot,
                                void* stream);
 
+/*
+ * The sigmoid resist loss of images [batch][nz][n] against targets [batch][n] (float32, device):
+ * *loss = sum (s - t)^2, s = 1 / (1 + exp(-steepness (I - threshold))), summed in FP64; grad, when not NULL, is its
+ * derivative by the images.  work: oi_resist_loss_workspace bytes (device).
+ */
+OI_API int oi_resist_loss_workspace(long long* bytes);
+OI_API int oi_resist_loss(const float* image, const float* target, int batch, int nz, long long n, float steepness,
+                          float threshold, float* grad, float* loss, void* work, long long work_bytes, void* stream);
+
+/*
+ * Field weights of an Abbe model for source weights `values` (double [points], device): weights [nz][fields] float32,
+ * index_image v_j / sum v for the fields_per_point fields of point j, in the order [state][point][component].
+ */
+OI_API int oi_source_weights(const double* values, int points, int fields_per_point, int fields, int nz, double index_image,
+                             float* weights, void* stream);
+
+/*
+ * dL/dv [batch][points] from the field dots [batch][nz][states][points][fields_per_point]: (n d_j - n / W sum d_i v_i) / W,
+ * d_j the sum of point j's dots, W the sum of v (dI/dv_j = (n I_j - I) / W, CalculateAerialImage.py:89-92).
+ */
+OI_API int oi_source_gradient(const float* dots, int batch, int nz, int states, int points, int fields_per_point,
+                              const double* values, double index_image, float* out, void* stream);
+
 /* The field dots of oi_coherent_adjoint alone (field_dot as there). */
 OI_API int oi_coherent_field_dots(const void* band, int batch, int nch, int m0r, int br, int m0c, int bc,
                                   const void* pupil, const float* weight, int nz, int nk, const float* gcoarse, int mr, int mc,

@@ -36,6 +36,10 @@ _SIGS = {
     'oi_spectrum_to_image_fft': [_vp, _i, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp],
     'oi_coherent_adjoint': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _vp,
                             _vp],
+    'oi_resist_loss_workspace': [_vp],
+    'oi_resist_loss': [_vp, _vp, _i, _i, _ll, _f, _f, _vp, _vp, _vp, _ll, _vp],
+    'oi_source_weights': [_vp, _i, _i, _i, _i, _d, _vp, _vp],
+    'oi_source_gradient': [_vp, _i, _i, _i, _i, _i, _vp, _d, _vp, _vp],
     'oi_coherent_field_dots': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _vp],
     'oi_hermitian_half': [_vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
     'oi_band_spectrum_noalloc': [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp],

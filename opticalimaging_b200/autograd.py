@@ -134,6 +134,7 @@ class _CoherentImage(torch.autograd.Function):
         ctx.model = model
         with torch.no_grad():
             m = mask.detach().contiguous()
+            model.check_grid(m)
             band = band_spectrum(m, N.FIELD_REAL_F32, model.plan, form=model.form)
             image = coherent_image(band, *model.fields_for(N.FIELD_REAL_F32), model.plan, form=model.form)
         # the backward pass starts from the FP32 band spectrum: the forward's own, unless that ran in split form
@@ -173,11 +174,14 @@ def source_weight_gradient(model: CoherentModel, mask: torch.Tensor, g: torch.Te
         band = band_spectrum(mask.contiguous(), N.FIELD_REAL_F32, model.plan)
         gc = coarse_gradient(model, g.to(torch.float32).contiguous())
         dots = _field_dots(model, band, gc)                             # [B, Z, P*S*E]
+        B, Z, K = dots.shape
         S = values.numel()
         P = getattr(model, 'pol_states', 1)                              # incoherent polarisation states
-        E = model.count // (S * P)
-        d = dots.view(dots.shape[0], dots.shape[1], P, S, E).sum(dim=(1, 2, 4)).double()   # <g, I_j>
-        v = values.to(d.device, torch.float64).reshape(1, -1)
-        W = v.sum()
-        gI = (d * v).sum(dim=1, keepdim=True) * index_image / W               # <g, I>
-        return ((index_image * d - gI) / W).float()
+        E = K // (S * P)
+        if S * P * E != K:
+            raise ValueError(f'{S} source weights do not divide the model\'s {K} fields')
+        v = values.detach().to(dots.device, torch.float64).reshape(-1).contiguous()
+        out = torch.empty((B, S), dtype=torch.float32, device=dots.device)
+        N.call('oi_source_gradient', N.ptr(dots), B, Z, P, S, E, N.ptr(v), float(index_image), N.ptr(out),
+               N.stream_handle(dots.device))
+        return out

@@ -527,6 +527,10 @@ class CoherentModel:
         return {torch.float32: N.FIELD_REAL_F32, torch.uint8: N.FIELD_U8,
                 torch.complex64: N.FIELD_COMPLEX_C64}[masks.dtype]
 
+    def check_grid(self, masks: torch.Tensor) -> None:
+        if masks.shape[1] != self.ny or masks.shape[2] != self.nx:
+            raise ValueError(f'mask grid {tuple(masks.shape[1:3])} != model grid {(self.ny, self.nx)}')
+
     def image(self, masks: torch.Tensor, kind: int | None = None, nch: int = 1, scale: float = 1.0,
               out: torch.Tensor | None = None, marks=None, form: str | None = None) -> torch.Tensor:
         """Aerial images of a batch of masks -> [B, Z, ny, nx] float32.
@@ -541,8 +545,7 @@ class CoherentModel:
             kind = self._kind(masks)
         if form is None:
             form = self.form
-        if masks.shape[1] != self.ny or masks.shape[2] != self.nx:
-            raise ValueError(f'mask grid {tuple(masks.shape[1:3])} != model grid {(self.ny, self.nx)}')
+        self.check_grid(masks)
         _mark(marks, 'start')
         band = band_spectrum(masks.contiguous(), kind, self.plan, nch=nch, scale=scale, form=form)
         _mark(marks, 'band_spectrum')

@@ -17,8 +17,11 @@ The reference has no optimisation loop; it differentiates its SOCS image by torc
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
+from . import _native as N
 from .autograd import aerial_image, source_weight_gradient
 from .engine import CoherentModel
 
@@ -33,9 +36,48 @@ class ResistModel:
         return torch.sigmoid(self.steepness * (image - self.threshold))
 
 
+class _ResistLoss(torch.autograd.Function):
+    """sum (sigmoid(a (I - thr)) - target)^2 in one pass over the images, which also leaves the derivative by the images
+    for the backward pass (no other buffer is saved).  A backward pass that is itself recorded (create_graph) goes through
+    the composition of torch operations instead."""
+
+    @staticmethod
+    def forward(ctx, image, target, steepness, threshold):
+        img = image.contiguous()
+        B, Z, ny, nx = img.shape
+        grad = torch.empty_like(img) if ctx.needs_input_grad[0] else None
+        loss = torch.empty((), dtype=torch.float32, device=img.device)
+        nbytes = ctypes.c_longlong(0)
+        N.call('oi_resist_loss_workspace', ctypes.byref(nbytes))
+        work = torch.empty(nbytes.value, dtype=torch.uint8, device=img.device)
+        N.call('oi_resist_loss', N.ptr(img), N.ptr(target), B, Z, ny * nx, steepness, threshold, N.ptr(grad), N.ptr(loss),
+               N.ptr(work), nbytes.value, N.stream_handle(img.device))
+        if grad is not None:
+            ctx.save_for_backward(grad)
+            ctx.composed = (image, target, steepness, threshold)
+        return loss
+
+    @staticmethod
+    def backward(ctx, g):
+        if torch.is_grad_enabled():
+            image, target, a, thr = ctx.composed
+            s = torch.sigmoid(a * (image - thr))
+            return g * (2.0 * (s - target[:, None])) * (a * s * (1.0 - s)), None, None, None
+        (grad,) = ctx.saved_tensors
+        if not torch._C._autograd._get_current_graph_task_keep_graph():
+            ctx.composed = None      # freed with the graph, as saved tensors are
+        return grad * g, None, None, None
+
+
 def ilt_loss(model: CoherentModel, mask: torch.Tensor, target: torch.Tensor, resist: ResistModel):
     """(loss, image): ||R(I(mask)) - target||^2 over pixels and planes; mask [B, ny, nx], target [B, ny, nx]."""
     image = aerial_image(model, mask)                        # [B, Z, ny, nx]
+    # one float32 target per mask and the sigmoid resist itself: the fused loss; any other resist callable, broadcast or
+    # differentiable target: torch operations
+    if (type(resist) is ResistModel and target.dtype == torch.float32 and target.device == image.device
+            and target.shape == (image.shape[0],) + image.shape[2:] and target.is_contiguous()
+            and not target.requires_grad):
+        return _ResistLoss.apply(image, target, float(resist.steepness), float(resist.threshold)), image
     loss = torch.sum((resist(image) - target[:, None]) ** 2)
     return loss, image
 
@@ -72,13 +114,14 @@ def set_source_weights(model: CoherentModel, values: torch.Tensor, index_image: 
     if model.kind != 'abbe':
         raise ValueError('source weights belong to an Abbe model (abbe_model)')
     Z, K = model.weights.shape
-    v = values.to(model.device, torch.float64).reshape(-1)
-    if K % v.numel():
-        raise ValueError(f'{v.numel()} source weights do not divide the model\'s {K} fields')
-    w = (index_image / v.sum()) * v
-    P = getattr(model, 'pol_states', 1)          # fields are [polarisation state][point][component]
-    per = w.repeat_interleave(K // (P * v.numel())).repeat(P)
-    model.weights.copy_(per.to(torch.float32)[None].expand(Z, K))
+    v = values.detach().to(model.device, torch.float64).reshape(-1).contiguous()
+    S, P = v.numel(), getattr(model, 'pol_states', 1)      # fields are [polarisation state][point][component]
+    if K % (P * S):
+        raise ValueError(f'{S} source weights do not divide the model\'s {K} fields')
+    w = model.weights if model.weights.is_contiguous() else torch.empty_like(model.weights, memory_format=torch.contiguous_format)
+    N.call('oi_source_weights', N.ptr(v), S, K // (P * S), K, Z, float(index_image), N.ptr(w), N.stream_handle(model.device))
+    if w is not model.weights:
+        model.weights.copy_(w)
     model.packed = None   # packed for the previous weights
 
 
