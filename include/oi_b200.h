@@ -175,6 +175,11 @@ OI_API int oi_fft_supported(int ny, int nx);
 OI_API int oi_band_spectrum_fft(const void* field, int kind, int batch, int ny, int nx, int m0r, int br, int m0c,
                                 int bc, const void* wn_x, const void* wn_y, float scale, void* scratch, void* band,
                                 void* stream);
+
+/* oi_band_spectrum_fft for complex fields [batch][ny][nx][nch]: band [batch][nch][br][bc]; scratch batch*nch*ny*bc complex. */
+OI_API int oi_band_spectrum_fft_c64(const void* field, int batch, int ny, int nx, int nch, int m0r, int br, int m0c, int bc,
+                                    const void* wn_x, const void* wn_y, float scale, void* scratch, void* band,
+                                    void* stream);
 OI_API int oi_coarse_to_image_fft(float* coarse, int nparts, int count, int mr, int mc, int br, int bc,
                                   const void* gc, const void* gr, const void* wm_r, const void* wm_c,
                                   const void* wn_y, const void* wn_x, int ny, int nx, void* scratch_ihat,

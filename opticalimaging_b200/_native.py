@@ -30,6 +30,7 @@ _SIGS = {
     'oi_tcc_assemble64_marked': [_vp, _i, _i, _i, _vp, _vp, _ll, _vp],
     'oi_fft_supported': [_i, _i],
     'oi_band_spectrum_fft': [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp, _vp],
+    'oi_band_spectrum_fft_c64': [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp, _vp],
     'oi_coarse_to_image_fft': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp,
                                _vp],
     'oi_spectrum_to_image': [_vp, _i, _i, _i, _vp, _vp, _i, _i, _vp, _vp],

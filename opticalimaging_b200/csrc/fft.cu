@@ -142,50 +142,157 @@ __device__ __forceinline__ void outer_bin2(const float2* ys, const float2* t1, i
 }
 
 // --------------------------------------------------------------------------------- forward, rows
-// field rows [nrows = batch*ny][N] (real or u8) -> t[b][ic][y], ic over the band m0c .. m0c+bc-1.
-// Z is evaluated on the contiguous frequency range u0 .. u0+nu-1 that holds the band and its mirror.
-template <int N1, int KIND>
-__global__ void __launch_bounds__(256, 3) fft_rows_fwd_kernel(const void* __restrict__ field, long long nrows, int ny,
+// cos(2 pi t / 64) for t = 0..16 (exact decimal expansions of the standard values; the even ones are c32's), and for any
+// t >= 0.  Inlined without recursion, so that a constant t leaves a constant.
+__host__ __device__ __forceinline__ constexpr float c64q(int t) {
+  return t == 16 ? 0.0f : t % 2 == 0 ? c32(t / 2) : t == 1 ? 0.995184726672196886f : t == 3 ? 0.956940335732208865f
+       : t == 5 ? 0.881921264348355029f : t == 7 ? 0.773010453362736960f : t == 9 ? 0.634393284163645498f
+       : t == 11 ? 0.471396736825997649f : t == 13 ? 0.290284677254462367f : 0.098017140329560602f;
+}
+__host__ __device__ __forceinline__ constexpr float c64h(int t) { return t > 16 ? -c64q(32 - t) : c64q(t); }   // t <= 32
+__host__ __device__ __forceinline__ constexpr float c64(int t) { return (t & 63) > 32 ? c64h(64 - (t & 63)) : c64h(t & 63); }
+__host__ __device__ __forceinline__ constexpr float s64(int t) { return c64(t + 48); }
+
+// The outer sums of the bins k2 + 32 k1, -H <= k1 < H, from one row of twiddled values: out[k1 + H] = sum over the NT values
+// n1 of row[n1] exp(+2 pi i k1 n1 / N1).  The row is read once for all 2 H bins and the twiddles are constants; +k1 and -k1
+// share their products with cos and sin.
+template <int N1, int H, int NT>
+__device__ __forceinline__ void outer_sums(float2 (&out)[2 * H], const float2* row) {
+  float2 a0 = make_float2(0.f, 0.f), last = a0, ca[H], sa[H];
+#pragma unroll
+  for (int p = 0; p < H; ++p) ca[p] = sa[p] = a0;
+#pragma unroll
+  for (int n1 = 0; n1 < NT; ++n1) {
+    const float2 y = row[n1];
+    a0.x += y.x;
+    a0.y += y.y;
+#pragma unroll
+    for (int p = 1; p < H; ++p) {
+      const float c = c64(64 / N1 * p * n1), s = s64(64 / N1 * p * n1);
+      ca[p].x = fmaf(y.x, c, ca[p].x);
+      ca[p].y = fmaf(y.y, c, ca[p].y);
+      sa[p].x = fmaf(y.x, s, sa[p].x);
+      sa[p].y = fmaf(y.y, s, sa[p].y);
+    }
+    cfma(last, y, make_float2(c64(64 / N1 * H * n1), -s64(64 / N1 * H * n1)));   // k1 = -H
+  }
+  out[0] = last;
+  out[H] = a0;
+#pragma unroll
+  for (int p = 1; p < H; ++p) {
+    out[H + p] = make_float2(ca[p].x - sa[p].y, ca[p].y + sa[p].x);
+    out[H - p] = make_float2(ca[p].x + sa[p].y, ca[p].y - sa[p].x);
+  }
+}
+
+// Real masks (float32 or uint8): field rows [nrows = batch*ny][N], two rows per group as one complex row.  Complex fields
+// [batch][ny][N][nch]: rows (b, y, c), c fastest (the channels of a row share its cache lines), one per group.
+// -> t[(b, c)][ic][y], ic over the band m0c .. m0c+bc-1.  Z is evaluated on the contiguous frequency range u0 .. u0+nu-1
+// that holds the band and, for real rows, its mirror; H: that range lies within [-32 H, 32 H) (0: any).
+// Bound: instruction issue (about 1500 a warp for two rows of 1024) and latency: 24 warps an SM, all their registers.
+// With one bin per thread at a time, its twiddles read from global memory, the outer sums cost twice the loads and
+// stalled on them: 4 masks of 2048 x 2048, 117 columns: 41.0 -> 30.3 us; 8 of 1024, 59: 14.2 -> 12.2.
+// Two fields of 512 x 512 x 3 complex: 41.5 (as a dense product) -> 6.7 us.
+template <int N1, int KIND, int H>
+__global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_fwd_kernel(const void* __restrict__ field, long long nrows, int ny, int nch,
                                                            const float2* __restrict__ wn_g, int m0c, int bc, int u0,
                                                            int nu, float2* __restrict__ t, int nparts,
                                                            long long pstride) {
   // nparts > 1 (float32 only): the field is the sum of nparts arrays pstride elements apart
-  constexpr int N = 32 * N1, G = 256 / N1;  // G row pairs per block
+  constexpr bool CPLX = KIND == OI_FIELD_COMPLEX_C64;
+  constexpr int N = 32 * N1, G = 256 / N1, PER = CPLX ? 1 : 2;  // G groups per block, PER rows each
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const float2* t2 = wn_g;                    // global [32][N1], read through L1 (warp-coalesced)
   const float2* t1 = wn_g + 32 * N1;          // global [N1][N1]
   float2* ys = (float2*)smem_raw;             // [G][32][N1+1]
   float2* zs = ys + G * 32 * (N1 + 1);        // [G][nu]
   const int tid = threadIdx.x, g = tid / N1, n1 = tid % N1;
-  const long long r0 = (long long)blockIdx.x * (2 * G) + 2 * g;
+  const long long r0 = (long long)blockIdx.x * (PER * G) + PER * g;
   float2 z[32];
-  if (r0 + 1 < nrows) {
-    const long long o0 = r0 * N, o1 = o0 + N;
+  if constexpr (CPLX) {
+    if (r0 < nrows) {
+      const float2* f = (const float2*)field + (r0 / nch * N + n1) * nch + r0 % nch;
+      const long long step = (long long)N1 * nch;
 #pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2)
-      z[n2] = make_float2(load_real<KIND>(field, o0 + n1 + N1 * n2), load_real<KIND>(field, o1 + n1 + N1 * n2));
-    for (int p = 1; p < nparts; ++p) {
-      const long long op = p * pstride;
+      for (int n2 = 0; n2 < 32; ++n2) z[n2] = __ldg(f + n2 * step);
+    } else {
 #pragma unroll
-      for (int n2 = 0; n2 < 32; ++n2) {
-        z[n2].x += load_real<KIND>(field, op + o0 + n1 + N1 * n2);
-        z[n2].y += load_real<KIND>(field, op + o1 + n1 + N1 * n2);
-      }
+      for (int n2 = 0; n2 < 32; ++n2) z[n2] = make_float2(0.f, 0.f);
     }
   } else {
+    if (r0 + 1 < nrows) {
+      const long long o0 = r0 * N, o1 = o0 + N;
 #pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2) z[n2] = make_float2(0.f, 0.f);
+      for (int n2 = 0; n2 < 32; ++n2)
+        z[n2] = make_float2(load_real<KIND>(field, o0 + n1 + N1 * n2), load_real<KIND>(field, o1 + n1 + N1 * n2));
+      for (int p = 1; p < nparts; ++p) {
+        const long long op = p * pstride;
+#pragma unroll
+        for (int n2 = 0; n2 < 32; ++n2) {
+          z[n2].x += load_real<KIND>(field, op + o0 + n1 + N1 * n2);
+          z[n2].y += load_real<KIND>(field, op + o1 + n1 + N1 * n2);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int n2 = 0; n2 < 32; ++n2) z[n2] = make_float2(0.f, 0.f);
+    }
   }
   fft32<+1>(z);
-  __syncthreads();  // tables ready
   float2* yg = ys + g * 32 * (N1 + 1);
   twiddle_store<+1, N1>(z, t2, n1, yg);
   __syncthreads();
   float2* zg = zs + g * nu;
-  for (int q = n1; q < nu; q += N1) zg[q] = outer_bin<+1, N1>(yg, t1, (u0 + q) & (N - 1));
+  if constexpr (H == 0) {
+    for (int q = n1; q < nu; q += N1) zg[q] = outer_bin<+1, N1>(yg, t1, (u0 + q) & (N - 1));
+  } else {
+    // k2 = n1 + N1 j, all N1 terms; N1 = 64: k2 = n1 % 32, the upper half of the threads the upper half of the terms, whose
+    // twiddles are those of the lower half times (-1)^k1
+    constexpr int NT = N1 < 32 ? N1 : 32;
+    const bool upper = N1 == 64 && n1 >= 32;
+#pragma unroll
+    for (int k2 = n1 & 31; k2 < 32; k2 += NT) {
+      float2 o[2 * H];
+      outer_sums<N1, H, NT>(o, yg + k2 * (N1 + 1) + (upper ? 32 : 0));
+      if constexpr (N1 == 64) {
+        if (upper) {
+#pragma unroll
+          for (int i = 0; i < 2 * H; ++i) {
+            const int q = k2 + 32 * (i - H) - u0;
+            const float sg = (i - H) & 1 ? -1.f : 1.f;
+            if (q >= 0 && q < nu) zg[q] = make_float2(sg * o[i].x, sg * o[i].y);
+          }
+        }
+        __syncthreads();
+      }
+      if (!upper) {
+#pragma unroll
+        for (int i = 0; i < 2 * H; ++i) {
+          const int q = k2 + 32 * (i - H) - u0;
+          if (q < 0 || q >= nu) continue;
+          if (N1 == 64) {
+            const float2 v = zg[q];
+            o[i].x += v.x;
+            o[i].y += v.y;
+          }
+          zg[q] = o[i];
+        }
+      }
+    }
+  }
   __syncthreads();
+  const long long rblk = (long long)blockIdx.x * (PER * G);
+  if constexpr (CPLX) {
+    for (int e = tid; e < bc * G; e += 256) {
+      const int ic = e / G, gg = e % G;
+      const long long r = rblk + gg;
+      if (r >= nrows) continue;
+      const long long line = r / nch, b = line / ny;
+      t[((b * nch + r % nch) * bc + ic) * (long long)ny + line - b * ny] = zs[gg * nu + (m0c + ic - u0)];
+    }
+    return;
+  }
   // separate the two real rows and write t[b][ic][y] with y fastest (2G consecutive rows of one image)
-  const long long rblk = (long long)blockIdx.x * (2 * G);
   for (int e = tid; e < bc * 2 * G; e += 256) {
     const int ic = e / (2 * G), rr = e % (2 * G), gg = rr >> 1;
     const long long r = rblk + rr;
@@ -733,30 +840,53 @@ template <int N1>
 static size_t smem_cols_fwd() { return sizeof(float2) * ((COLS_T / N1) * 32 * (N1 + 1)); }
 
 
-template <int N1>
-static int band_fft(const void* field, int kind, int batch, int ny, int nx, int m0r, int br, int m0c, int bc,
-                    const float2* wn_x, const float2* wn_y, float scale, float2* t, float2* band, cudaStream_t s,
-                    int nparts = 1, long long pstride = 0) {
-  // row transforms have length nx = 32 * N1; the column kernel picks its own N1 for ny
-  const int u0 = min(m0c, -(m0c + bc - 1)), u1 = max(m0c + bc - 1, -m0c), nu = u1 - u0 + 1;
-  constexpr int G = 256 / N1;
-  const long long nrows = (long long)batch * ny;
-  size_t smem = smem_rows_fwd<N1>(nu);
-  int rc;
-  if (kind == OI_FIELD_U8) {
-    rc = set_smem(fft_rows_fwd_kernel<N1, OI_FIELD_U8>, smem, "oi_band_spectrum_fft/rows");
-    if (rc) return rc;
-    fft_rows_fwd_kernel<N1, OI_FIELD_U8><<<(unsigned)ceil_div(nrows, 2 * G), 256, smem, s>>>(
-        field, nrows, ny, wn_x, m0c, bc, u0, nu, t, 1, 0LL);
-    oi::note_launch();
-  } else {
-    rc = set_smem(fft_rows_fwd_kernel<N1, OI_FIELD_REAL_F32>, smem, "oi_band_spectrum_fft/rows");
-    if (rc) return rc;
-    fft_rows_fwd_kernel<N1, OI_FIELD_REAL_F32><<<(unsigned)ceil_div(nrows, 2 * G), 256, smem, s>>>(
-        field, nrows, ny, wn_x, m0c, bc, u0, nu, t, nparts, pstride);
-    oi::note_launch();
-  }
+template <int N1, int KIND, int H>
+static int rows_fwd_h(const void* field, long long nrows, int ny, int nch, int m0c, int bc, int u0, int nu, const float2* wn_x,
+                      float2* t, cudaStream_t s, int nparts, long long pstride) {
+  constexpr int ROWS = (KIND == OI_FIELD_COMPLEX_C64 ? 1 : 2) * (256 / N1);
+  const size_t smem = smem_rows_fwd<N1>(nu);
+  if (int rc = set_smem(fft_rows_fwd_kernel<N1, KIND, H>, smem, "oi_band_spectrum_fft/rows")) return rc;
+  fft_rows_fwd_kernel<N1, KIND, H><<<(unsigned)ceil_div(nrows, ROWS), 256, smem, s>>>(field, nrows, ny, nch, wn_x, m0c, bc, u0,
+                                                                                     nu, t, nparts, pstride);
+  oi::note_launch();
   return check_launch("oi_band_spectrum_fft/rows");
+}
+template <int N1, int KIND>
+static int rows_fwd(const void* field, int batch, int ny, int nch, int m0c, int bc, const float2* wn_x, float2* t, cudaStream_t s,
+                    int nparts = 1, long long pstride = 0) {
+  int u0 = m0c, u1 = m0c + bc - 1;
+  if (KIND != OI_FIELD_COMPLEX_C64) {   // the band and its mirror
+    u0 = min(m0c, -(m0c + bc - 1));
+    u1 = max(m0c + bc - 1, -m0c);
+  }
+  const int nu = u1 - u0 + 1;
+  const long long nrows = (long long)batch * ny * nch;
+  auto within = [&](int h) { return u0 >= -32 * h && u1 < 32 * h; };
+  if (within(1)) return rows_fwd_h<N1, KIND, 1>(field, nrows, ny, nch, m0c, bc, u0, nu, wn_x, t, s, nparts, pstride);
+  if (within(2)) return rows_fwd_h<N1, KIND, 2>(field, nrows, ny, nch, m0c, bc, u0, nu, wn_x, t, s, nparts, pstride);
+  if (within(4)) return rows_fwd_h<N1, KIND, 4>(field, nrows, ny, nch, m0c, bc, u0, nu, wn_x, t, s, nparts, pstride);
+  return rows_fwd_h<N1, KIND, 0>(field, nrows, ny, nch, m0c, bc, u0, nu, wn_x, t, s, nparts, pstride);
+}
+
+// row transforms have length nx = 32 * N1; the column kernel picks its own N1 for ny
+template <int N1>
+static int band_fft(const void* field, int kind, int batch, int ny, int nch, int m0c, int bc, const float2* wn_x, float2* t,
+                    cudaStream_t s, int nparts = 1, long long pstride = 0) {
+  switch (kind) {
+    case OI_FIELD_U8: return rows_fwd<N1, OI_FIELD_U8>(field, batch, ny, nch, m0c, bc, wn_x, t, s);
+    case OI_FIELD_COMPLEX_C64: return rows_fwd<N1, OI_FIELD_COMPLEX_C64>(field, batch, ny, nch, m0c, bc, wn_x, t, s);
+  }
+  return rows_fwd<N1, OI_FIELD_REAL_F32>(field, batch, ny, nch, m0c, bc, wn_x, t, s, nparts, pstride);
+}
+static int band_rows(int nx1, const void* field, int kind, int batch, int ny, int nch, int m0c, int bc, const void* wn_x, float2* t,
+                     cudaStream_t s, int nparts = 1, long long pstride = 0) {
+  const float2* wx = (const float2*)wn_x;
+  switch (nx1) {
+    case 8: return band_fft<8>(field, kind, batch, ny, nch, m0c, bc, wx, t, s, nparts, pstride);
+    case 16: return band_fft<16>(field, kind, batch, ny, nch, m0c, bc, wx, t, s, nparts, pstride);
+    case 32: return band_fft<32>(field, kind, batch, ny, nch, m0c, bc, wx, t, s, nparts, pstride);
+  }
+  return band_fft<64>(field, kind, batch, ny, nch, m0c, bc, wx, t, s, nparts, pstride);
 }
 
 // bco: the output band width (SYM: bc = (bco + 1) / 2 input columns; else bco = bc)
@@ -887,19 +1017,36 @@ extern "C" int oi_band_spectrum_fft(const void* field, int kind, int batch, int 
     return fail(OI_ERANGE, "oi_band_spectrum_fft: band (%d+%d, %d+%d) too wide for %dx%d", m0r, br, m0c, bc, ny, nx);
   cudaStream_t s = (cudaStream_t)stream;
   float2* t = (float2*)scratch;
-  int rc;
-  switch (nx1) {
-    case 8: rc = band_fft<8>(field, kind, batch, ny, nx, m0r, br, m0c, bc, (const float2*)wn_x, (const float2*)wn_y, scale, t, (float2*)band, s); break;
-    case 16: rc = band_fft<16>(field, kind, batch, ny, nx, m0r, br, m0c, bc, (const float2*)wn_x, (const float2*)wn_y, scale, t, (float2*)band, s); break;
-    case 32: rc = band_fft<32>(field, kind, batch, ny, nx, m0r, br, m0c, bc, (const float2*)wn_x, (const float2*)wn_y, scale, t, (float2*)band, s); break;
-    default: rc = band_fft<64>(field, kind, batch, ny, nx, m0r, br, m0c, bc, (const float2*)wn_x, (const float2*)wn_y, scale, t, (float2*)band, s); break;
-  }
+  int rc = band_rows(nx1, field, kind, batch, ny, 1, m0c, bc, wn_x, t, s);
   if (rc) return rc;
   switch (ny1) {
     case 8: return cols_fwd<8>(t, batch, bc, (const float2*)wn_y, m0r, br, scale, (float2*)band, s);
     case 16: return cols_fwd<16>(t, batch, bc, (const float2*)wn_y, m0r, br, scale, (float2*)band, s);
     case 32: return cols_fwd<32>(t, batch, bc, (const float2*)wn_y, m0r, br, scale, (float2*)band, s);
     default: return cols_fwd<64>(t, batch, bc, (const float2*)wn_y, m0r, br, scale, (float2*)band, s);
+  }
+}
+
+extern "C" int oi_band_spectrum_fft_c64(const void* field, int batch, int ny, int nx, int nch, int m0r, int br, int m0c, int bc,
+                                        const void* wn_x, const void* wn_y, float scale, void* scratch, void* band,
+                                        void* stream) {
+  using namespace oi;
+  if (!field || !wn_x || !wn_y || !scratch || !band || batch <= 0 || nch <= 0 || br <= 0 || bc <= 0)
+    return fail(OI_EINVAL, "oi_band_spectrum_fft_c64: bad arguments");
+  const int nx1 = n1_of(nx), ny1 = n1_of(ny);
+  if (!nx1 || !ny1) return fail(OI_ERANGE, "oi_band_spectrum_fft_c64: grid %dx%d is not 256..2048, power of 2", ny, nx);
+  const int maxc = max(abs(m0c), abs(m0c + bc - 1));
+  if (2 * maxc >= nx || br > ny || (long long)batch * nch > 0x7fffffffLL)
+    return fail(OI_ERANGE, "oi_band_spectrum_fft_c64: band (%d+%d, %d+%d) too wide for %dx%d", m0r, br, m0c, bc, ny, nx);
+  cudaStream_t s = (cudaStream_t)stream;
+  float2* t = (float2*)scratch;
+  if (int rc = band_rows(nx1, field, OI_FIELD_COMPLEX_C64, batch, ny, nch, m0c, bc, wn_x, t, s)) return rc;
+  const float2* wy = (const float2*)wn_y;
+  switch (ny1) {
+    case 8: return cols_fwd<8>(t, batch * nch, bc, wy, m0r, br, scale, (float2*)band, s);
+    case 16: return cols_fwd<16>(t, batch * nch, bc, wy, m0r, br, scale, (float2*)band, s);
+    case 32: return cols_fwd<32>(t, batch * nch, bc, wy, m0r, br, scale, (float2*)band, s);
+    default: return cols_fwd<64>(t, batch * nch, bc, wy, m0r, br, scale, (float2*)band, s);
   }
 }
 
@@ -924,13 +1071,7 @@ extern "C" int oi_coarse_half_spectrum_fft(const float* coarse, int nparts, int 
   const int nq = 2 * br - 1, m0r = -(br - 1);
   const float scale = 1.f / ((float)mr * (float)mc);
   const long long pstride = (long long)count * mr * mc;
-  int rc;
-  switch (nx1) {
-    case 8: rc = band_fft<8>(coarse, OI_FIELD_REAL_F32, count, mr, mc, m0r, nq, 0, bc, (const float2*)wn_c, (const float2*)wn_r, scale, t, out, s, nparts, pstride); break;
-    case 16: rc = band_fft<16>(coarse, OI_FIELD_REAL_F32, count, mr, mc, m0r, nq, 0, bc, (const float2*)wn_c, (const float2*)wn_r, scale, t, out, s, nparts, pstride); break;
-    case 32: rc = band_fft<32>(coarse, OI_FIELD_REAL_F32, count, mr, mc, m0r, nq, 0, bc, (const float2*)wn_c, (const float2*)wn_r, scale, t, out, s, nparts, pstride); break;
-    default: rc = band_fft<64>(coarse, OI_FIELD_REAL_F32, count, mr, mc, m0r, nq, 0, bc, (const float2*)wn_c, (const float2*)wn_r, scale, t, out, s, nparts, pstride); break;
-  }
+  int rc = band_rows(nx1, coarse, OI_FIELD_REAL_F32, count, mr, 1, 0, bc, wn_c, t, s, nparts, pstride);
   if (rc) return rc;
   switch (ny1) {
     case 8: return cols_fwd<8>(t, count, bc, (const float2*)wn_r, m0r, nq, scale, out, s, 0, 1);

@@ -266,7 +266,7 @@ def band_spectrum(field: torch.Tensor, kind: int, plan: Plan, nch: int = 1, scal
 
     field: float32 [B, ny, nx] (FIELD_REAL_F32), uint8 [B, ny, nx] (FIELD_U8) or complex64 [B, ny, nx, nch]
     (FIELD_COMPLEX_C64), contiguous on the plan's device.  `scale` multiplies the 1/(ny nx) normalisation.
-    form: 'fft' (default where the grid allows: real or uint8 masks on 256..2048 power-of-two grids) or 'dft'.
+    form: 'fft' (default where the grid allows: 256..2048 power-of-two grids) or 'dft'.
     """
     b = plan.band
     batch = field.shape[0]
@@ -284,6 +284,9 @@ def band_spectrum(field: torch.Tensor, kind: int, plan: Plan, nch: int = 1, scal
                N.ptr(plan.rows_consts(0)), N.ptr(plan.wn_y), sc, N.ptr(scratch), N.ptr(band), s)
     elif plan.use_fft(form) and kind != N.FIELD_COMPLEX_C64 and nch == 1:
         N.call('oi_band_spectrum_fft', N.ptr(field), kind, batch, plan.ny, plan.nx, b.m0r, b.br, b.m0c, b.bc,
+               N.ptr(plan.wn_x), N.ptr(plan.wn_y), sc, N.ptr(scratch), N.ptr(band), s)
+    elif plan.use_fft(form) and kind == N.FIELD_COMPLEX_C64:
+        N.call('oi_band_spectrum_fft_c64', N.ptr(field), batch, plan.ny, plan.nx, nch, b.m0r, b.br, b.m0c, b.bc,
                N.ptr(plan.wn_x), N.ptr(plan.wn_y), sc, N.ptr(scratch), N.ptr(band), s)
     else:
         N.call('oi_band_spectrum', N.ptr(field), kind, batch, plan.ny, plan.nx, nch, b.br, b.bc, N.ptr(plan.wx),
