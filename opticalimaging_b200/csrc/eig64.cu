@@ -608,10 +608,11 @@ __global__ void output_kernel(int n, int p, int k, const double2* __restrict__ X
 constexpr int SMS = 148, GRAM_BLOCKS = 2 * SMS;
 
 // Shares of the K loop for `tiles` output tiles and `chunks` chunks of K: four blocks per SM (two are resident; tiles
-// differ in their non-zero blocks, and smaller shares even that out), at least four chunks each, at most 32 shares.
+// differ in their non-zero blocks, and smaller shares even that out), at least eight chunks each (each share is an array the
+// fold reads), at most 32 shares.
 static int shares(int tiles, int chunks) {
   const int s = std::max(1, 4 * SMS / tiles);
-  return std::max(1, std::min(std::min(s, 32), chunks / 4));
+  return std::max(1, std::min(std::min(s, 32), chunks / 8));
 }
 
 struct Sizes {

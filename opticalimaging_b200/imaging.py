@@ -543,8 +543,8 @@ def _placement(n, length):
     return (n - length + 1) // 2 + n // 2 - n
 
 
-def socs_kernels_from_tcc(tcc, FG_ValidSize, Nfg, numerics) -> SocsKernels:
-    """Top-K SOCS kernels sqrt(lambda_k) u_k in band form, placed as the reference places them."""
+def _socs_from_tcc(tcc, FG_ValidSize, Nfg, numerics):
+    """Top-K SOCS kernels sqrt(lambda_k) u_k [K, br, bc] complex64 and their band, placed as the reference places them."""
     nf, ng = Nfg
     lg, lf = FG_ValidSize
     if lf > ng or lg > nf:
@@ -559,38 +559,47 @@ def socs_kernels_from_tcc(tcc, FG_ValidSize, Nfg, numerics) -> SocsKernels:
         lam, U = _eig_desc(tcc)
         k = _socs_count(numerics, lam, U.shape[1])
     kb = (U[:, :k] * torch.sqrt(lam[:k])).T.reshape(k, lf, lg)
-    band = Band(_placement(ng, lf), lf, _placement(nf, lg), lg)
-    return SocsKernels(kb.to(torch.complex64), band, ng, nf)
+    return kb.to(torch.complex64), Band(_placement(ng, lf), lf, _placement(nf, lg), lg)
 
 
-def socs_kernels_from_pupils(h, FG_ValidSize, Nfg, numerics) -> SocsKernels:
-    """Top-K SOCS kernels from the pupil matrix h [ne, FG, S] of TCC = sum_e h_e h_e^H, without forming the TCC
-    when its rank bound ne*S is below FG: with H = [h_0 | .. | h_ne-1] (FG x ne*S), the Gram matrix H^H H has the
-    TCC's non-zero eigenvalues, and its eigenvectors v give the kernels sqrt(lambda) u = H v (FP64 on the device).
-    Kernels equal socs_kernels_from_tcc's up to a phase per kernel (images are unchanged)."""
+def socs_kernels_from_tcc(tcc, FG_ValidSize, Nfg, numerics) -> SocsKernels:
+    """Top-K SOCS kernels sqrt(lambda_k) u_k in band form, placed as the reference places them."""
+    kb, band = _socs_from_tcc(tcc, FG_ValidSize, Nfg, numerics)
+    return SocsKernels(kb, band, Nfg[1], Nfg[0])
+
+
+def _socs_from_pupils(h, FG_ValidSize, Nfg, numerics):
+    """_socs_from_tcc for TCC = sum_e h_e h_e^H given by the pupil matrix h [ne, FG, S], without forming the TCC when its
+    rank bound ne*S is below FG: with H = [h_0 | .. | h_ne-1] (FG x ne*S), the Gram matrix H^H H has the TCC's non-zero
+    eigenvalues, and its eigenvectors v give the kernels sqrt(lambda) u = H v (FP64 on the device)."""
     ne, fg, s = h.shape
     if ne * s >= fg:
-        return socs_kernels_from_tcc(_assemble_tcc(h), FG_ValidSize, Nfg, numerics)
+        return _socs_from_tcc(_assemble_tcc(h), FG_ValidSize, Nfg, numerics)
     nf, ng = Nfg
     lg, lf = FG_ValidSize
     if lf > ng or lg > nf:
         raise ValueError(f'TCC grid {lf}x{lg} does not fit the {ng}x{nf} image grid')
+    band = Band(_placement(ng, lf), lf, _placement(nf, lg), lg)
     top = None
     if numerics.Hopkins_SettingType.lower() == 'order':   # leading kernels of h h^H, the TCC never formed
         top = eig_topk(min(numerics.Hopkins_Order, fg - 1, ne * s), h=h)
     if top is not None:
         lam, U = top
-        k = lam.numel()
-        kb = (U * torch.sqrt(lam)).T.reshape(k, lf, lg)
-        band = Band(_placement(ng, lf), lf, _placement(nf, lg), lg)
-        return SocsKernels(kb.to(torch.complex64).contiguous(), band, ng, nf)
+        kb = (U * torch.sqrt(lam)).T.reshape(lam.numel(), lf, lg)
+        return kb.to(torch.complex64).contiguous(), band
     H = h.permute(1, 0, 2).reshape(fg, ne * s)
     lam, V = torch.linalg.eigh(H.conj().T @ H)
     lam, V = torch.clamp(lam.flip(0), min=0), V.flip(1)
     k = min(_socs_count(numerics, lam, fg), V.shape[1])   # kernels past the rank bound are zero
     kb = (H @ V[:, :k]).T.reshape(k, lf, lg)
-    band = Band(_placement(ng, lf), lf, _placement(nf, lg), lg)
-    return SocsKernels(kb.to(torch.complex64).contiguous(), band, ng, nf)
+    return kb.to(torch.complex64).contiguous(), band
+
+
+def socs_kernels_from_pupils(h, FG_ValidSize, Nfg, numerics) -> SocsKernels:
+    """Top-K SOCS kernels from the pupil matrix h [ne, FG, S] of TCC = sum_e h_e h_e^H, without forming the TCC when its
+    rank bound ne*S is below FG.  Kernels equal socs_kernels_from_tcc's up to a phase per kernel (images are unchanged)."""
+    kb, band = _socs_from_pupils(h, FG_ValidSize, Nfg, numerics)
+    return SocsKernels(kb, band, Nfg[1], Nfg[0])
 
 
 def DecomposeTCC_SOCS(TCCMatrix_Stacked, FG_ValidSize, Nfg, numerics):
@@ -633,14 +642,13 @@ def socs_model(source, projector, numerics, period_y, period_x, ny, nx, focus=No
     sets = []
     for z in zs:
         h, fg = tcc_pupil_matrix(source, [period_y, period_x], projector, z, numerics)
-        sets.append(socs_kernels_from_pupils(h, fg, [nx, ny], numerics))
-    k = max(s.count for s in sets)   # 'threshold' may keep a different count per plane: pad with zero kernels
-    pupils = torch.zeros((len(zs), k, sets[0].band.br, sets[0].band.bc), dtype=torch.complex64,
-                         device=sets[0].kernels.device)
-    for i, s in enumerate(sets):
-        pupils[i, :s.count] = s.kernels
-    return CoherentModel(pupils, torch.ones((len(zs), k), device=pupils.device), sets[0].band, ny, nx, 'socs',
-                         pack=pack)
+        sets.append(_socs_from_pupils(h, fg, [nx, ny], numerics))   # bare kernels: only the model below is packed
+    k = max(kb.shape[0] for kb, _ in sets)   # 'threshold' may keep a different count per plane: pad with zero kernels
+    band = sets[0][1]
+    pupils = torch.zeros((len(zs), k, band.br, band.bc), dtype=torch.complex64, device=sets[0][0].device)
+    for i, (kb, _) in enumerate(sets):
+        pupils[i, :kb.shape[0]] = kb
+    return CoherentModel(pupils, torch.ones((len(zs), k), device=pupils.device), band, ny, nx, 'socs', pack=pack)
 
 
 def hopkins_intensity(source, scatter, projector, numerics, h=None):
