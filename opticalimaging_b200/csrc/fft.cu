@@ -122,25 +122,6 @@ __device__ __forceinline__ float2 outer_bin(const float2* ys, const float2* t1, 
   for (int n1 = 0; n1 < N1; ++n1) cfma(acc, row[n1], sgn<SIGN>(tw[n1]));
   return acc;
 }
-// Two bins at once (ka, kb), each summed in two interleaved halves: four independent chains.
-template <int SIGN, int N1>
-__device__ __forceinline__ void outer_bin2(const float2* ys, const float2* t1, int ka, int kb, float2& va, float2& vb) {
-  const float2* ra = ys + (ka & 31) * (N1 + 1);
-  const float2* rb = ys + (kb & 31) * (N1 + 1);
-  const float2* ta = t1 + (ka >> 5) * N1;
-  const float2* tb = t1 + (kb >> 5) * N1;
-  float2 a0 = make_float2(0.f, 0.f), a1 = a0, b0 = a0, b1 = a0;
-#pragma unroll 4
-  for (int n1 = 0; n1 < N1; n1 += 2) {
-    cfma(a0, ra[n1], sgn<SIGN>(ta[n1]));
-    cfma(a1, ra[n1 + 1], sgn<SIGN>(ta[n1 + 1]));
-    cfma(b0, rb[n1], sgn<SIGN>(tb[n1]));
-    cfma(b1, rb[n1 + 1], sgn<SIGN>(tb[n1 + 1]));
-  }
-  va = make_float2(a0.x + a1.x, a0.y + a1.y);
-  vb = make_float2(b0.x + b1.x, b0.y + b1.y);
-}
-
 // --------------------------------------------------------------------------------- forward, rows
 // cos(2 pi t / 64) for t = 0..16 (exact decimal expansions of the standard values; the even ones are c32's), and for any
 // t >= 0.  Inlined without recursion, so that a constant t leaves a constant.
@@ -328,8 +309,10 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-template <int N1, bool SYM>
-__global__ void __launch_bounds__(COLS_T, 6) fft_cols_fwd_kernel(const float2* __restrict__ t, long long ncols, int bc,
+// H: the bins lie within [-32 H, 32 H) (0: any); they come from outer_sums, as the row pass's (one bin per thread at a time
+// with loaded twiddles: 8 images of 1024 x 1024, 59 x 59 band 5.4 us, now 4.0; 4 of 2048, 117 x 117 10.0, now 6.1).
+template <int N1, bool SYM, int H>
+__global__ void __launch_bounds__(COLS_T, H == 4 ? 4 : 6) fft_cols_fwd_kernel(const float2* __restrict__ t, long long ncols, int bc,
                                                               const float2* __restrict__ wn_g, int m0r, int br,
                                                               float scale, float2* __restrict__ band, int bco,
                                                               int dbl_from) {
@@ -365,26 +348,49 @@ __global__ void __launch_bounds__(COLS_T, 6) fft_cols_fwd_kernel(const float2* _
   float2* yg = ys + g * 32 * (N1 + 1);
   twiddle_store<+1, N1>(z, t2, n1, yg);
   __syncthreads();
-  if (col >= ncols) return;
-  const long long b = col / bc;
-  const int ic = (int)(col - b * bc);
-  if (!SYM) {   // columns ic >= dbl_from are doubled (a Hermitian half-spectrum standing for both halves)
-    const float sc = ic >= dbl_from ? 2.f * scale : scale;
-    for (int ir = n1; ir < br; ir += N1) {
-      float2 v = outer_bin<+1, N1>(yg, t1, (m0r + ir) & (N - 1));
+  const bool live = col < ncols;
+  const long long b = live ? col / bc : 0;
+  const int ic = (int)(col - b * bc), half = (bco - 1) / 2;
+  // columns ic >= dbl_from are doubled (a Hermitian half-spectrum standing for both halves)
+  const float sc = !SYM && ic >= dbl_from ? 2.f * scale : scale;
+  auto put = [&](int ir, float2 v) {
+    if (!SYM) {
       band[(b * br + ir) * (long long)bc + ic] = make_float2(v.x * sc, v.y * sc);
+    } else {
+      band[(b * br + ir) * (long long)bco + half + ic] = make_float2(v.x * sc, v.y * sc);
+      if (ic > 0) band[(b * br + br - 1 - ir) * (long long)bco + half - ic] = make_float2(v.x * sc, -v.y * sc);
     }
-  } else {   // bins ir and ir + N1 together
-    const int h = (bco - 1) / 2;
-    for (int ir = n1; ir < br; ir += 2 * N1) {
-      float2 v[2];
-      outer_bin2<+1, N1>(yg, t1, (m0r + ir) & (N - 1), (m0r + ir + N1) & (N - 1), v[0], v[1]);
+  };
+  if constexpr (H == 0) {
+    if (!live) return;
+    for (int ir = n1; ir < br; ir += N1) put(ir, outer_bin<+1, N1>(yg, t1, (m0r + ir) & (N - 1)));
+  } else {
+    // k2 = n1 + N1 j, all N1 terms; N1 = 64: half of the terms per thread, met in shared memory (as in the row pass)
+    constexpr int NT = N1 < 32 ? N1 : 32;
+    const bool upper = N1 == 64 && n1 >= 32;
+    float2* zs = ys + G * 32 * (N1 + 1);   // [G][32][2 H], N1 = 64 only
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int r = ir + u * N1;
-        if (r >= br) break;
-        band[(b * br + r) * (long long)bco + h + ic] = make_float2(v[u].x * scale, v[u].y * scale);
-        if (ic > 0) band[(b * br + br - 1 - r) * (long long)bco + h - ic] = make_float2(v[u].x * scale, -v[u].y * scale);
+    for (int k2 = n1 & 31; k2 < 32; k2 += NT) {
+      float2 o[2 * H];
+      outer_sums<N1, H, NT>(o, yg + k2 * (N1 + 1) + (upper ? 32 : 0));
+      if constexpr (N1 == 64) {
+        if (upper) {
+#pragma unroll
+          for (int i = 0; i < 2 * H; ++i) zs[(g * 32 + k2) * 2 * H + i] = o[i];
+        }
+        __syncthreads();
+        if (upper) continue;
+#pragma unroll
+        for (int i = 0; i < 2 * H; ++i) {
+          const float2 v = zs[(g * 32 + k2) * 2 * H + i];
+          const float sg = (i - H) & 1 ? -1.f : 1.f;
+          o[i] = make_float2(fmaf(sg, v.x, o[i].x), fmaf(sg, v.y, o[i].y));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2 * H; ++i) {
+        const int ir = k2 + 32 * (i - H) - m0r;
+        if (live && ir >= 0 && ir < br) put(ir, o[i]);
       }
     }
   }
@@ -632,7 +638,7 @@ __global__ void __launch_bounds__(COARSE_T) coarse_rows_kernel(const float* __re
     float4 acc[PER];
 #pragma unroll
     for (int k = 0; k < PER; ++k) acc[k] = __ldg(src + LOADERS * k);
-#pragma unroll 4
+#pragma unroll(PER <= 2 ? 8 / PER : 4)   // an Abbe image of a few fields per block has up to a hundred parts
     for (int p = 1; p < nparts; ++p) {
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
@@ -686,8 +692,11 @@ __global__ void __launch_bounds__(COARSE_T) coarse_cols_kernel(long long ncols, 
   float2* us = (float2*)smem_raw;           // [G][MR]
   float2* ys = us + G * MR;                 // [G][32][N1R + 1]
   float2* cs = ys + G * 32 * (N1R + 1);     // [G][nq]
+  __shared__ float2 t1[N1R * N1R];          // exp(+2 pi i k1 n1 / N1R)
   const int tid = threadIdx.x;
   const long long col0 = (long long)blockIdx.x * G;
+  const int qc0 = (int)(col0 % bc);         // band column of the block's first
+  if (tid < N1R * N1R) t1[tid] = __ldg(wr + ((32 * (tid / N1R) * (tid % N1R)) & (MR - 1)));
   for (int e = tid; e < G * MR; e += COARSE_T) {
     const int g = e / MR;
     us[e] = col0 + g < ncols ? v[(col0 + g) * N + e % MR] : make_float2(0.f, 0.f);
@@ -706,17 +715,22 @@ __global__ void __launch_bounds__(COARSE_T) coarse_cols_kernel(long long ncols, 
     }
   }
   __syncthreads();
-  for (int e = tid; e < G * nq; e += COARSE_T) {
-    const int g = e / nq, jr = e - g * nq, k = (jr - (br - 1)) & (MR - 1);
-    const float2* y = ys + (g * 32 + (k & 31)) * (N1R + 1);
-    float2 a = make_float2(0.f, 0.f);
+  // thread: column g = tid / N1, bins tid % N1 + N1 i
+  const int g = tid / N1, n1 = tid % N1;
+  {
+    const float s = (qc0 + g) % bc == 0 ? norm : 2.f * norm;
+    const float2* yg = ys + g * 32 * (N1R + 1);
+#pragma unroll 4
+    for (int jr = n1; jr < nq; jr += N1) {
+      const int k = (jr - (br - 1)) & (MR - 1);
+      const float2* y = yg + (k & 31) * (N1R + 1);
+      float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int n1 = 0; n1 < N1R; ++n1) cfma(a, y[n1], __ldg(wr + ((32 * (k >> 5) * n1) & (MR - 1))));
-    const float s = (col0 + g) % bc == 0 ? norm : 2.f * norm;
-    cs[e] = make_float2(a.x * s, a.y * s);
+      for (int i = 0; i < N1R; ++i) cfma(a, y[i], t1[(k >> 5) * N1R + i]);
+      cs[g * nq + jr] = make_float2(a.x * s, a.y * s);
+    }
   }
   __syncthreads();
-  const int g = tid / N1, n1 = tid % N1;
   if (col0 + g >= ncols) return;
   inverse_gather<N1, H>(z, cs + g * nq, br - 1, wn_g, wn_g + 32 * N1, n1);
   float2* dst = v + (col0 + g) * N;
@@ -836,8 +850,8 @@ static int launch_coarse_spec_fft(float* coarse, int nparts, int count, int br, 
 
 template <int N1>
 static size_t smem_rows_fwd(int nu) { return sizeof(float2) * ((256 / N1) * 32 * (N1 + 1) + (256 / N1) * nu); }
-template <int N1>
-static size_t smem_cols_fwd() { return sizeof(float2) * ((COLS_T / N1) * 32 * (N1 + 1)); }
+template <int N1, int H>
+static size_t smem_cols_fwd() { return sizeof(float2) * ((COLS_T / N1) * 32 * (N1 + 1 + (N1 == 64 ? 2 * H : 0))); }
 
 
 template <int N1, int KIND, int H>
@@ -890,19 +904,28 @@ static int band_rows(int nx1, const void* field, int kind, int batch, int ny, in
 }
 
 // bco: the output band width (SYM: bc = (bco + 1) / 2 input columns; else bco = bc)
+template <int N1, bool SYM, int H>
+static int cols_fwd_h(const float2* t, long long ncols, int bc, const float2* wn_y, int m0r, int br, float scale,
+                      float2* band, cudaStream_t s, int bco, int dbl_from) {
+  constexpr int G = COLS_T / N1;
+  const size_t smem = smem_cols_fwd<N1, H>();
+  if (int rc = set_smem(fft_cols_fwd_kernel<N1, SYM, H>, smem, "oi_band_spectrum_fft/cols")) return rc;
+  (void)launch_pdl(fft_cols_fwd_kernel<N1, SYM, H>, dim3((unsigned)ceil_div(ncols, G)), dim3(COLS_T), smem, s, t, ncols, bc,
+                   wn_y, m0r, br, scale, band, bco, dbl_from);
+  oi::note_launch();
+  return check_launch("oi_band_spectrum_fft/cols");
+}
 template <int N1, bool SYM = false>
 static int cols_fwd(const float2* t, int batch, int bc, const float2* wn_y, int m0r, int br, float scale,
                     float2* band, cudaStream_t s, int bco = 0, int dbl_from = 0x7fffffff) {
-  constexpr int G = COLS_T / N1;
   if ((uintptr_t)t % 16) return fail(OI_EINVAL, "oi_band_spectrum_fft/cols: scratch must be 16-byte aligned");
-  size_t smem = smem_cols_fwd<N1>();
-  int rc = set_smem(fft_cols_fwd_kernel<N1, SYM>, smem, "oi_band_spectrum_fft/cols");
-  if (rc) return rc;
   const long long ncols = (long long)batch * bc;
-  (void)launch_pdl(fft_cols_fwd_kernel<N1, SYM>, dim3((unsigned)ceil_div(ncols, G)), dim3(COLS_T), smem, s,
-                   (const float2*)t, ncols, bc, wn_y, m0r, br, scale, band, SYM ? bco : bc, dbl_from);
-  oi::note_launch();
-  return check_launch("oi_band_spectrum_fft/cols");
+  bco = SYM ? bco : bc;
+  auto within = [&](int h) { return m0r >= -32 * h && m0r + br <= 32 * h; };
+  if (within(1)) return cols_fwd_h<N1, SYM, 1>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  if (within(2)) return cols_fwd_h<N1, SYM, 2>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  if (within(4)) return cols_fwd_h<N1, SYM, 4>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  return cols_fwd_h<N1, SYM, 0>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
 }
 
 template <int N1, int H>
