@@ -89,6 +89,13 @@ OI_API int oi_band_spectrum(const void* field, int kind, int batch, int ny, int 
                             const void* wx, const void* wy, float scale, void* scratch, void* band, void* stream);
 
 /*
+ * oi_band_spectrum for one real channel (float32 or uint8 masks) on band columns m0c .. m0c+bc-1 that hold frequency 0: half
+ * the products of the row pass (t[-k] = conj t[k]).  scratch: batch * ny * max(bc, |largest column frequency| + 1) complex.
+ */
+OI_API int oi_band_spectrum_real(const void* field, int kind, int batch, int ny, int nx, int br, int m0c, int bc,
+                                 const void* wx, const void* wy, float scale, void* scratch, void* band, void* stream);
+
+/*
  * oi_band_spectrum without a scratch argument, for callers that cannot allocate device memory -- code handed
  * only the pointers of a host application that owns every allocation, or running inside a memory budget that
  * is already fully given out.  No counterpart in the reference (which allocates freely through torch).

@@ -17,6 +17,7 @@ _SIGS = {
     'oi_version': [],
     'oi_twiddle': [_vp, _i, _i, _ll, _ll, _ll, _i, _d, _vp],
     'oi_band_spectrum': [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp, _vp],
+    'oi_band_spectrum_real': [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp, _vp],
     'oi_abbe_pupils': [_vp, _vp, _i, _i, _vp, _vp, _vp, _i, _d, _vp, _i, _vp, _i, _vp, _d, _d, _d, _d, _vp, _vp,
                        _vp],
     'oi_coherent_coarse': [_vp, _i, _i, _i, _i, _vp, _ll, _vp, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp],

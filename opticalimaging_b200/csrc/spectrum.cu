@@ -38,6 +38,47 @@ template <int KIND> struct BandX {
   __device__ __forceinline__ void put(int, int R, int ic, float2 v) const { t[(r0 + R) * bc + ic] = v; }
 };
 
+// A real field's row transform on a band that holds frequency 0: t[-k] = conj t[k], so the x pass forms k = 0 .. kc-1 only
+// (kc - 1 the largest |frequency|; a k beyond the band's own end is the conjugate of the column at -k) and the y pass reads
+// the others mirrored.  Half the products of the x pass: four 1000 x 750 masks, 35 -> 19.7 us.
+template <int KIND> struct BandXHalf {
+  using A = float;
+  static constexpr bool A_K = true;
+  const void* field;
+  long long r0;
+  int nx, bc, m0c, kc;
+  const float2* wx;
+  float2* t;
+  __device__ __forceinline__ float a(int, int R, int x) const {
+    return KIND == OI_FIELD_U8 ? (float)__ldg((const uint8_t*)field + (r0 + R) * nx + x)
+                               : __ldg((const float*)field + (r0 + R) * nx + x);
+  }
+  __device__ __forceinline__ float2 b(int, int x, int k) const {
+    const bool own = k < m0c + bc;
+    const float2 w = __ldg(wx + (long long)x * bc + (own ? k : -k) - m0c);
+    return own ? w : make_float2(w.x, -w.y);
+  }
+  __device__ __forceinline__ void put(int, int R, int k, float2 v) const { t[(r0 + R) * kc + k] = v; }
+};
+struct BandYHalf {
+  using A = float2;
+  static constexpr bool A_K = false;
+  const float2* t;
+  int ny, br, bc, m0c, kc;
+  const float2* wy;
+  float scale;
+  float2* band;
+  __device__ __forceinline__ float2 a(int, int ir, int y) const { return __ldg(wy + (long long)y * br + ir); }
+  __device__ __forceinline__ float2 b(int mat, int y, int ic) const {
+    const int m = m0c + ic;
+    const float2 v = t[((long long)mat * ny + y) * kc + (m < 0 ? -m : m)];
+    return m < 0 ? make_float2(v.x, -v.y) : v;
+  }
+  __device__ __forceinline__ void put(int mat, int ir, int ic, float2 v) const {
+    band[((long long)mat * br + ir) * bc + ic] = make_float2(v.x * scale, v.y * scale);
+  }
+};
+
 // pass y: per image-channel matrix, band = scale * wy^T t.
 struct BandY {
   using A = float2;
@@ -65,7 +106,40 @@ static int band_x(const void* field, int batch, int ny, int nx, int nch, int bc,
   return OI_OK;
 }
 
+template <int KIND>
+static int band_half(const void* field, int batch, int ny, int nx, int m0c, int br, int bc, const float2* wx, const float2* wy,
+                     float scale, float2* t, float2* band, cudaStream_t s) {
+  const int kc = max(-m0c, m0c + bc - 1) + 1;
+  const long long rows = (long long)batch * ny, slice = 1LL << 30;
+  for (long long r0 = 0; r0 < rows; r0 += slice) {
+    const int n = (int)(rows - r0 < slice ? rows - r0 : slice);
+    const BandXHalf<KIND> op{field, r0, nx, bc, m0c, kc, wx, t};
+    const int rc = kc <= 32 ? dg::gemm<128, 32, 8, 2>(op, 1, n, kc, nx, s, "oi_band_spectrum_real/x")
+                            : dg::gemm<64, 64, 4, 4>(op, 1, n, kc, nx, s, "oi_band_spectrum_real/x");
+    if (rc) return rc;
+  }
+  return dg::gemm<32, 32, 2, 2>(BandYHalf{t, ny, br, bc, m0c, kc, wy, scale, band}, batch, br, bc, ny, s,
+                                "oi_band_spectrum_real/y");
+}
+
 }  // namespace oi
+
+extern "C" int oi_band_spectrum_real(const void* field, int kind, int batch, int ny, int nx, int br, int m0c, int bc,
+                                     const void* wx, const void* wy, float scale, void* scratch, void* band,
+                                     void* stream) {
+  using namespace oi;
+  if (!field || !wx || !wy || !scratch || !band || batch <= 0 || ny <= 0 || nx <= 0 || br <= 0 || bc <= 0)
+    return fail(OI_EINVAL, "oi_band_spectrum_real: bad arguments (batch=%d ny=%d nx=%d br=%d bc=%d)", batch, ny, nx, br, bc);
+  if (kind != OI_FIELD_REAL_F32 && kind != OI_FIELD_U8)
+    return fail(OI_EINVAL, "oi_band_spectrum_real: real float32 or uint8 masks only (kind=%d)", kind);
+  if (batch > 65535) return fail(OI_ERANGE, "oi_band_spectrum_real: batch too large");
+  if (m0c > 0 || m0c + bc <= 0) return fail(OI_ERANGE, "oi_band_spectrum_real: band %d+%d does not hold frequency 0", m0c, bc);
+  cudaStream_t s = (cudaStream_t)stream;
+  return kind == OI_FIELD_U8 ? band_half<OI_FIELD_U8>(field, batch, ny, nx, m0c, br, bc, (const float2*)wx, (const float2*)wy,
+                                                      scale, (float2*)scratch, (float2*)band, s)
+                             : band_half<OI_FIELD_REAL_F32>(field, batch, ny, nx, m0c, br, bc, (const float2*)wx,
+                                                            (const float2*)wy, scale, (float2*)scratch, (float2*)band, s);
+}
 
 extern "C" int oi_band_spectrum(const void* field, int kind, int batch, int ny, int nx, int nch, int br, int bc,
                                 const void* wx, const void* wy, float scale, void* scratch, void* band,

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256) coarse_spec_kernel(const float* __restric
 
 // The same spectrum as two tile products (dft_gemm.cuh), U = coarse * gc and ihat = gr^T U, when the caller has room for
 // U: the partial sums are added as the first product's operand is read.  Four 128 x 128 coarse images of 59 x 59 bands:
-// 239 us (16 blocks, one output per thread at a time) -> 20 us, and the separate addition of the parts (4 us) goes.
+// 239 us (16 blocks, one output per thread at a time) -> 14 us, and the separate addition of the parts (4 us) goes.
 struct SpecRows {
   using A = float;
   static constexpr bool A_K = true;
@@ -211,8 +211,12 @@ int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, co
   if ((long long)count * mr * bc * (long long)sizeof(float2) <= room_bytes) {
     float2* u = (float2*)room;
     const int nq = 2 * br - 1;
-    int rc = dg::gemm<64, 64, 4, 4>(SpecRows{coarse, nparts, (long long)count * mr * mc, mc, bc, (const float2*)gc, u}, 1,
-                                    count * mr, bc, mc, s, "coarse spectrum/rows");
+    const SpecRows op{coarse, nparts, (long long)count * mr * mc, mc, bc, (const float2*)gc, u};
+    // 32 x 32 tiles until the 64 x 64 ones alone fill the SMs (148): K is too short for a cluster to make up for it
+    // (four 128 x 128 images: 14.7 us as 64 x 64 tiles, 8.9 as 32 x 32)
+    int rc = (long long)ceil_div(count * mr, 64) * ceil_div(bc, 64) >= 148
+                 ? dg::gemm<64, 64, 4, 4>(op, 1, count * mr, bc, mc, s, "coarse spectrum/rows")
+                 : dg::gemm<32, 32, 2, 2>(op, 1, count * mr, bc, mc, s, "coarse spectrum/rows");
     if (rc) return rc;
     return dg::gemm<32, 32, 2, 2>(SpecCols{u, mr, nq, bc, (const float2*)gr, 1.0f / ((float)mr * (float)mc), (float2*)ihat},
                                   count, nq, bc, mr, s, "coarse spectrum/columns");

@@ -288,6 +288,10 @@ def band_spectrum(field: torch.Tensor, kind: int, plan: Plan, nch: int = 1, scal
     elif plan.use_fft(form) and kind == N.FIELD_COMPLEX_C64:
         N.call('oi_band_spectrum_fft_c64', N.ptr(field), batch, plan.ny, plan.nx, nch, b.m0r, b.br, b.m0c, b.bc,
                N.ptr(plan.wn_x), N.ptr(plan.wn_y), sc, N.ptr(scratch), N.ptr(band), s)
+    elif kind != N.FIELD_COMPLEX_C64 and nch == 1 and b.m0c <= 0 < b.m0c + b.bc:
+        # (at most bc columns are formed: a band that holds 0 reaches bc - 1 at most)
+        N.call('oi_band_spectrum_real', N.ptr(field), kind, batch, plan.ny, plan.nx, b.br, b.m0c, b.bc, N.ptr(plan.wx),
+               N.ptr(plan.wy), sc, N.ptr(scratch), N.ptr(band), s)
     else:
         N.call('oi_band_spectrum', N.ptr(field), kind, batch, plan.ny, plan.nx, nch, b.br, b.bc, N.ptr(plan.wx),
                N.ptr(plan.wy), sc, N.ptr(scratch), N.ptr(band), s)

@@ -21,6 +21,10 @@ TOL = 3e-6
     (1, 130, 250, (-30, 59, -32, 65)),
     (2, 500, 333, (-65, 131, -64, 129)),
     (9, 129, 1000, (-29, 59, -30, 59)),
+    (2, 70, 130, (-5, 11, -2, 30)),       # columns up to 27: most of the half are the mirrors of none
+    (2, 70, 130, (-5, 11, -27, 28)),      # 0 is the band's end: every other column is a mirror
+    (2, 70, 130, (-5, 11, 3, 20)),        # without frequency 0: the general product
+    (200, 20, 100, (-3, 7, -31, 64)),
 ])
 def test_band_spectrum(kind, batch, ny, nx, band):
     from opticalimaging_b200 import engine as eng, _native as N
