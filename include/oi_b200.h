@@ -174,8 +174,10 @@ OI_API int oi_coarse_to_image(float* coarse, int nparts, int count, int mr, int 
  *   buffer.  scratch: float2 [batch * bc * ny].  band: float2 [batch][br][bc].
  * oi_coarse_to_image_fft: as oi_coarse_to_image (same gc, gr tables), with the y and x syntheses done as
  *   pruned inverse FFTs; the coarse input holds `nparts` partial sums one after another (count*mr*mc floats
- *   each).  When wm_r / wm_c (oi_twiddle(1, m, 1, 0, m, +1) for m = mr / mc) are given and mr, mc are 64 or
- *   128, the coarse spectrum is an FFT too (one block per image); else it is the DFT of oi_coarse_to_image.
+ *   each).  When wm_r / wm_c (oi_twiddle(1, m, 1, 0, m, +1) for m = mr / mc) are given and mr, mc are 64, 128
+ *   or 256, the coarse spectrum is an FFT too, in scratch_v, and its columns go on to ny points in the same pass
+ *   (scratch_ihat is not touched); else, and for a coarse that is not 16-byte aligned, it is the DFT of
+ *   oi_coarse_to_image.
  *   scratch_ihat: float2 [count * (2br-1) * bc]; scratch_v: float2 [count * bc * ny].
  */
 OI_API int oi_fft_supported(int ny, int nx);

@@ -1118,7 +1118,8 @@ extern "C" int oi_coarse_to_image_fft(float* coarse, int nparts, int count, int 
   int rc;
   float2* v = (float2*)scratch_v;
   auto small = [](int m) { return m == 64 || m == 128 || m == 256; };
-  if (wm_r && wm_c && small(mr) && small(mc) && mr <= ny && 2 * br - 1 <= mr && 2 * bc - 1 <= mc && count <= 65535) {
+  if (wm_r && wm_c && small(mr) && small(mc) && mr <= ny && 2 * br - 1 <= mr && 2 * bc - 1 <= mc && count <= 65535 &&
+      (uintptr_t)coarse % alignof(float4) == 0) {
     const float2 *tr = (const float2*)wm_r, *tc = (const float2*)wm_c;
     rc = mc == 64    ? coarse_rows<2>(coarse, nparts, count, mr, bc, tc, ny, v, s)
          : mc == 128 ? coarse_rows<4>(coarse, nparts, count, mr, bc, tc, ny, v, s)

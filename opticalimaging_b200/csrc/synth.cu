@@ -208,7 +208,8 @@ int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, co
   if (mr < 2 * br - 1 || mc < 2 * bc - 1)
     return fail(OI_EINVAL, "coarse grid %dx%d too small for band %dx%d", mr, mc, br, bc);
   if (mr > 1024 || count > 65535) return fail(OI_ERANGE, "coarse grid mr=%d or count=%d out of range", mr, count);
-  if ((long long)count * mr * bc * (long long)sizeof(float2) <= room_bytes) {
+  // (a caller's images may start at any float; the pairs of U may not)
+  if ((long long)count * mr * bc * (long long)sizeof(float2) <= room_bytes && (uintptr_t)room % alignof(float2) == 0) {
     float2* u = (float2*)room;
     const int nq = 2 * br - 1;
     const SpecRows op{coarse, nparts, (long long)count * mr * mc, mc, bc, (const float2*)gc, u};

@@ -92,3 +92,21 @@ def test_coarse_to_image_dft(nparts, count, m, b, ny, nx):
     ex = np.exp(-2j * np.pi * np.outer(q, np.arange(nx)) / nx)
     want = (ey @ spec @ ex).real
     assert band.br == b and rel_err(out.cpu().numpy(), want) < TOL
+
+
+def test_coarse_to_image_odd_out():
+    """Images that start at an odd float of their buffer: no room for the spectrum's pairs there, same values."""
+    from opticalimaging_b200 import engine as eng, _native as N
+    dev = torch.device('cuda')
+    m, b, ny, nx = 64, 20, 70, 90
+    plan = eng.Plan(ny, nx, eng.Band(0, b, 0, b), dev, coarse=(m, m))
+    parts = torch.rand((3, 2, m, m), generator=torch.Generator().manual_seed(1)).to(dev)
+    ihat = torch.empty(2 * (2 * b - 1) * b, dtype=torch.complex64, device=dev)
+    images = []
+    for shift in (0, 1):
+        c, buf = parts.clone(), torch.empty(2 * ny * nx + 1, device=dev)
+        out = buf[shift:shift + 2 * ny * nx]
+        N.call('oi_coarse_to_image', N.ptr(c), 3, 2, m, m, b, b, N.ptr(plan.gc), N.ptr(plan.gr), N.ptr(plan.sy),
+               N.ptr(plan.sx), ny, nx, N.ptr(ihat), N.ptr(out), N.stream_handle())
+        images.append(out.cpu().numpy())
+    assert rel_err(images[1], images[0]) < TOL
