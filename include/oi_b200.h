@@ -332,6 +332,16 @@ OI_API int oi_coarse_half_spectrum_fft(const float* coarse, int nparts, int coun
                                        const void* wn_c, const void* wn_r, void* scratch, void* ihat, void* stream);
 
 /*
+ * The adjoint's coarse copy of an image gradient g [count][ny][nx] (256..2048 per axis, powers of two) on 128 x 128 points:
+ *   out[i][s] = scale sum_{|qr| < br, |qc| < bc} ghat_i(q) exp(-2 pi i q.s / 128), ghat_i(q) = sum_r g_i(r) exp(+2 pi i q.r / N)
+ * br, bc <= 64.  wn_x / wn_y / wn_m: the FFT tables of nx, ny and 128 points; wm: oi_twiddle(1, 128, 1, 0, 128, +1).
+ * scratch: float2 [count * bc * (ny + 128)], 16-byte aligned.
+ */
+OI_API int oi_coarse_gradient_fft(const float* g, int count, int ny, int nx, int br, int bc, const void* wn_x,
+                                  const void* wn_y, const void* wn_m, const void* wm, float scale, void* scratch,
+                                  float* out, void* stream);
+
+/*
  * Adjoint of the coherent sum (inverse lithography; no counterpart in the reference, whose gradients come from
  * torch autograd through its FFTs).  For fields A_f = P[z][k] .* band[b][c] and the band-limited coarse copy
  * gcoarse[b][z] (mr x mc = 128 x 128) of dL/dI:

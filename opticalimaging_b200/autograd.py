@@ -64,16 +64,14 @@ def _coarse_gradient(model: CoherentModel, g: torch.Tensor, scale: float) -> tor
     ib = Band(-(b.br - 1), 2 * b.br - 1, 0, b.bc)                     # image band, Hermitian half in x
     gplan = Plan.get(ny, nx, ib, model.device)
     g = g.reshape(B * Z, ny, nx).contiguous()
-    if gplan.fft:   # the half-spectrum with qc > 0 doubled, 1 / (ny nx) folded out of the last scale
-        t = torch.empty(B * Z * ny * b.bc, dtype=torch.complex64, device=model.device)
-        gh = torch.empty((B * Z, 2 * b.br - 1, b.bc), dtype=torch.complex64, device=model.device)
-        N.call('oi_coarse_half_spectrum_fft', N.ptr(g), 1, B * Z, ny, nx, b.br, b.bc, N.ptr(gplan.wn_x),
-               N.ptr(gplan.wn_y), N.ptr(t), N.ptr(gh), N.stream_handle(model.device))
-        if scale * ny * nx != 1.0:
-            gh = gh * (scale * ny * nx)
-    else:
-        gh = band_spectrum(g, N.FIELD_REAL_F32, gplan, scale=scale * ny * nx)[:, 0]   # [B*Z, 2br-1, bc]
-        gh[:, :, 1:] *= 2.0
+    if gplan.fft:
+        t = torch.empty(B * Z * b.bc * (ny + plan.mr), dtype=torch.complex64, device=model.device)
+        gc = torch.empty((B, Z, plan.mr, plan.mc), dtype=torch.float32, device=model.device)
+        N.call('oi_coarse_gradient_fft', N.ptr(g), B * Z, ny, nx, b.br, b.bc, N.ptr(gplan.wn_x), N.ptr(gplan.wn_y),
+               N.ptr(plan.coarse_fft_tables()[0]), N.ptr(plan.wm_c), scale, N.ptr(t), N.ptr(gc), N.stream_handle(model.device))
+        return gc
+    gh = band_spectrum(g, N.FIELD_REAL_F32, gplan, scale=scale * ny * nx)[:, 0]   # [B*Z, 2br-1, bc]
+    gh[:, :, 1:] *= 2.0
     return _half_spectrum_to_image(gh, b.br, b.bc, plan.mr, plan.mc).view(B, Z, plan.mr, plan.mc)
 
 

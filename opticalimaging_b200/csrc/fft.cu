@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_fwd_kernel(const
 
 // ------------------------------------------------------------------------------ forward, columns
 // t[b][ic][y] (N = ny) -> band[b][ir][ic] = scale * sum_y t exp(+2 pi i (m0r+ir) y / ny).
-// SYM: t holds the non-negative columns kx = 0 .. bc-1 of a real mask's row transform and the band is the
+// COLS_SYM: t holds the non-negative columns kx = 0 .. bc-1 of a real mask's row transform and the band is the
 // symmetric bco x br band (m0c = -(bco-1)/2, m0r = -(br-1)/2): column kx lands at ic = kx + (bco-1)/2 and, for
 // kx > 0, its mirror band[-ky][-kx] = conj(band[ky][kx]) at row br-1-ir, column (bco-1)/2 - kx.
 // Blocks of COLS_T threads (G = COLS_T / N1 columns each, 32 KB of t): the block's columns are contiguous in t
@@ -299,7 +299,14 @@ __global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_fwd_kernel(const
 // another thread's progress), from where each thread reads its 32 strided values; the twiddled rows then reuse
 // the same shared memory.  At the symmetric band's 30 columns per image a batch of 64 has 1920 columns: 480
 // blocks, all resident at once.
-constexpr int COLS_T = 128;
+// COLS_COARSE: the bins stay in shared memory and go on to GRAD_M points, band[col][s] = sum_q bin(q) exp(-2 pi i q s /
+// GRAD_M), |q| <= (br-1) / 2 < GRAD_M / 2 (wn_m: that transform's tables), four threads per column.
+constexpr int COLS_T = 128, GRAD_M = 128;
+enum ColsMode { COLS_BAND, COLS_SYM, COLS_COARSE };
+
+template <int N1, int H>
+__device__ __forceinline__ void inverse_gather(float2 (&z)[32], const float2* cq, int qmax, const float2* t2, const float2* t1,
+                                               int n1);
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -311,12 +318,13 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // H: the bins lie within [-32 H, 32 H) (0: any); they come from outer_sums, as the row pass's (one bin per thread at a time
 // with loaded twiddles: 8 images of 1024 x 1024, 59 x 59 band 5.4 us, now 4.0; 4 of 2048, 117 x 117 10.0, now 6.1).
-template <int N1, bool SYM, int H>
+template <int N1, ColsMode MODE, int H>
 __global__ void __launch_bounds__(COLS_T, H == 4 ? 4 : 6) fft_cols_fwd_kernel(const float2* __restrict__ t, long long ncols, int bc,
                                                               const float2* __restrict__ wn_g, int m0r, int br,
                                                               float scale, float2* __restrict__ band, int bco,
-                                                              int dbl_from) {
+                                                              int dbl_from, const float2* __restrict__ wn_m) {
   constexpr int N = 32 * N1, G = COLS_T / N1;
+  constexpr bool SYM = MODE == COLS_SYM;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const float2* t2 = wn_g;
   const float2* t1 = wn_g + 32 * N1;
@@ -353,8 +361,11 @@ __global__ void __launch_bounds__(COLS_T, H == 4 ? 4 : 6) fft_cols_fwd_kernel(co
   const int ic = (int)(col - b * bc), half = (bco - 1) / 2;
   // columns ic >= dbl_from are doubled (a Hermitian half-spectrum standing for both halves)
   const float sc = !SYM && ic >= dbl_from ? 2.f * scale : scale;
+  float2* cs = ys + G * 32 * (N1 + 1 + (N1 == 64 ? 2 * H : 0));   // [G][br], COLS_COARSE only
   auto put = [&](int ir, float2 v) {
-    if (!SYM) {
+    if (MODE == COLS_COARSE) {
+      cs[g * br + ir] = make_float2(v.x * sc, v.y * sc);
+    } else if (!SYM) {
       band[(b * br + ir) * (long long)bc + ic] = make_float2(v.x * sc, v.y * sc);
     } else {
       band[(b * br + ir) * (long long)bco + half + ic] = make_float2(v.x * sc, v.y * sc);
@@ -393,6 +404,52 @@ __global__ void __launch_bounds__(COLS_T, H == 4 ? 4 : 6) fft_cols_fwd_kernel(co
         if (live && ir >= 0 && ir < br) put(ir, o[i]);
       }
     }
+  }
+  if constexpr (MODE == COLS_COARSE) {
+    constexpr int M1 = GRAD_M / 32;
+    __syncthreads();
+    const int gm = tid / M1, nm = tid % M1;
+    if (gm >= G || col0 + gm >= ncols) return;
+    inverse_gather<M1, 2>(z, cs + gm * br, (br - 1) / 2, wn_m, wn_m + 32 * M1, nm);
+    float2* dst = band + (col0 + gm) * GRAD_M;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) dst[nm + M1 * bitrev5(i)] = z[i];
+  }
+}
+
+// v[i][qc][y] (qc < bc, y < GRAD_M; qc > 0 doubled) -> out[i][y][x] = sum_qc Re(v exp(-2 pi i qc x / GRAD_M)): 2 R rows per
+// block, a thread per column x and row group; column x + GRAD_M / 2 differs by the sign of the odd terms.  One read of v per
+// row and a table of GRAD_M twiddles; bound: latency.  8 images of 1024 x 1024, 59 x 59 band: the gradient's coarse copy was
+// 5.5 (bins) + 16.7 (a DFT that summed each row's spectrum per block) us after its row pass, now 9.9 + 4.8.
+template <int R>
+__global__ void __launch_bounds__(GRAD_M) coarse_gradient_rows_kernel(const float2* __restrict__ v, int bc,
+                                                                      const float2* __restrict__ wm, float* __restrict__ out) {
+  constexpr int ROWS = 2 * R, X = GRAD_M / 2;
+  __shared__ float2 vs[X][ROWS], tab[GRAD_M];   // bc <= X
+  const int tid = threadIdx.x, y0 = blockIdx.x * ROWS;
+  const long long i = blockIdx.y;
+  tab[tid] = __ldg(wm + tid);
+  for (int e = tid; e < bc * ROWS; e += GRAD_M) vs[e / ROWS][e % ROWS] = __ldg(v + (i * bc + e / ROWS) * GRAD_M + y0 + e % ROWS);
+  __syncthreads();
+  const int x = tid % X, g = tid / X * R;
+  float acc[2][R] = {};   // sums of the even and the odd qc
+  for (int q = 0; q < bc; q += 2) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (q + u >= bc) break;
+      const float2 w = tab[((q + u) * x) & (GRAD_M - 1)];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float2 c = vs[q + u][g + r];
+        acc[u][r] = fmaf(c.x, w.x, fmaf(c.y, w.y, acc[u][r]));
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float* o = out + (i * GRAD_M + y0 + g + r) * GRAD_M + x;
+    o[0] = acc[0][r] + acc[1][r];
+    o[X] = acc[0][r] - acc[1][r];
   }
 }
 
@@ -904,14 +961,14 @@ static int band_rows(int nx1, const void* field, int kind, int batch, int ny, in
 }
 
 // bco: the output band width (SYM: bc = (bco + 1) / 2 input columns; else bco = bc)
-template <int N1, bool SYM, int H>
+template <int N1, ColsMode MODE, int H>
 static int cols_fwd_h(const float2* t, long long ncols, int bc, const float2* wn_y, int m0r, int br, float scale,
-                      float2* band, cudaStream_t s, int bco, int dbl_from) {
+                      float2* band, cudaStream_t s, int bco, int dbl_from, const float2* wn_m = nullptr) {
   constexpr int G = COLS_T / N1;
-  const size_t smem = smem_cols_fwd<N1, H>();
-  if (int rc = set_smem(fft_cols_fwd_kernel<N1, SYM, H>, smem, "oi_band_spectrum_fft/cols")) return rc;
-  (void)launch_pdl(fft_cols_fwd_kernel<N1, SYM, H>, dim3((unsigned)ceil_div(ncols, G)), dim3(COLS_T), smem, s, t, ncols, bc,
-                   wn_y, m0r, br, scale, band, bco, dbl_from);
+  const size_t smem = smem_cols_fwd<N1, H>() + (MODE == COLS_COARSE ? sizeof(float2) * G * br : 0);
+  if (int rc = set_smem(fft_cols_fwd_kernel<N1, MODE, H>, smem, "oi_band_spectrum_fft/cols")) return rc;
+  (void)launch_pdl(fft_cols_fwd_kernel<N1, MODE, H>, dim3((unsigned)ceil_div(ncols, G)), dim3(COLS_T), smem, s, t, ncols, bc,
+                   wn_y, m0r, br, scale, band, bco, dbl_from, wn_m);
   oi::note_launch();
   return check_launch("oi_band_spectrum_fft/cols");
 }
@@ -921,11 +978,22 @@ static int cols_fwd(const float2* t, int batch, int bc, const float2* wn_y, int 
   if ((uintptr_t)t % 16) return fail(OI_EINVAL, "oi_band_spectrum_fft/cols: scratch must be 16-byte aligned");
   const long long ncols = (long long)batch * bc;
   bco = SYM ? bco : bc;
+  constexpr ColsMode MODE = SYM ? COLS_SYM : COLS_BAND;
   auto within = [&](int h) { return m0r >= -32 * h && m0r + br <= 32 * h; };
-  if (within(1)) return cols_fwd_h<N1, SYM, 1>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
-  if (within(2)) return cols_fwd_h<N1, SYM, 2>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
-  if (within(4)) return cols_fwd_h<N1, SYM, 4>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
-  return cols_fwd_h<N1, SYM, 0>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  if (within(1)) return cols_fwd_h<N1, MODE, 1>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  if (within(2)) return cols_fwd_h<N1, MODE, 2>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  if (within(4)) return cols_fwd_h<N1, MODE, 4>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+  return cols_fwd_h<N1, MODE, 0>(t, ncols, bc, wn_y, m0r, br, scale, band, s, bco, dbl_from);
+}
+
+// Columns of GRAD_M points from the columns of ny = 32 N1 in t (br frequencies per side, the positive columns doubled)
+template <int N1>
+static int cols_coarse(const float2* t, int count, int bc, const float2* wn_y, int br, float scale, const float2* wn_m, float2* v,
+                       cudaStream_t s) {
+  const long long ncols = (long long)count * bc;
+  const int nq = 2 * br - 1;
+  return br <= 32 ? cols_fwd_h<N1, COLS_COARSE, 1>(t, ncols, bc, wn_y, 1 - br, nq, scale, v, s, bc, 1, wn_m)
+                  : cols_fwd_h<N1, COLS_COARSE, 2>(t, ncols, bc, wn_y, 1 - br, nq, scale, v, s, bc, 1, wn_m);
 }
 
 template <int N1, int H>
@@ -1102,6 +1170,40 @@ extern "C" int oi_coarse_half_spectrum_fft(const float* coarse, int nparts, int 
     case 32: return cols_fwd<32>(t, count, bc, (const float2*)wn_r, m0r, nq, scale, out, s, 0, 1);
     default: return cols_fwd<64>(t, count, bc, (const float2*)wn_r, m0r, nq, scale, out, s, 0, 1);
   }
+}
+
+// out[i][s] = scale sum_{|qr| < br, |qc| < bc} ghat_i(q) exp(-2 pi i q.s / 128) on 128 x 128 points, ghat_i(q) = sum_r g_i(r)
+// exp(+2 pi i q.r / N) over the ny x nx grid (256..2048, powers of two); br, bc <= 64.
+extern "C" int oi_coarse_gradient_fft(const float* g, int count, int ny, int nx, int br, int bc, const void* wn_x,
+                                      const void* wn_y, const void* wn_m, const void* wm, float scale, void* scratch,
+                                      float* out, void* stream) {
+  using namespace oi;
+  if (!g || !wn_x || !wn_y || !wn_m || !wm || !scratch || !out || count <= 0 || br <= 0 || bc <= 0)
+    return fail(OI_EINVAL, "oi_coarse_gradient_fft: bad arguments");
+  const int nx1 = n1_of(nx), ny1 = n1_of(ny);
+  if (!nx1 || !ny1) return fail(OI_ERANGE, "oi_coarse_gradient_fft: grid %dx%d is not 256..2048, power of 2", ny, nx);
+  if (br > GRAD_M / 2 || bc > GRAD_M / 2 || count > 65535)
+    return fail(OI_ERANGE, "oi_coarse_gradient_fft: band %dx%d or count %d out of range", br, bc, count);
+  if ((uintptr_t)scratch % 16) return fail(OI_EINVAL, "oi_coarse_gradient_fft: scratch must be 16-byte aligned");
+  cudaStream_t s = (cudaStream_t)stream;
+  float2 *t = (float2*)scratch, *v = t + (long long)count * bc * ny;
+  const float2 *wy = (const float2*)wn_y, *wv = (const float2*)wn_m;
+  int rc = band_rows(nx1, g, OI_FIELD_REAL_F32, count, ny, 1, 0, bc, wn_x, t, s);
+  if (rc) return rc;
+  switch (ny1) {
+    case 8: rc = cols_coarse<8>(t, count, bc, wy, br, scale, wv, v, s); break;
+    case 16: rc = cols_coarse<16>(t, count, bc, wy, br, scale, wv, v, s); break;
+    case 32: rc = cols_coarse<32>(t, count, bc, wy, br, scale, wv, v, s); break;
+    default: rc = cols_coarse<64>(t, count, bc, wy, br, scale, wv, v, s); break;
+  }
+  if (rc) return rc;
+  // four rows per block while that gives every SM (148) a block, else two
+  if ((long long)count * (GRAD_M / 4) >= 148)
+    coarse_gradient_rows_kernel<2><<<dim3(GRAD_M / 4, count), GRAD_M, 0, s>>>(v, bc, (const float2*)wm, out);
+  else
+    coarse_gradient_rows_kernel<1><<<dim3(GRAD_M / 2, count), GRAD_M, 0, s>>>(v, bc, (const float2*)wm, out);
+  oi::note_launch();
+  return check_launch("oi_coarse_gradient_fft/rows");
 }
 
 extern "C" int oi_coarse_to_image_fft(float* coarse, int nparts, int count, int mr, int mc, int br, int bc,
