@@ -493,10 +493,76 @@ __device__ __forceinline__ void inverse_gather(float2 (&z)[32], const float2* cq
 // The H of a band of b frequencies per side (qmax = b - 1).  For N1 = 8 (N = 256) 32 H must stay below N / 2 + 1.
 __host__ __device__ constexpr int gather_blocks(int b) { return b <= 64 ? 2 : b <= 128 ? 4 : 0; }
 
+// exp(-2 pi i b k / L) sums of L = 4 or 8 values (b = 0 .. L-1, natural order in and out)
+__device__ __forceinline__ void dft_short(float2 (&v)[4]) {
+  const float2 a = make_float2(v[0].x + v[2].x, v[0].y + v[2].y), b = make_float2(v[0].x - v[2].x, v[0].y - v[2].y);
+  const float2 c = make_float2(v[1].x + v[3].x, v[1].y + v[3].y), d = make_float2(v[1].y - v[3].y, v[3].x - v[1].x);
+  v[0] = make_float2(a.x + c.x, a.y + c.y);
+  v[1] = make_float2(b.x + d.x, b.y + d.y);
+  v[2] = make_float2(a.x - c.x, a.y - c.y);
+  v[3] = make_float2(b.x - d.x, b.y - d.y);
+}
+__device__ __forceinline__ void dft_short(float2 (&v)[8]) {
+  float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+  dft_short(e);
+  dft_short(o);
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const float2 w = rot32<-1>(o[b], 4 * b);
+    v[b] = make_float2(e[b].x + w.x, e[b].y + w.y);
+    v[b + 4] = make_float2(e[b].x - w.x, e[b].y - w.y);
+  }
+}
+
+// inverse_gather for |q| < 32 H in two steps: ys[k2][n1] (row stride N1 + 1; the group's own) = sum_k1 coef(k2 + 32 k1)
+// W_N1^{-k1 n1} for all n1 of a k2 by one thread, 2 H inputs as N1 / (2 H) short transforms with constant twiddles; a
+// barrier of the block; then each thread its column n1.  The gather's 2 H terms per value (8 H instructions with their
+// loads) become about 8 and an exchange, and with fewer values live at a time three blocks of H = 4 share an SM's registers
+// where two did.  Rows of 4 images of 2048 x 2048, 117 columns: 37.7 -> 27.1 us (30.9 with two blocks); of 8 of 1024 x 1024,
+// 59 columns: 16.4 before and after.
+template <int N1, int H>
+__device__ __forceinline__ void inverse_outer(float2 (&z)[32], const float2* cq, int qmax, float2* ys, const float2* t2, int n1) {
+  constexpr int L = 2 * H, A = N1 / L, NT = N1 < 32 ? N1 : 32, AT = N1 == 64 ? A / 2 : A;
+  const bool upper = N1 == 64 && n1 >= 32;   // N1 = 64: two threads per k2, the upper one offset by AT in n1
+  const float2* c0 = cq + qmax;
+#pragma unroll
+  for (int k2 = n1 & 31; k2 < 32; k2 += NT) {
+    float2 c[L];
+#pragma unroll
+    for (int i = 0; i < L; ++i) {
+      const int k1 = i < H ? i : i - L, q = k2 + 32 * k1;
+      c[i] = q <= qmax && q >= -qmax ? c0[q] : make_float2(0.f, 0.f);
+      if constexpr (N1 == 64) {
+        const float2 r = cmul(c[i], make_float2(c64(64 / N1 * k1 * AT), -s64(64 / N1 * k1 * AT)));
+        if (upper) c[i] = r;
+      }
+    }
+    float2* row = ys + k2 * (N1 + 1) + (upper ? AT : 0);
+#pragma unroll
+    for (int a = 0; a < AT; ++a) {
+      float2 v[L];
+#pragma unroll
+      for (int i = 0; i < L; ++i) {
+        const int t = 64 / N1 * (i < H ? i : i - L) * a;
+        v[i] = t == 0 ? c[i] : cmul(c[i], make_float2(c64(t), -s64(t)));
+      }
+      dft_short(v);
+#pragma unroll
+      for (int b = 0; b < L; ++b) row[a + A * b] = v[b];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k2 = 0; k2 < 32; ++k2) z[k2] = cmul(ys[k2 * (N1 + 1) + n1], sgn<-1>(t2[k2 * N1 + n1]));
+  fft32<-1>(z);
+}
+// complex values of ys for the 256 / N1 groups of a block
+template <int N1, int H> __host__ __device__ constexpr int outer_f2() { return H ? 256 / N1 * 32 * (N1 + 1) : 0; }
+
 // ------------------------------------------------------------------------------ inverse, columns
 // ihat[i][jr][qc] (qr = jr - (br-1)) -> v[i][qc][y] = sum_qr ihat exp(-2 pi i qr y / ny)
 template <int N1, int H>
-__global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_cols_inv_kernel(const float2* __restrict__ ihat, long long ncols, int br,
+__global__ void __launch_bounds__(256, 3) fft_cols_inv_kernel(const float2* __restrict__ ihat, long long ncols, int br,
                                                            int bc, const float2* __restrict__ wn_g,
                                                            float2* __restrict__ v) {
   constexpr int N = 32 * N1, G = 256 / N1;
@@ -504,7 +570,8 @@ __global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_cols_inv_kernel(const
   const float2* t2 = wn_g;
   const float2* t1 = wn_g + 32 * N1;
   const int nq = 2 * br - 1;
-  float2* cs = (float2*)smem_raw;  // [G][nq]
+  float2* ys = (float2*)smem_raw;        // [G][32][N1 + 1] (H > 0)
+  float2* cs = ys + outer_f2<N1, H>();   // [G][nq]
   const int tid = threadIdx.x, g = tid / N1, n1 = tid % N1;
   const long long col0 = (long long)blockIdx.x * G;
   for (int e = tid; e < G * nq; e += 256) {
@@ -521,7 +588,8 @@ __global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_cols_inv_kernel(const
   __syncthreads();
   const long long col = col0 + g;
   float2 z[32];
-  inverse_gather<N1, H>(z, cs + g * nq, br - 1, t2, t1, n1);
+  if constexpr (H > 0) inverse_outer<N1, H>(z, cs + g * nq, br - 1, ys + g * 32 * (N1 + 1), t2, n1);
+  else inverse_gather<N1, H>(z, cs + g * nq, br - 1, t2, t1, n1);
   if (col >= ncols) return;
   float2* dst = v + col * N;
 #pragma unroll
@@ -617,7 +685,7 @@ static int cols_inv_tiles(const float2* ihat, int count, int br, int bc, int ny,
 // --------------------------------------------------------------------------------- inverse, rows
 // v[i][qc][y] (qc = 0..bc-1, qc > 0 doubled) -> out[i][y][x] = sum_qc Re(v exp(-2 pi i qc x / nx))
 template <int N1, int H>
-__global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_inv_kernel(const float2* __restrict__ v, long long nrows, int ny,
+__global__ void __launch_bounds__(256, 3) fft_rows_inv_kernel(const float2* __restrict__ v, long long nrows, int ny,
                                                            int bc, const float2* __restrict__ wn_g,
                                                            float* __restrict__ out) {
   constexpr int N = 32 * N1, G = 256 / N1;
@@ -625,8 +693,8 @@ __global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_inv_kernel(const
   const float2* t2 = wn_g;
   const float2* t1 = wn_g + 32 * N1;
   const int nq = 2 * bc - 1;
-  float2* vs = (float2*)smem_raw;      // [bc][2G + 1] (padded against bank conflicts)
-  float2* cs = vs + bc * (2 * G + 1);  // [G][nq]
+  float2* vs = (float2*)smem_raw;      // [bc][2G + 1] (padded against bank conflicts), then [G][32][N1 + 1] (H > 0)
+  float2* cs = vs + max(bc * (2 * G + 1), outer_f2<N1, H>());   // [G][nq]
   const int tid = threadIdx.x, g = tid / N1, n1 = tid % N1;
   const long long rblk = (long long)blockIdx.x * (2 * G);
   for (int e = tid; e < bc * 2 * G; e += 256) {
@@ -655,7 +723,8 @@ __global__ void __launch_bounds__(256, H == 4 ? 2 : 3) fft_rows_inv_kernel(const
   __syncthreads();
   const long long r0 = rblk + 2 * g;
   float2 z[32];
-  inverse_gather<N1, H>(z, cs + g * nq, bc - 1, t2, t1, n1);
+  if constexpr (H > 0) inverse_outer<N1, H>(z, cs + g * nq, bc - 1, vs + g * 32 * (N1 + 1), t2, n1);
+  else inverse_gather<N1, H>(z, cs + g * nq, bc - 1, t2, t1, n1);
   if (r0 >= nrows) return;
   float* o0 = out + r0 * N;
   float* o1 = o0 + N;
@@ -999,7 +1068,7 @@ static int cols_coarse(const float2* t, int count, int bc, const float2* wn_y, i
 template <int N1, int H>
 static int cols_inv_h(const float2* ihat, int count, int br, int bc, const float2* wn_y, float2* v, cudaStream_t s) {
   constexpr int G = 256 / N1;
-  size_t smem = sizeof(float2) * (G * (2 * br - 1));
+  size_t smem = sizeof(float2) * (outer_f2<N1, H>() + G * (2 * br - 1));
   int rc = set_smem(fft_cols_inv_kernel<N1, H>, smem, "oi_coarse_to_image_fft/cols");
   if (rc) return rc;
   const long long ncols = (long long)count * bc;
@@ -1019,7 +1088,7 @@ static int cols_inv(const float2* ihat, int count, int br, int bc, const float2*
 template <int N1, int H>
 static int rows_inv_h(const float2* v, int count, int ny, int bc, const float2* wn_x, float* out, cudaStream_t s) {
   constexpr int G = 256 / N1;
-  size_t smem = sizeof(float2) * (bc * (2 * G + 1) + G * (2 * bc - 1));
+  size_t smem = sizeof(float2) * (max(bc * (2 * G + 1), outer_f2<N1, H>()) + G * (2 * bc - 1));
   int rc = set_smem(fft_rows_inv_kernel<N1, H>, smem, "oi_coarse_to_image_fft/rows");
   if (rc) return rc;
   const long long nrows = (long long)count * ny;
