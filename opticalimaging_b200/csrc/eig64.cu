@@ -32,16 +32,18 @@ namespace oi {
 namespace zg {
 
 __global__ void __launch_bounds__(256) mark_blocks_kernel(const double2* __restrict__ M, int rows, int cols,
-                                                          unsigned char* __restrict__ flags, int fc) {
+                                                          unsigned char* __restrict__ flags, int fc,
+                                                          const int* __restrict__ perm) {
   const int col = blockIdx.x * 256 + threadIdx.x, r16 = blockIdx.y;
   const double2* m = M + (long long)blockIdx.z * rows * cols;
   bool nz = false, bad = false;
   if (col < cols) {
+    const int pc = perm ? __ldg(perm + col) : col;
 #pragma unroll 4
     for (int i = 0; i < KC; ++i) {
       const int r = r16 * KC + i;
       if (r >= rows) break;
-      const double2 v = __ldg(m + (long long)r * cols + col);
+      const double2 v = __ldg(m + (long long)(perm ? __ldg(perm + r) : r) * cols + pc);
       nz |= v.x != 0.0 || v.y != 0.0;
       bad |= !isfinite(v.x) || !isfinite(v.y);
     }
@@ -55,10 +57,10 @@ __global__ void __launch_bounds__(256) mark_blocks_kernel(const double2* __restr
   }
 }
 
-int mark_blocks(const double2* M, int batch, int rows, int cols, unsigned char* flags, cudaStream_t s) {
+int mark_blocks(const double2* M, int batch, int rows, int cols, unsigned char* flags, cudaStream_t s, const int* perm) {
   dim3 grid((unsigned)ceil_div(cols, 256), (unsigned)flag_dim(rows), (unsigned)batch);
   if (grid.y > 65535 || grid.z > 65535) return fail(OI_ERANGE, "mark_blocks: %d x %d x %d too large", batch, rows, cols);
-  mark_blocks_kernel<<<grid, 256, 0, s>>>(M, rows, cols, flags, flag_dim(cols));
+  mark_blocks_kernel<<<grid, 256, 0, s>>>(M, rows, cols, flags, flag_dim(cols), perm);
   note_launch();
   return check_launch("mark_blocks");
 }
@@ -94,6 +96,7 @@ struct GemmArgs {
   double2* parts;
   const unsigned char* flags;    // of M (zg::mark_blocks)
   int fr, fc;
+  const int* perm;               // the order of a dense T's rows and columns (null: its own)
 };
 template <bool AH>
 __global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs a) {
@@ -118,6 +121,8 @@ __global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs a) {
     const int e = c / per, k0 = (c - e * per) * zg::KC;
     if (AH)
       zg::load_cols(As, M, a.m, m0, a.m, k0, a.k);
+    else if (a.perm)
+      zg::load_rows_perm(As, M, a.k, m0, a.m, k0, a.k, a.perm);
     else
       zg::load_rows(As, M + e * a.sm, a.k, m0, a.m, k0, a.k);
     zg::load_cols(Bs, a.B + (long long)e * a.k * a.p, a.p, 0, a.p, k0, a.k);
@@ -128,6 +133,45 @@ __global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs a) {
     const int r = m0 + zg::tile_row() + i, c = zg::tile_col() + j;
     if (r < a.m && c < a.p) out[(long long)r * a.p + c] = v;
   });
+}
+
+// The order of a dense T's indices: those with a zero on the diagonal (of a Hermitian, positive semi-definite T the
+// ones whose whole row and column are zero: frequencies outside every shifted pupil) go to the two ends, so that the
+// others fill whole tiles in the middle.  Any order gives the same eigenpairs, only the number of non-zero blocks
+// differs: 0.62 -> 0.41 of the blocks of a 3481 x 3481 TCC, whose whole set-up takes 5.97 ms instead of 6.58.  One block;
+// perm[place] = index.
+__global__ void __launch_bounds__(1024) order_kernel(int n, const double2* __restrict__ T, int* __restrict__ perm) {
+  __shared__ int wsum[32];
+  const int tid = threadIdx.x, lane = tid & 31, per = (n + 1023) / 1024, i0 = min(n, tid * per), i1 = min(n, i0 + per);
+  auto on = [&](int i) {
+    const double2 d = __ldg(T + (long long)i * n + i);
+    return !(d.x == 0.0 && d.y == 0.0);
+  };
+  int c = 0;
+  for (int i = i0; i < i1; ++i) c += on(i);
+  int incl = c;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, s);
+    if (lane >= s) incl += v;
+  }
+  if (lane == 31) wsum[tid >> 5] = incl;
+  __syncthreads();
+  int before = incl - c, total = 0;
+  for (int w = 0; w < 32; ++w) {
+    if (w < tid >> 5) before += wsum[w];
+    total += wsum[w];
+  }
+  const int off = (n - total) / 2 / zg::T * zg::T;
+  int zeros = i0 - before;   // zero indices before i0
+  for (int i = i0; i < i1; ++i) {
+    if (on(i)) {
+      perm[off + before++] = i;
+    } else {
+      perm[zeros < off ? zeros : total + zeros] = i;
+      ++zeros;
+    }
+  }
 }
 
 // Row-block kernels: each block takes groups of RB rows (g, g + gridDim.x, ...) of n x p arrays, held in shared memory
@@ -596,11 +640,11 @@ __global__ void __launch_bounds__(1024, 1) heev_jacobi_kernel(int p, const doubl
   for (int e = t; e < p * p; e += 1024) Q[(e / p) * p + place[e % p]] = V[(e / p) * JN + e % p];
 }
 
-// Output: vecs [n][k] = columns 0..k-1 of XQ (row-major n x p), vals[i] = max(w[i], 0).
+// Output: vecs [n][k] = columns 0..k-1 of XQ (row-major n x p, rows in the order perm, if any), vals[i] = max(w[i], 0).
 __global__ void output_kernel(int n, int p, int k, const double2* __restrict__ XQ, const double* __restrict__ w,
-                              double2* vecs, double* vals) {
+                              const int* __restrict__ perm, double2* vecs, double* vals) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < (long long)n * k) vecs[e] = XQ[(e / k) * p + e % k];
+  if (e < (long long)n * k) vecs[(perm ? perm[e / k] : e / k) * k + e % k] = XQ[(e / k) * p + e % k];
   if (e < k) vals[e] = w[e] > 0 ? w[e] : 0.0;
 }
 
@@ -616,9 +660,10 @@ static int shares(int tiles, int chunks) {
 }
 
 struct Sizes {
-  long long np, pp, parts, flags;
+  long long np, pp, parts, flags, perm;
   int ne, s_;
   Sizes(int n, int p, int ne_, int s) : ne(ne_), s_(s) {
+    perm = ne > 0 ? 0 : (long long)n * 4;
     np = (long long)n * p;
     pp = (long long)p * p;
     const int tn = ceil_div(n, zg::T);
@@ -635,7 +680,7 @@ struct Sizes {
   }
   long long wf() const { return (long long)ne * s_ * PMAX; }
   long long complex_values() const { return 2 * np + wf() + 3 * pp + parts + (long long)GRAM_BLOCKS * PMAX * PMAX; }
-  long long bytes(int p) const { return 16 * complex_values() + 8 * ((long long)GRAM_BLOCKS * PMAX + 3 * p) + flags + 256; }
+  long long bytes(int p) const { return 16 * complex_values() + 8 * ((long long)GRAM_BLOCKS * PMAX + 3 * p) + flags + perm + 256; }
 };
 
 struct Solver {
@@ -643,6 +688,7 @@ struct Solver {
   int n, p, ne, seg;           // T: dense (ne = 0, seg = n) or ne pupil matrices [n][seg]
   const double2* M;
   const unsigned char* flags;
+  const int* perm;
   double2 *Wf, *parts, *gparts, *G, *Rinv;
   double* rdiag;
   int status = OI_OK;
@@ -672,13 +718,13 @@ struct Solver {
     const int tn = ceil_div(n, zg::T);
     if (ne > 0) {
       const int ts = ceil_div(seg, zg::T), sh = shares(ts * ne, ceil_div(n, zg::KC));
-      GemmArgs g{M, (long long)n * seg, seg, n, 1, p, in, parts, flags, zg::flag_dim(n), zg::flag_dim(seg)};
+      GemmArgs g{M, (long long)n * seg, seg, n, 1, p, in, parts, flags, zg::flag_dim(n), zg::flag_dim(seg), nullptr};
       run("oi_eig_topk64/gemm", gemm_kernel<true>, dim3(ts, sh, ne), 256, zg::SMEM, g);   // Wf_e = h_e^H in
       fold(FoldArgs{parts, sh, seg, p, 1.0, 0.0, 0.0, nullptr, nullptr, nullptr, Wf, nullptr}, ne);
       B = Wf;
     }
     const int nseg = ne > 0 ? ne : 1, sh = shares(tn, nseg * ceil_div(seg, zg::KC));
-    GemmArgs g{M, (long long)n * seg, n, seg, nseg, p, B, parts, flags, zg::flag_dim(n), zg::flag_dim(seg)};
+    GemmArgs g{M, (long long)n * seg, n, seg, nseg, p, B, parts, flags, zg::flag_dim(n), zg::flag_dim(seg), perm};
     run("oi_eig_topk64/gemm", gemm_kernel<false>, dim3(tn, sh, 1), 256, zg::SMEM, g);
     fold(FoldArgs{parts, sh, n, p, alpha, beta, gamma, b1, b0, left, out, gram ? gparts : nullptr});
   }
@@ -741,8 +787,14 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
   double* rdiag = res + p;
   unsigned char* flags = (unsigned char*)(rdiag + p);
   const double2* M = (const double2*)(dense ? tcc : h);
-  if (int rc = zg::mark_blocks(M, dense ? 1 : ne, n, s, flags, st)) return rc;
-  Solver sv{st, n, p, ne, s, M, flags, Wf, parts, gparts, G, Rinv, rdiag};
+  int* perm = dense ? (int*)(flags + sz.flags) : nullptr;   // flags: a multiple of 16 bytes
+  if (dense) {
+    order_kernel<<<1, 1024, 0, st>>>(n, M, perm);
+    note_launch();
+    if (int rc = check_launch("oi_eig_topk64/order")) return rc;
+  }
+  if (int rc = zg::mark_blocks(M, dense ? 1 : ne, n, s, flags, st, perm)) return rc;
+  Solver sv{st, n, p, ne, s, M, flags, perm, Wf, parts, gparts, G, Rinv, rdiag};
 
   start_block_kernel<<<(unsigned)ceil_div(sz.np, 256), 256, 0, st>>>(Z, sz.np, 0x5eed0f71ull + (unsigned long long)n);
   note_launch();
@@ -842,7 +894,7 @@ extern "C" int oi_eig_topk64(const void* tcc, const void* h, int ne, int n, int 
   if (iters) *iters = converged ? it : -it;
   // X holds the Ritz vectors (columns by descending w)
   output_kernel<<<(unsigned)ceil_div((long long)n * k > p ? (long long)n * k : p, 256), 256, 0, st>>>(
-      n, p, k, X, w, (double2*)vecs, vals);
+      n, p, k, X, w, perm, (double2*)vecs, vals);
   note_launch();
   return check_launch("oi_eig_topk64/output");
 }

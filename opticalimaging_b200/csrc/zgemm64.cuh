@@ -146,6 +146,17 @@ __device__ __forceinline__ void load_rows(double2* s, const double2* src, long l
     cp16(s + k * LD + r, on ? src + (long long)(r0 + r) * ld + k0 + k : src, on);
   }
 }
+// load_rows of the block of src with its rows and columns taken in the order perm.
+__device__ __forceinline__ void load_rows_perm(double2* s, const double2* src, long long ld, int r0, int nr, int k0, int nk,
+                                               const int* __restrict__ perm) {
+  const int k = threadIdx.x & 15, col = k0 + k < nk ? __ldg(perm + k0 + k) : 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = (threadIdx.x >> 4) + 16 * i;
+    const bool on = r0 + r < nr && k0 + k < nk;
+    cp16(s + k * LD + r, on ? src + (long long)__ldg(perm + r0 + r) * ld + col : src, on);
+  }
+}
 __device__ __forceinline__ void load_cols(double2* s, const double2* src, long long ld, int c0, int nc, int k0, int nk) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -157,9 +168,10 @@ __device__ __forceinline__ void load_cols(double2* s, const double2* src, long l
 
 // Marks of the 16 x 16 blocks of M [batch][rows][cols]: flags[b][r16][c16], pitches fr = flag_rows(rows) and
 // fc = flag_cols(cols) (padded to whole 64-row / 64-column tiles); bit 0 a non-zero value, bit 1 a value that is not
-// finite.  One block per 16 rows x 256 columns.
+// finite.  One block per 16 rows x 256 columns.  perm (may be null): the order in which M's rows and columns are taken.
 __host__ __device__ inline int flag_dim(int n) { return (n + T - 1) / T * (T / KC); }
-int mark_blocks(const double2* M, int batch, int rows, int cols, unsigned char* flags, cudaStream_t s);
+int mark_blocks(const double2* M, int batch, int rows, int cols, unsigned char* flags, cudaStream_t s,
+                const int* perm = nullptr);
 
 }  // namespace zg
 }  // namespace oi

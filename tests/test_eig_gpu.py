@@ -61,6 +61,23 @@ def test_factored_matches_dense_and_skips_zero_blocks(ne, s, n):
     assert float((T @ vecs - vecs * vals).norm(dim=0).max()) < 1e-12 * top
 
 
+@pytest.mark.parametrize('n', [64, 130, 961, 2400])
+@pytest.mark.parametrize('live', ['one', 'few', 'most', 'ends'])
+def test_dense_with_zero_rows(n, live):
+    """Zero rows and columns scattered over T, as of frequencies outside every pupil (a pair's residual there is its value times its rows)."""
+    from opticalimaging_b200 import imaging as oi
+    rng = np.random.default_rng(n)
+    on = {'one': rng.permutation(n) < 1, 'few': rng.random(n) < 0.1, 'most': rng.random(n) < 0.9,
+          'ends': np.arange(n) % (n - 1) == 0}[live]
+    h = (rng.standard_normal((n, 40)) + 1j * rng.standard_normal((n, 40))) * on[:, None] * 2.0 ** -np.arange(40)
+    T = torch.from_numpy(h @ h.conj().T).cuda()
+    vals, vecs = oi.eig_topk(4, tcc=T)
+    lam = torch.from_numpy(np.linalg.svd(h, compute_uv=False)[:4] ** 2).cuda()
+    top = float(lam[0])
+    assert float((vals - lam).abs().max()) < 1e-12 * top
+    assert float((T @ vecs - vecs * vals).norm(dim=0).max()) < 1e-12 * top
+
+
 def test_small_blocks_and_the_iteration_limit():
     """The C entry with a block of fewer than 64 vectors, and a limit it cannot meet: the status says so."""
     from opticalimaging_b200 import _native as N
