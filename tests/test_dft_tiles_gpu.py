@@ -68,6 +68,25 @@ def test_spectrum_to_image(count, ny, nx, br, bc):
     assert rel_err(out.cpu().numpy(), want) < TOL
 
 
+@pytest.mark.parametrize('nx', [1, 2, 3, 254, 255, 256, 510, 511, 766, 767, 768, 1022, 1024, 1534, 2048])
+@pytest.mark.parametrize('count,ny', [(1, 5), (150, 9), (150, 17)])
+def test_mirrored_columns(nx, count, ny):
+    """Columns x and nx - x from one product: halves around one to nine groups of 128, rows around half blocks."""
+    from opticalimaging_b200 import engine as eng, _native as N
+    rng = np.random.default_rng(nx + ny)
+    br, bc = 3, min(9, (nx + 1) // 2)
+    ih = (rng.standard_normal((count, 2 * br - 1, bc)) + 1j * rng.standard_normal((count, 2 * br - 1, bc))).astype(np.complex64)
+    dev = torch.device('cuda')
+    t = lambda *a: eng.twiddle(*a, device=dev)  # noqa: E731
+    sy, sx = t(ny, 2 * br - 1, 0, -(br - 1), ny, -1), t(bc, nx, 0, 0, nx, -1)
+    out = torch.full((count, ny, nx), 9.0, device=dev)
+    ihd = torch.from_numpy(ih).to(dev)
+    N.call('oi_spectrum_to_image', N.ptr(ihd), count, br, bc, N.ptr(sy), N.ptr(sx), ny, nx, N.ptr(out), N.stream_handle())
+    ey = np.exp(-2j * np.pi * np.outer(np.arange(ny), np.arange(-(br - 1), br)) / ny)
+    ex = np.exp(-2j * np.pi * np.outer(np.arange(bc), np.arange(nx)) / nx)
+    assert rel_err(out.cpu().numpy(), (ey @ ih.astype(np.complex128) @ ex).real) < TOL
+
+
 @pytest.mark.parametrize('nparts', [1, 2, 5])
 @pytest.mark.parametrize('count,m,b,ny,nx', [(1, 64, 5, 9, 11), (1, 64, 31, 70, 90), (2, 128, 59, 300, 257), (1, 192, 90, 201, 400),
                                              (20, 128, 64, 131, 150)])
