@@ -365,6 +365,11 @@ OI_API int oi_resist_loss_workspace(long long* bytes);
 OI_API int oi_resist_loss(const float* image, const float* target, int batch, int nz, long long n, float steepness,
                           float threshold, float* grad, float* loss, void* work, long long work_bytes, void* stream);
 
+/* oi_resist_loss that also writes s (resist, float32 as the images), when not NULL: d grad / d I follows from grad and s. */
+OI_API int oi_resist_loss_terms(const float* image, const float* target, int batch, int nz, long long n, float steepness,
+                                float threshold, float* grad, float* resist, float* loss, void* work,
+                                long long work_bytes, void* stream);
+
 /*
  * Field weights of an Abbe model for source weights `values` (double [points], device): weights [nz][fields] float32,
  * index_image v_j / sum v for the fields_per_point fields of point j, in the order [state][point][component].

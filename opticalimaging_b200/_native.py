@@ -40,6 +40,7 @@ _SIGS = {
                             _vp],
     'oi_resist_loss_workspace': [_vp],
     'oi_resist_loss': [_vp, _vp, _i, _i, _ll, _f, _f, _vp, _vp, _vp, _ll, _vp],
+    'oi_resist_loss_terms': [_vp, _vp, _i, _i, _ll, _f, _f, _vp, _vp, _vp, _vp, _ll, _vp],
     'oi_source_weights': [_vp, _i, _i, _i, _i, _d, _vp, _vp],
     'oi_source_gradient': [_vp, _i, _i, _i, _i, _i, _vp, _d, _vp, _vp],
     'oi_coherent_field_dots': [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _vp],

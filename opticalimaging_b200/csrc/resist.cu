@@ -1,10 +1,10 @@
 // The parts of an optimisation iteration outside the transforms: the sigmoid resist loss with its image gradient, the
 // field weights of a new source, and the source gradient from the field dot products.  The reference composes the first
 // from torch operations behind its image (CalculateAerialImage_SOCS.py:3-11); as such a composition it was a dozen passes
-// over the images and as many launches (8 images of 1024 x 1024: 107 us forward and backward, now 41), the other two about
-// twenty launches on a few hundred values.
+// over the images and as many launches (8 images of 1024 x 1024: 107 us forward and backward, now 41 and 4 for the s that a
+// recorded backward pass needs), the other two about twenty launches on a few hundred values.
 //
-// Bound: memory for the loss (image and target in, gradient out), the launch for the others.
+// Bound: memory for the loss (image and target in, gradient and s out), the launch for the others.
 #include "oi_common.cuh"
 #include <algorithm>
 #include <cstdint>
@@ -14,15 +14,17 @@ namespace oi {
 constexpr int RL_T = 256, RL_BLOCKS = 148 * 8;
 
 // loss += (s - t)^2, s = 1 / (1 + exp(-a (I - thr))) over images [batch][nz][n] against targets [batch][n]; with grad,
-// grad = 2 (s - t) a s (1 - s).  Sums in FP64, per block to partial[blockIdx.x].
+// grad = 2 (s - t) a s (1 - s), and with resist, resist = s.  Sums in FP64, per block to partial[blockIdx.x].
 template <int V>
 __global__ void __launch_bounds__(RL_T) resist_loss_kernel(const float* __restrict__ image, const float* __restrict__ target,
                                                            int nz, long long n, long long total, float a, float thr,
-                                                           float* __restrict__ grad, double* __restrict__ partial) {
+                                                           float* __restrict__ grad, float* __restrict__ resist,
+                                                           double* __restrict__ partial) {
   __shared__ double sh[RL_T / 32];
   double acc = 0.0;
-  auto one = [&](float I, float t) {
-    const float s = 1.f / (1.f + expf(-(a * (I - thr)))), r = s - t;
+  auto one = [&](float I, float t, float& s) {
+    s = 1.f / (1.f + expf(-(a * (I - thr))));
+    const float r = s - t;
     acc += (double)r * (double)r;
     return 2.f * r * a * (s * (1.f - s));
   };
@@ -30,11 +32,15 @@ __global__ void __launch_bounds__(RL_T) resist_loss_kernel(const float* __restri
     const long long plane = e / n, t0 = (plane / nz) * n + (e - plane * n);
     if constexpr (V == 4) {
       const float4 I = *(const float4*)(image + e), t = *(const float4*)(target + t0);
-      const float4 g = make_float4(one(I.x, t.x), one(I.y, t.y), one(I.z, t.z), one(I.w, t.w));
+      float4 s;
+      const float4 g = make_float4(one(I.x, t.x, s.x), one(I.y, t.y, s.y), one(I.z, t.z, s.z), one(I.w, t.w, s.w));
       if (grad) *(float4*)(grad + e) = g;
+      if (resist) *(float4*)(resist + e) = s;
     } else {
-      const float g = one(image[e], target[t0]);
+      float s;
+      const float g = one(image[e], target[t0], s);
       if (grad) grad[e] = g;
+      if (resist) resist[e] = s;
     }
   }
 #pragma unroll
@@ -113,8 +119,9 @@ extern "C" int oi_resist_loss_workspace(long long* bytes) {
   return OI_OK;
 }
 
-extern "C" int oi_resist_loss(const float* image, const float* target, int batch, int nz, long long n, float steepness,
-                              float threshold, float* grad, float* loss, void* work, long long work_bytes, void* stream) {
+extern "C" int oi_resist_loss_terms(const float* image, const float* target, int batch, int nz, long long n, float steepness,
+                                    float threshold, float* grad, float* resist, float* loss, void* work,
+                                    long long work_bytes, void* stream) {
   using namespace oi;
   if (!image || !target || !loss || !work || batch <= 0 || nz <= 0 || n <= 0)
     return fail(OI_EINVAL, "oi_resist_loss: bad arguments");
@@ -122,17 +129,20 @@ extern "C" int oi_resist_loss(const float* image, const float* target, int batch
     return fail(OI_ERANGE, "oi_resist_loss: %lld workspace bytes given, %lld needed", work_bytes, (long long)sizeof(double) * RL_BLOCKS);
   cudaStream_t s = (cudaStream_t)stream;
   const long long total = (long long)batch * nz * n;
-  const bool v4 = n % 4 == 0 && ((uintptr_t)image | (uintptr_t)target | (uintptr_t)grad) % 16 == 0;
+  const bool v4 = n % 4 == 0 && ((uintptr_t)image | (uintptr_t)target | (uintptr_t)grad | (uintptr_t)resist) % 16 == 0;
   const int blocks = (int)std::min((long long)RL_BLOCKS, (long long)ceil_div(total, RL_T * (v4 ? 4 : 1)));
-  if (v4)
-    resist_loss_kernel<4><<<blocks, RL_T, 0, s>>>(image, target, nz, n, total, steepness, threshold, grad, (double*)work);
-  else
-    resist_loss_kernel<1><<<blocks, RL_T, 0, s>>>(image, target, nz, n, total, steepness, threshold, grad, (double*)work);
+  auto kern = v4 ? resist_loss_kernel<4> : resist_loss_kernel<1>;
+  kern<<<blocks, RL_T, 0, s>>>(image, target, nz, n, total, steepness, threshold, grad, resist, (double*)work);
   note_launch();
   if (int rc = check_launch("oi_resist_loss")) return rc;
   resist_sum_kernel<<<1, RL_T, 0, s>>>((const double*)work, blocks, loss);
   note_launch();
   return check_launch("oi_resist_loss/sum");
+}
+
+extern "C" int oi_resist_loss(const float* image, const float* target, int batch, int nz, long long n, float steepness,
+                              float threshold, float* grad, float* loss, void* work, long long work_bytes, void* stream) {
+  return oi_resist_loss_terms(image, target, batch, nz, n, steepness, threshold, grad, nullptr, loss, work, work_bytes, stream);
 }
 
 extern "C" int oi_source_weights(const double* values, int points, int fields_per_point, int fields, int nz, double index_image,

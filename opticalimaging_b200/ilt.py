@@ -36,37 +36,49 @@ class ResistModel:
         return torch.sigmoid(self.steepness * (image - self.threshold))
 
 
-class _ResistLoss(torch.autograd.Function):
-    """sum (sigmoid(a (I - thr)) - target)^2 in one pass over the images, which also leaves the derivative by the images
-    for the backward pass (no other buffer is saved).  A backward pass that is itself recorded (create_graph) goes through
-    the composition of torch operations instead."""
+class _ResistTerms(torch.autograd.Function):
+    """(loss, D, s) in one pass over the images: loss = sum (s - target)^2, s = sigmoid(a (I - thr)), D = dloss/dI.
+
+    With q = a s (1 - s): dloss = D dI, ds = q dI, dD = (2 q^2 + a D (1 - 2 s)) dI.  D and s are outputs, so that a
+    backward pass that is itself recorded (create_graph) differentiates through them, to any order, and neither the
+    image nor the target is kept: what the caller does with them afterwards changes no derivative."""
 
     @staticmethod
     def forward(ctx, image, target, steepness, threshold):
         img = image.contiguous()
         B, Z, ny, nx = img.shape
-        grad = torch.empty_like(img) if ctx.needs_input_grad[0] else None
+        grad, s = (torch.empty_like(img), torch.empty_like(img)) if ctx.needs_input_grad[0] else (None, None)
         loss = torch.empty((), dtype=torch.float32, device=img.device)
         nbytes = ctypes.c_longlong(0)
         N.call('oi_resist_loss_workspace', ctypes.byref(nbytes))
         work = torch.empty(nbytes.value, dtype=torch.uint8, device=img.device)
-        N.call('oi_resist_loss', N.ptr(img), N.ptr(target), B, Z, ny * nx, steepness, threshold, N.ptr(grad), N.ptr(loss),
-               N.ptr(work), nbytes.value, N.stream_handle(img.device))
+        N.call('oi_resist_loss_terms', N.ptr(img), N.ptr(target), B, Z, ny * nx, steepness, threshold, N.ptr(grad), N.ptr(s),
+               N.ptr(loss), N.ptr(work), nbytes.value, N.stream_handle(img.device))
         if grad is not None:
-            ctx.save_for_backward(grad)
-            ctx.composed = (image, target, steepness, threshold)
-        return loss
+            ctx.set_materialize_grads(False)
+            ctx.steepness = steepness
+            ctx.save_for_backward(grad, s)
+        return loss, grad, s
 
     @staticmethod
-    def backward(ctx, g):
-        if torch.is_grad_enabled():
-            image, target, a, thr = ctx.composed
-            s = torch.sigmoid(a * (image - thr))
-            return g * (2.0 * (s - target[:, None])) * (a * s * (1.0 - s)), None, None, None
-        (grad,) = ctx.saved_tensors
-        if not torch._C._autograd._get_current_graph_task_keep_graph():
-            ctx.composed = None      # freed with the graph, as saved tensors are
-        return grad * g, None, None, None
+    def backward(ctx, g_loss, g_grad, g_s):
+        d, s = ctx.saved_tensors
+        g = None if g_loss is None else d * g_loss
+        if g_grad is not None or g_s is not None:   # from a recorded backward pass
+            a = ctx.steepness
+            q = a * s * (1.0 - s)
+            for g_out, slope in ((g_grad, 2.0 * q * q + a * d * (1.0 - 2.0 * s)), (g_s, q)):
+                if g_out is not None:
+                    g = g_out * slope if g is None else g + g_out * slope
+        return g, None, None, None
+
+
+class _ResistLoss:
+    """sum (sigmoid(a (I - thr)) - target)^2 with its derivatives by the images."""
+
+    @staticmethod
+    def apply(image, target, steepness, threshold):
+        return _ResistTerms.apply(image, target, steepness, threshold)[0]
 
 
 def ilt_loss(model: CoherentModel, mask: torch.Tensor, target: torch.Tensor, resist: ResistModel):
