@@ -84,9 +84,11 @@ class _ResistLoss:
 def ilt_loss(model: CoherentModel, mask: torch.Tensor, target: torch.Tensor, resist: ResistModel):
     """(loss, image): ||R(I(mask)) - target||^2 over pixels and planes; mask [B, ny, nx], target [B, ny, nx]."""
     image = aerial_image(model, mask)                        # [B, Z, ny, nx]
-    # one float32 target per mask and the sigmoid resist itself: the fused loss; any other resist callable, broadcast or
+    # one float32 target per mask and the sigmoid resist itself, its parameters plain numbers: the fused loss; any other
+    # resist callable, parameters that are tensors (they may want a gradient, or differ by pixel), broadcast or
     # differentiable target: torch operations
-    if (type(resist) is ResistModel and target.dtype == torch.float32 and target.device == image.device
+    if (type(resist) is ResistModel and isinstance(resist.steepness, (int, float))
+            and isinstance(resist.threshold, (int, float)) and target.dtype == torch.float32 and target.device == image.device
             and target.shape == (image.shape[0],) + image.shape[2:] and target.is_contiguous()
             and not target.requires_grad):
         return _ResistLoss.apply(image, target, float(resist.steepness), float(resist.threshold)), image
