@@ -110,8 +110,10 @@ def coherent_adjoint(model: CoherentModel, band: torch.Tensor, gc: torch.Tensor,
 
 
 def mask_gradient_from_w(model: CoherentModel, w: torch.Tensor) -> torch.Tensor:
-    """dL/dt [B, ny, nx] = 2/(ny nx) Re sum_{m in band} W(m) exp(-2 pi i m.y/N) for W [B, br, bc]."""
-    return _mask_gradient(model, w.contiguous()[None, :, None], 2.0 / (model.ny * model.nx))
+    """dL/dt [B, ny, nx] = 2/(ny nx) Re sum_{m in band} W(m) exp(-2 pi i m.y/N) for W [B, br, bc] (of any type and device;
+    [B, 1, bc] and the like are broadcast)."""
+    full = torch.empty((w.shape[0], model.band.br, model.band.bc), dtype=torch.complex64, device=model.device).copy_(w)
+    return _mask_gradient(model, full[None, :, None], 2.0 / (model.ny * model.nx))
 
 
 def _mask_gradient(model: CoherentModel, shares: torch.Tensor, scale: float) -> torch.Tensor:
