@@ -126,8 +126,14 @@ def ptr(t):
 
 
 def stream_handle(device=None):
-    """The current CUDA stream of a device (the current one for None) as an integer handle."""
-    index = None if device is None else torch.device(device).index
+    """The current CUDA stream of a device (the current one for None) as an integer handle.  Any other kind of device is
+    refused: calls pass their tensors' device here, and a host tensor's address must not reach a kernel."""
+    index = None
+    if device is not None:
+        d = torch.device(device)
+        if d.type != 'cuda':
+            raise ValueError(f'expected a CUDA device, got {d}')
+        index = d.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
