@@ -1114,10 +1114,14 @@ static int coarse_rows(const float* coarse, int nparts, int count, int mr, int b
   auto run = [&](auto kern, int pairs) {
     const size_t smem = sizeof(float2) * ((size_t)pairs * MC + pairs * 32 * (N1C + 1));
     if (int rc = set_smem(kern, smem, "coarse rows fft")) return rc;
-    kern<<<dim3((unsigned)(mr / (2 * pairs)), (unsigned)count), COARSE_T, smem, s>>>(
-        coarse, nparts, (long long)count * mr * MC, mr, bc, wc, ny, v);
-    oi::note_launch();
-    return check_launch("coarse rows fft");
+    constexpr int MOST = 65535;   // images per launch: the grid's second dimension
+    for (int i = 0; i < count; i += min(MOST, count - i)) {
+      kern<<<dim3((unsigned)(mr / (2 * pairs)), (unsigned)min(MOST, count - i)), COARSE_T, smem, s>>>(
+          coarse + (long long)i * mr * MC, nparts, (long long)count * mr * MC, mr, bc, wc, ny, v + (long long)i * bc * ny);
+      oi::note_launch();
+      if (int rc = check_launch("coarse rows fft")) return rc;
+    }
+    return (int)OI_OK;
   };
   // 16 rows per block write whole 128-byte lines; 8 or 4 rows while that leaves SMs (148) without a block
   if ((long long)count * mr / 16 >= 148) return run(coarse_rows_kernel<N1C, 8>, 8);
@@ -1289,7 +1293,7 @@ extern "C" int oi_coarse_to_image_fft(float* coarse, int nparts, int count, int 
   int rc;
   float2* v = (float2*)scratch_v;
   auto small = [](int m) { return m == 64 || m == 128 || m == 256; };
-  if (wm_r && wm_c && small(mr) && small(mc) && mr <= ny && 2 * br - 1 <= mr && 2 * bc - 1 <= mc && count <= 65535 &&
+  if (wm_r && wm_c && small(mr) && small(mc) && mr <= ny && 2 * br - 1 <= mr && 2 * bc - 1 <= mc &&
       (uintptr_t)coarse % alignof(float4) == 0) {
     const float2 *tr = (const float2*)wm_r, *tc = (const float2*)wm_c;
     rc = mc == 64    ? coarse_rows<2>(coarse, nparts, count, mr, bc, tc, ny, v, s)
