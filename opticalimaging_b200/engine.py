@@ -285,7 +285,8 @@ def band_spectrum(field: torch.Tensor, kind: int, plan: Plan, nch: int = 1, scal
     elif plan.use_fft(form) and kind != N.FIELD_COMPLEX_C64 and nch == 1:
         N.call('oi_band_spectrum_fft', N.ptr(field), kind, batch, plan.ny, plan.nx, b.m0r, b.br, b.m0c, b.bc,
                N.ptr(plan.wn_x), N.ptr(plan.wn_y), sc, N.ptr(scratch), N.ptr(band), s)
-    elif plan.use_fft(form) and kind == N.FIELD_COMPLEX_C64:
+    elif plan.use_fft(form) and kind == N.FIELD_COMPLEX_C64 and N.ptr(scratch) % 16 == 0:
+        # (its column pass copies 16 bytes at a time; a caller's scratch may start at any complex value)
         N.call('oi_band_spectrum_fft_c64', N.ptr(field), batch, plan.ny, plan.nx, nch, b.m0r, b.br, b.m0c, b.bc,
                N.ptr(plan.wn_x), N.ptr(plan.wn_y), sc, N.ptr(scratch), N.ptr(band), s)
     elif kind != N.FIELD_COMPLEX_C64 and nch == 1 and b.m0c <= 0 < b.m0c + b.bc:
