@@ -185,7 +185,10 @@ OI_API int oi_band_spectrum_fft(const void* field, int kind, int batch, int ny, 
                                 int bc, const void* wn_x, const void* wn_y, float scale, void* scratch, void* band,
                                 void* stream);
 
-/* oi_band_spectrum_fft for complex fields [batch][ny][nx][nch]: band [batch][nch][br][bc]; scratch batch*nch*ny*bc complex. */
+/*
+ * oi_band_spectrum_fft for complex fields [batch][ny][nx][nch], batch * nch <= 65535: band [batch][nch][br][bc]; scratch
+ * batch*nch*ny*bc complex, 16-byte aligned.
+ */
 OI_API int oi_band_spectrum_fft_c64(const void* field, int batch, int ny, int nx, int nch, int m0r, int br, int m0c, int bc,
                                     const void* wn_x, const void* wn_y, float scale, void* scratch, void* band,
                                     void* stream);

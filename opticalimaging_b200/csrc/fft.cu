@@ -1200,7 +1200,8 @@ extern "C" int oi_band_spectrum_fft_c64(const void* field, int batch, int ny, in
   const int nx1 = n1_of(nx), ny1 = n1_of(ny);
   if (!nx1 || !ny1) return fail(OI_ERANGE, "oi_band_spectrum_fft_c64: grid %dx%d is not 256..2048, power of 2", ny, nx);
   const int maxc = max(abs(m0c), abs(m0c + bc - 1));
-  if (2 * maxc >= nx || br > ny || (long long)batch * nch > 0x7fffffffLL)
+  if ((long long)batch * nch > 65535) return fail(OI_ERANGE, "oi_band_spectrum_fft_c64: batch too large");   // as oi_band_spectrum
+  if (2 * maxc >= nx || br > ny)
     return fail(OI_ERANGE, "oi_band_spectrum_fft_c64: band (%d+%d, %d+%d) too wide for %dx%d", m0r, br, m0c, bc, ny, nx);
   cudaStream_t s = (cudaStream_t)stream;
   float2* t = (float2*)scratch;
