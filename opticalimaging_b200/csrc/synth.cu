@@ -212,9 +212,13 @@ __global__ void sum_parts_kernel(float* __restrict__ coarse, int nparts, long lo
   *(float4*)(coarse + i) = acc;
 }
 
+static int check_parts(int nparts, long long n) {
+  return nparts > 1 && n % 4 != 0 ? fail(OI_EINVAL, "partial sums of %lld floats are not float4 aligned", n) : (int)OI_OK;
+}
+
 int fold_parts(float* coarse, int nparts, long long n, cudaStream_t s) {
+  if (int rc = check_parts(nparts, n)) return rc;
   if (nparts <= 1) return OI_OK;
-  if (n % 4 != 0) return fail(OI_EINVAL, "partial sums of %lld floats are not float4 aligned", n);
   sum_parts_kernel<<<(unsigned)ceil_div(n / 4, 256), 256, 0, s>>>(coarse, nparts, n);
   oi::note_launch();
   return check_launch("coarse spectrum/sum parts");
@@ -225,6 +229,7 @@ int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, co
   if (mr < 2 * br - 1 || mc < 2 * bc - 1)
     return fail(OI_EINVAL, "coarse grid %dx%d too small for band %dx%d", mr, mc, br, bc);
   if (mr > 1024 || count > 65535) return fail(OI_ERANGE, "coarse grid mr=%d or count=%d out of range", mr, count);
+  if (int rc = check_parts(nparts, (long long)count * mr * mc)) return rc;   // whichever form runs
   // (a caller's images may start at any float; the pairs of U may not)
   if ((long long)count * mr * bc * (long long)sizeof(float2) <= room_bytes && (uintptr_t)room % alignof(float2) == 0) {
     float2* u = (float2*)room;
