@@ -128,14 +128,19 @@ def set_source_weights(model: CoherentModel, values: torch.Tensor, index_image: 
     if model.kind != 'abbe':
         raise ValueError('source weights belong to an Abbe model (abbe_model)')
     Z, K = model.weights.shape
-    v = values.detach().to(model.device, torch.float64).reshape(-1).contiguous()
-    S, P = v.numel(), getattr(model, 'pol_states', 1)      # fields are [polarisation state][point][component]
+    w = model.weights
+    S, P = values.numel(), getattr(model, 'pol_states', 1)      # fields are [polarisation state][point][component]
     if K % (P * S):
         raise ValueError(f'{S} source weights do not divide the model\'s {K} fields')
-    w = model.weights if model.weights.is_contiguous() else torch.empty_like(model.weights, memory_format=torch.contiguous_format)
-    N.call('oi_source_weights', N.ptr(v), S, K // (P * S), K, Z, float(index_image), N.ptr(w), N.stream_handle(model.device))
-    if w is not model.weights:
-        model.weights.copy_(w)
+    v = values.to(model.device, torch.float64).reshape(-1).contiguous()
+    if (w.dtype == torch.float32 and w.is_contiguous()
+            and not (w.requires_grad or v.requires_grad or w.is_inference())):
+        N.call('oi_source_weights', N.ptr(v), S, K // (P * S), K, Z, float(index_image), N.ptr(w),
+               N.stream_handle(model.device))
+        torch.autograd.graph.increment_version(w)   # an in-place change, to whatever has saved the weights
+    else:   # what autograd has to see or to refuse
+        per = ((index_image / v.sum()) * v).repeat_interleave(K // (P * S)).repeat(P)
+        w.copy_(per.to(torch.float32)[None].expand(Z, K))
     model.packed = None   # packed for the previous weights
 
 
