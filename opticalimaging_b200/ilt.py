@@ -20,6 +20,7 @@ from __future__ import annotations
 import ctypes
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _native as N
 from .autograd import aerial_image, source_weight_gradient
@@ -81,6 +82,11 @@ class _ResistLoss:
         return _ResistTerms.apply(image, target, steepness, threshold)[0]
 
 
+def _differentiated(t: torch.Tensor) -> bool:
+    """Whether autograd follows t, backward or forward (a dual tensor)."""
+    return t.requires_grad or forward_ad.unpack_dual(t).tangent is not None
+
+
 def ilt_loss(model: CoherentModel, mask: torch.Tensor, target: torch.Tensor, resist: ResistModel):
     """(loss, image): ||R(I(mask)) - target||^2 over pixels and planes; mask [B, ny, nx], target [B, ny, nx]."""
     image = aerial_image(model, mask)                        # [B, Z, ny, nx]
@@ -90,7 +96,7 @@ def ilt_loss(model: CoherentModel, mask: torch.Tensor, target: torch.Tensor, res
     if (type(resist) is ResistModel and isinstance(resist.steepness, (int, float))
             and isinstance(resist.threshold, (int, float)) and target.dtype == torch.float32 and target.device == image.device
             and target.shape == (image.shape[0],) + image.shape[2:] and target.is_contiguous()
-            and not target.requires_grad):
+            and not _differentiated(target)):
         return _ResistLoss.apply(image, target, float(resist.steepness), float(resist.threshold)), image
     loss = torch.sum((resist(image) - target[:, None]) ** 2)
     return loss, image
@@ -134,7 +140,7 @@ def set_source_weights(model: CoherentModel, values: torch.Tensor, index_image: 
         raise ValueError(f'{S} source weights do not divide the model\'s {K} fields')
     v = values.to(model.device, torch.float64).reshape(-1).contiguous()
     if (w.dtype == torch.float32 and w.is_contiguous()
-            and not (w.requires_grad or v.requires_grad or w.is_inference())):
+            and not (_differentiated(w) or _differentiated(v) or w.is_inference())):
         N.call('oi_source_weights', N.ptr(v), S, K // (P * S), K, Z, float(index_image), N.ptr(w),
                N.stream_handle(model.device))
         torch.autograd.graph.increment_version(w)   # an in-place change, to whatever has saved the weights

@@ -1,6 +1,7 @@
-"""ilt_loss with a resist whose parameters are tensors."""
+"""ilt_loss with a resist whose parameters are tensors, and with a target that carries a tangent."""
 import pytest
 import torch
+import torch.autograd.forward_ad as fwd
 
 from tests.fixtures import load
 
@@ -33,3 +34,16 @@ def test_resist_parameters_that_are_tensors(name, per_pixel):
     # FP32 sums of up to ny * nx terms of one order of magnitude
     assert value.grad is not None and abs(float(loss) - float(l64)) < 1e-5 * float(l64)
     assert float((value.grad - v64.grad).abs().max()) < 1e-4 * float(v64.grad.abs().max())
+
+
+def test_target_with_a_tangent():
+    from opticalimaging_b200 import ilt
+    model, mask, target = _setup()
+    with fwd.dual_level():
+        v = torch.randn(target.shape, generator=torch.Generator(device='cuda').manual_seed(1), device='cuda')
+        loss, image = ilt.ilt_loss(model, mask, fwd.make_dual(target, v), ilt.ResistModel(30.0, 0.25))
+        got = fwd.unpack_dual(loss).tangent
+    r = torch.sigmoid(30.0 * (image.double() - 0.25)) - target.double()[:, None]
+    want = float((-2.0 * r * v[:, None]).sum())
+    # an FP32 sum of ny * nx terms of both signs
+    assert got is not None and abs(float(got) - want) < 1e-5 * float((2.0 * r * v[:, None]).abs().sum())

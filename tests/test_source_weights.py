@@ -1,9 +1,10 @@
 """set_source_weights writes the model's weights as an in-place torch copy does: seen by autograd's version check, and with
-the gradient of values that require one."""
+the gradient or the tangent of values that have one."""
 from types import SimpleNamespace
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwd
 
 from opticalimaging_b200 import ilt
 
@@ -49,3 +50,14 @@ def test_autograd_sees_the_change(strided):
     assert torch.allclose(model.weights, _want(v, 3, 2, 1.3))
     with pytest.raises(RuntimeError, match='modified by an inplace operation'):
         loss.backward()
+
+
+def test_values_with_a_tangent():
+    model = _model('cpu')
+    v = torch.tensor([0.5, 1.0, 2.0, 0.25], dtype=torch.float64)
+    d = torch.tensor([1.0, -2.0, 0.5, 3.0], dtype=torch.float64)
+    with fwd.dual_level():
+        ilt.set_source_weights(model, fwd.make_dual(v, d), 1.3)
+        w, t = fwd.unpack_dual(model.weights)
+    u, j = _want(v, 3, 2, 1.3), 1.3 * (d / v.sum() - v * d.sum() / v.sum() ** 2)
+    assert torch.allclose(w, u) and torch.allclose(t, j.repeat_interleave(3).float().expand(2, -1))
