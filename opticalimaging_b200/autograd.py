@@ -16,6 +16,7 @@ tests compare both, and central finite differences in FP64.
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _native as N
 from .engine import Band, CoherentModel, Plan, band_spectrum, coherent_image, field_split_sm
@@ -180,7 +181,12 @@ def source_weight_gradient(model: CoherentModel, mask: torch.Tensor, g: torch.Te
         E = K // (S * P)
         if S * P * E != K:
             raise ValueError(f'{S} source weights do not divide the model\'s {K} fields')
-        v = values.detach().to(dots.device, torch.float64).reshape(-1).contiguous()
+        v = values.to(dots.device, torch.float64).reshape(-1)
+        if forward_ad.unpack_dual(v).tangent is not None:   # torch operations carry the tangent
+            d = dots.view(B, Z, P, S, E).sum(dim=(1, 2, 4)).double()    # <g, I_j>
+            W = v.sum()
+            return ((index_image * d - (d * v).sum(dim=1, keepdim=True) * index_image / W) / W).float()
+        v = v.contiguous()
         out = torch.empty((B, S), dtype=torch.float32, device=dots.device)
         N.call('oi_source_gradient', N.ptr(dots), B, Z, P, S, E, N.ptr(v), float(index_image), N.ptr(out),
                N.stream_handle(dots.device))

@@ -47,3 +47,24 @@ def test_target_with_a_tangent():
     want = float((-2.0 * r * v[:, None]).sum())
     # an FP32 sum of ny * nx terms of both signs
     assert got is not None and abs(float(got) - want) < 1e-5 * float((2.0 * r * v[:, None]).abs().sum())
+
+
+def test_source_gradient_with_a_tangent():
+    from opticalimaging_b200.engine import Band, CoherentModel
+    from opticalimaging_b200.autograd import source_weight_gradient
+    g = torch.Generator(device='cuda').manual_seed(2)
+    S, n = 5, 256
+    pupils = torch.randn((1, S, 9, 9), generator=g, dtype=torch.complex64, device='cuda')
+    model = CoherentModel(pupils, torch.ones((1, S), device='cuda'), Band(-4, 9, -4, 9), n, n, 'abbe')
+    mask, grad = torch.rand((2, n, n), generator=g, device='cuda'), torch.randn((2, 1, n, n), generator=g, device='cuda')
+    v = 0.5 + torch.rand(S, generator=g, dtype=torch.float64, device='cuda')
+    t = torch.randn(S, generator=g, dtype=torch.float64, device='cuda')
+    at = lambda v: source_weight_gradient(model, mask, grad, v, 1.3)  # noqa: E731
+    with fwd.dual_level():
+        value, tangent = fwd.unpack_dual(at(fwd.make_dual(v, t)))
+    step = 1e-3
+    want = (at(v + step * t).double() - at(v - step * t).double()) / (2 * step)
+    # the central difference: FP32 results 2e-3 apart, and its own error of step^2
+    top = float(value.abs().max())
+    assert float((value - at(v)).abs().max()) < 1e-6 * top
+    assert tangent is not None and float((tangent - want).abs().max()) < 1e-3 * top
