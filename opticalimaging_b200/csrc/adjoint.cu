@@ -270,11 +270,16 @@ extern "C" int oi_hermitian_half(const void* w, int nparts, int batch, int nz, i
   using namespace oi;
   if (!w || !half || nparts <= 0 || batch <= 0 || nz <= 0 || br <= 0 || bc <= 0)
     return fail(OI_EINVAL, "oi_hermitian_half: bad arguments");
-  if (batch > 65535) return fail(OI_ERANGE, "oi_hermitian_half: batch=%d", batch);
   const int R = max(abs(m0r), abs(m0r + br - 1)), C = max(abs(m0c), abs(m0c + bc - 1));
-  dim3 grid((unsigned)ceil_div((long long)(2 * R + 1) * (C + 1), 32), (unsigned)batch);
-  hermitian_half_kernel<<<grid, 32 * HERM_Q, 0, (cudaStream_t)stream>>>((const float2*)w, nparts, (long long)batch * nz * br * bc, nz, br,
-                                                                bc, m0r, m0c, R, C, scale, (float2*)half);
-  oi::note_launch();
-  return check_launch("oi_hermitian_half");
+  const long long band = (long long)br * bc, size = (long long)(2 * R + 1) * (C + 1);
+  constexpr int MOST = 65535;   // images per launch: the grid's second dimension
+  for (int b = 0; b < batch; b += min(MOST, batch - b)) {
+    dim3 grid((unsigned)ceil_div(size, 32), (unsigned)min(MOST, batch - b));
+    hermitian_half_kernel<<<grid, 32 * HERM_Q, 0, (cudaStream_t)stream>>>((const float2*)w + (long long)b * nz * band, nparts,
+                                                                          (long long)batch * nz * band, nz, br, bc, m0r, m0c, R, C,
+                                                                          scale, (float2*)half + b * size);
+    oi::note_launch();
+    if (int rc = check_launch("oi_hermitian_half")) return rc;
+  }
+  return OI_OK;
 }

@@ -32,3 +32,19 @@ def test_synthesis_of_many_images(m):
         g = got[i0:i0 + 7 * 512]
         # the few images take row blocks of another size: the same sums, each of a few FP32 operations
         assert float((g - want.repeat(513, 1, 1)[:g.shape[0]]).abs().max()) < 1e-6
+
+
+def test_hermitian_half_of_many_images():
+    from opticalimaging_b200 import _native as N
+    B, nz, parts, br, bc = 65537, 2, 3, 3, 2
+    rng = np.random.default_rng(1)
+    w = (rng.standard_normal((parts, B, nz, br, bc)) + 1j * rng.standard_normal((parts, B, nz, br, bc))).astype(np.complex64)
+    wd = torch.from_numpy(w).cuda()
+    half = torch.full((B, 3, 2), 9.0, dtype=torch.complex64, device='cuda')
+    N.call('oi_hermitian_half', N.ptr(wd), parts, B, nz, -1, br, 0, bc, 1.5, N.ptr(half), N.stream_handle())
+    full = np.zeros((B, 3, 3), complex)
+    full[:, :, 1:] = w.astype(complex).sum(axis=(0, 2))
+    want = (full + np.conj(full[:, ::-1, ::-1]))[:, :, 1:] * 1.5
+    want[:, :, 0] *= 0.5
+    # sums of 12 FP32 values of a few units
+    assert np.max(np.abs(half.cpu().numpy() - want)) < 2e-5
