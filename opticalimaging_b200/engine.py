@@ -85,9 +85,16 @@ def fft_supported(ny: int, nx: int, band: Band) -> bool:
     return 2 * maxc < nx and band.br <= ny and 2 * band.br - 1 <= ny and 2 * band.bc - 1 <= nx
 
 
+def _shared(device) -> None:
+    """Tables just enqueued on the device's current stream will be read on any stream: wait for them once, here (but not
+    inside a graph capture, where a wait is not allowed and the tables belong to the graph)."""
+    if torch.device(device).type == 'cuda' and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(device).synchronize()
+
+
 class Plan:
-    """Phase tables for one (output grid, band); cached and shared by every call with the same key.  The cache
-    keeps the CACHE_SIZE most recently used plans (a model holds on to its own plan regardless)."""
+    """Phase tables for one (output grid, band); cached and shared by every call with the same key, on any stream.  The
+    cache keeps the CACHE_SIZE most recently used plans (a model holds on to its own plan regardless)."""
 
     CACHE_SIZE = 64
     _cache: collections.OrderedDict = collections.OrderedDict()
@@ -119,6 +126,7 @@ class Plan:
         if self.coarse_small:                                 # the coarse-grid FFT tables
             self.wm_r = t(1, self.mr, 1, 0, self.mr, +1)
             self.wm_c = t(1, self.mc, 1, 0, self.mc, +1)
+        _shared(device)
 
     def tc_constants(self) -> torch.Tensor:
         """The split DFT operand image of the tensor-core form (built once per plan; coarse grid 128 x 128)."""
@@ -129,6 +137,7 @@ class Plan:
             c = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             N.call('oi_tc_constants', b.m0r, b.m0c, N.ptr(self.wm_r), N.ptr(self.wm_c), N.ptr(c), nbytes,
                    N.stream_handle(self.device))
+            _shared(self.device)
             self._tc_consts = c
         return c
 
@@ -154,6 +163,7 @@ class Plan:
             nbytes = {0: (self.nx // 64) * 32768, 1: (self.nx // 128) * 65536, 2: (self.nx // 64) * 16384}[which]
             c = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             N.call('oi_rows_tc_constants', which, self.nx, b.m0c, b.bc, N.ptr(c), nbytes, N.stream_handle(self.device))
+            _shared(self.device)
             setattr(self, attr, c)
         return c
 
@@ -166,6 +176,7 @@ class Plan:
             nbytes = (1 + self.ny // 128) * 65536
             c = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             N.call('oi_synth_tc_constants', self.ny, b.br, b.bc, N.ptr(c), nbytes, N.stream_handle(self.device))
+            _shared(self.device)
             self._synth_consts = c
         return c
 
@@ -173,7 +184,9 @@ class Plan:
         """Four-step FFT tables of the coarse grid (for coarse grids of 256..2048 points per axis)."""
         t = getattr(self, '_coarse_fft_tables', None)
         if t is None:
-            t = self._coarse_fft_tables = (fft_tables(self.mr, self.device), fft_tables(self.mc, self.device))
+            t = (fft_tables(self.mr, self.device), fft_tables(self.mc, self.device))
+            _shared(self.device)
+            self._coarse_fft_tables = t
         return t
 
     def big_coarse_fft(self, form) -> bool:
@@ -522,11 +535,16 @@ class CoherentModel:
         b, p = self.band, self.plan
         nz = self.planes
         form = self.form if form is None else form
-        split = (field_split_sm(self.count * nch, batch * nz) if p.use_coarse_fft(None) or p.use_coarse256(form)
-                 else field_split(self.count * nch, batch * nz * ((p.mr + 15) // 16)))
+        fields = {nch * self.count}
+        if self.packed is not None and nch == 1:
+            fields.add(self.packed[0].shape[1])
         if form == 'bf16x3':
-            split = tc_parts_bound(batch * nz, self.count * nch)
+            split = max(tc_parts_bound(batch * nz, n) for n in fields)
             p = Plan.get(self.ny, self.nx, b, self.device, coarse=TC_COARSE)
+        elif p.use_coarse_fft(form) or p.use_coarse256(form):
+            split = max(field_split_sm(n, batch * nz) for n in fields)
+        else:
+            split = max(field_split(n, batch * nz * ((p.mr + 15) // 16)) for n in fields)
         tiles = batch * nz * p.ny * 512 if form == 'bf16x3' else 0
         return 8 * (batch * nch * p.ny * b.bc + batch * nch * b.br * b.bc + batch * nz * (2 * b.br - 1) * b.bc
                     + batch * nz * b.bc * p.ny) + 4 * split * batch * nz * p.mr * p.mc + tiles
