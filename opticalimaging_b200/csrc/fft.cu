@@ -865,19 +865,18 @@ __global__ void __launch_bounds__(COARSE_T) coarse_cols_kernel(long long ncols, 
 }
 
 // --------------------------------------------------------------- coarse intensity -> its spectrum
-// COARSE_PARTS blocks per coarse image, each for a range of the band columns qc (mr = 32 N1R, mc = 32 N1C, each
-// 64 or 128; U holds the block's columns only, so that two blocks fit an SM):
+// For the tensor-core synthesis.  COARSE_PARTS blocks per coarse image, each for a range of the band columns qc (mr = mc =
+// 128; U holds the block's columns only, so that two blocks fit an SM):
 //   ihat[i][jr][qc] = (qc ? 2 : 1) / (mr mc) * sum_{sr,sc} coarse[i][sr][sc] exp(+2 pi i (qr sr/mr + qc sc/mc))
 // for qr = jr - (br-1) in [-(br-1), br-1] and qc in [0, bc).  Row FFTs of the real image in pairs (two rows per
 // complex transform), the band bins of each separated into U[sr][qc]; then column FFTs of U at the qr bins.
-constexpr int COARSE_PARTS = 2;
-template <int N1R, int N1C>
+constexpr int COARSE_PARTS = 2, SPEC_N1 = 4, SPEC_M = 32 * SPEC_N1;
 __global__ void __launch_bounds__(512) coarse_spec_fft_kernel(const float* __restrict__ coarse, int nparts,
                                                               long long part_stride, int br, int bc,
                                                               const float2* __restrict__ wr_g,
                                                               const float2* __restrict__ wc_g, int area_f2,
                                                               float2* __restrict__ ihat) {
-  constexpr int MR = 32 * N1R, MC = 32 * N1C, T = 512;
+  constexpr int N1R = SPEC_N1, N1C = SPEC_N1, MR = SPEC_M, MC = SPEC_M, T = 512;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* r2 = (float2*)smem_raw;      // row-axis (MR) tables: [32][N1R], [N1R][N1R]
   float2* r1 = r2 + 32 * N1R;
@@ -957,15 +956,14 @@ __global__ void __launch_bounds__(512) coarse_spec_fft_kernel(const float* __res
   }
 }
 
-template <int N1R, int N1C>
 static int launch_coarse_spec_fft(float* coarse, int nparts, int count, int br, int bc, const float2* wr,
                                   const float2* wc, float2* ihat, cudaStream_t s) {
-  constexpr int MR = 32 * N1R, MC = 32 * N1C;
+  constexpr int N1R = SPEC_N1, N1C = SPEC_N1, MR = SPEC_M, MC = SPEC_M;
   const int cw = (bc + COARSE_PARTS - 1) / COARSE_PARTS;   // band columns per block (as in the kernel)
   const int rows_ys = (MR / 2) * 32 * (N1C + 1), c_f2 = MR * MC / 2, cols_ys = cw * 32 * (N1R + 1);
   const int area_f2 = max(rows_ys, max(c_f2, cols_ys));
   const size_t smem = sizeof(float2) * ((size_t)table_f2<N1R>() + table_f2<N1C>() + area_f2 + (size_t)MR * cw);
-  auto kern = coarse_spec_fft_kernel<N1R, N1C>;
+  auto kern = coarse_spec_fft_kernel;
   int rc = set_smem(kern, smem, "coarse spectrum fft");
   if (rc) return rc;
   (void)launch_pdl(kern, dim3((unsigned)count, COARSE_PARTS), dim3(512), smem, s, (const float*)coarse, nparts,
@@ -1430,7 +1428,7 @@ extern "C" int oi_coarse_to_image_tc(float* coarse, int nparts, int count, int b
     return fail(OI_ERANGE, "oi_coarse_to_image_tc: grid %dx%d / band %dx%d unsupported", ny, nx, br, bc);
   cudaStream_t s = (cudaStream_t)stream;
   float2* ih = (float2*)scratch_ihat;
-  int rc = launch_coarse_spec_fft<4, 4>(coarse, nparts, count, br, bc, (const float2*)wm_r, (const float2*)wm_c, ih, s);
+  int rc = launch_coarse_spec_fft(coarse, nparts, count, br, bc, (const float2*)wm_r, (const float2*)wm_c, ih, s);
   if (rc) return rc;
   unsigned char* tiles = (unsigned char*)scratch_tiles;
   const float2* wy = (const float2*)wn_y;

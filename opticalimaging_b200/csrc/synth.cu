@@ -16,10 +16,9 @@ namespace oi {
 constexpr int SP_QT = 16;  // qc per spec block
 
 // grid (ceil(bc/16), count).  ihat[i][jr][qc], jr = qr + br - 1.
-__global__ void __launch_bounds__(256) coarse_spec_kernel(const float* __restrict__ coarse, int nparts,
-                                                          long long part_stride, int mr, int mc, int br,
-                                                          int bc, const float2* __restrict__ gc,
-                                                          const float2* __restrict__ gr, float2* __restrict__ ihat) {
+__global__ void __launch_bounds__(256) coarse_spec_kernel(const float* __restrict__ coarse, int mr, int mc, int br, int bc,
+                                                          const float2* __restrict__ gc, const float2* __restrict__ gr,
+                                                          float2* __restrict__ ihat) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* us = (float2*)smem_raw;  // [mr][SP_QT]
   const int tid = threadIdx.x, ql = tid % SP_QT, rg = tid / SP_QT;  // rg 0..15
@@ -34,9 +33,8 @@ __global__ void __launch_bounds__(256) coarse_spec_kernel(const float* __restric
     if (qc < bc) {
       const float* row = cimg + (long long)sr * mc;
       for (int sc = 0; sc < mc; ++sc) {
-        float v = __ldg(row + sc);
-        for (int p = 1; p < nparts; ++p) v += __ldg(row + p * part_stride + sc);
-        float2 t = __ldg(gc + (long long)sc * bc + qc);
+        const float v = __ldg(row + sc);
+        const float2 t = __ldg(gc + (long long)sc * bc + qc);
         u.x = fmaf(v, t.x, u.x);
         u.y = fmaf(v, t.y, u.y);
       }
@@ -246,15 +244,13 @@ int coarse_spectrum(float* coarse, int count, int mr, int mc, int br, int bc, co
   }
   int rc = fold_parts(coarse, nparts, (long long)count * mr * mc, s);
   if (rc) return rc;
-  nparts = 1;
   size_t smem = sizeof(float2) * (size_t)mr * SP_QT;
   {
     int rc_smem = ensure_smem((const void*)coarse_spec_kernel, smem, "coarse spectrum");
     if (rc_smem) return rc_smem;
   }
   dim3 g1((unsigned)ceil_div(bc, SP_QT), (unsigned)count);
-  coarse_spec_kernel<<<g1, 256, smem, s>>>(coarse, nparts, (long long)count * mr * mc, mr, mc, br, bc,
-                                           (const float2*)gc, (const float2*)gr, (float2*)ihat);
+  coarse_spec_kernel<<<g1, 256, smem, s>>>(coarse, mr, mc, br, bc, (const float2*)gc, (const float2*)gr, (float2*)ihat);
   oi::note_launch();
   return check_launch("coarse spectrum");
 }
