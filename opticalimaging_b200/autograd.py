@@ -138,7 +138,8 @@ class _CoherentImage(torch.autograd.Function):
             model.check_grid(m)
             band = band_spectrum(m, N.FIELD_REAL_F32, model.plan, form=model.form)
             image = coherent_image(band, *model.fields_for(N.FIELD_REAL_F32), model.plan, form=model.form)
-        # the backward pass starts from the FP32 band spectrum: the forward's own, unless that ran in split form
+        # the backward pass starts from the plan's default FP32 band spectrum: the forward's own, or, for a model in another
+        # form ('dft', 'bf16x3'), one of its own
         ctx.save_for_backward(mask, band if model.form in (None, 'fft') else None)
         return image                                                        # [B, Z, ny, nx] for every model
 
