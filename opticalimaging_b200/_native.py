@@ -130,10 +130,11 @@ def stream_handle(device=None):
     refused: calls pass their tensors' device here, and a host tensor's address must not reach a kernel."""
     index = None
     if device is not None:
-        d = torch.device(device)
-        if d.type != 'cuda':
-            raise ValueError(f'expected a CUDA device, got {d}')
-        index = d.index
+        if not isinstance(device, torch.device):
+            device = torch.device(device)
+        if device.type != 'cuda':
+            raise ValueError(f'expected a CUDA device, got {device}')
+        index = device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 

@@ -18,6 +18,7 @@ The reference has no optimisation loop; it differentiates its SOCS image by torc
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 from torch.autograd import forward_ad
@@ -37,6 +38,14 @@ class ResistModel:
         return torch.sigmoid(self.steepness * (image - self.threshold))
 
 
+@functools.cache
+def _loss_workspace() -> int:
+    """Bytes of the loss kernel's partial sums (the library's own constant)."""
+    nbytes = ctypes.c_longlong(0)
+    N.call('oi_resist_loss_workspace', ctypes.byref(nbytes))
+    return nbytes.value
+
+
 class _ResistTerms(torch.autograd.Function):
     """(loss, D, s) in one pass over the images: loss = sum (s - target)^2, s = sigmoid(a (I - thr)), D = dloss/dI.
 
@@ -50,11 +59,10 @@ class _ResistTerms(torch.autograd.Function):
         B, Z, ny, nx = img.shape
         grad, s = (torch.empty_like(img), torch.empty_like(img)) if ctx.needs_input_grad[0] else (None, None)
         loss = torch.empty((), dtype=torch.float32, device=img.device)
-        nbytes = ctypes.c_longlong(0)
-        N.call('oi_resist_loss_workspace', ctypes.byref(nbytes))
-        work = torch.empty(nbytes.value, dtype=torch.uint8, device=img.device)
+        nbytes = _loss_workspace()
+        work = torch.empty(nbytes, dtype=torch.uint8, device=img.device)
         N.call('oi_resist_loss_terms', N.ptr(img), N.ptr(target), B, Z, ny * nx, steepness, threshold, N.ptr(grad), N.ptr(s),
-               N.ptr(loss), N.ptr(work), nbytes.value, N.stream_handle(img.device))
+               N.ptr(loss), N.ptr(work), nbytes, N.stream_handle(img.device))
         if grad is not None:
             ctx.set_materialize_grads(False)
             ctx.steepness = steepness
