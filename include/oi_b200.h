@@ -309,6 +309,12 @@ OI_API int oi_device_status(int* status, int reset);
  * tensor memory and returns.  For tests of the status reporting and of the context staying usable. */
 OI_API int oi_wait_probe(long long limit_ns, int tmem_cols, void* stream);
 
+/*
+ * Waits for the work enqueued on a stream so far; returns at once when the stream is being captured.  Allowed while another
+ * thread captures a stream in any mode.  For tables that later calls read on other streams.
+ */
+OI_API int oi_stream_wait(void* stream);
+
 /* Kernel launches this library has enqueued since it was loaded (launches captured into a CUDA graph are
  * counted once, at capture). */
 OI_API int oi_launch_count(long long* count);

@@ -87,6 +87,23 @@ extern "C" int oi_twiddle(void* out, int rows, int cols, long long a0, long long
   return oi::check_launch("oi_twiddle");
 }
 
+extern "C" int oi_stream_wait(void* stream) {
+  using namespace oi;
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &cap);
+  if (e != cudaSuccess) return fail(OI_ECUDA, "oi_stream_wait: cudaStreamIsCapturing: %s", cudaGetErrorString(e));
+  if (cap != cudaStreamCaptureStatusNone) return OI_OK;
+  // another thread may be capturing in the global mode, which forbids this thread the wait unless it asks for the relaxed one
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return fail(OI_ECUDA, "oi_stream_wait: capture mode: %s", cudaGetErrorString(e));
+  e = cudaStreamSynchronize(s);
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return fail(OI_ECUDA, "oi_stream_wait: %s", cudaGetErrorString(e));
+  return OI_OK;
+}
+
 extern "C" int oi_launch_count(long long* count) {
   if (!count) return oi::fail(OI_EINVAL, "oi_launch_count: null count");
   *count = oi::g_launches.load(std::memory_order_relaxed);

@@ -87,9 +87,8 @@ def fft_supported(ny: int, nx: int, band: Band) -> bool:
 
 def _shared(device) -> None:
     """Tables just enqueued on the device's current stream will be read on any stream: wait for them once, here (but not
-    inside a graph capture, where a wait is not allowed and the tables belong to the graph)."""
-    if torch.device(device).type == 'cuda' and not torch.cuda.is_current_stream_capturing():
-        torch.cuda.current_stream(device).synchronize()
+    where the stream is being captured: there the tables belong to the graph)."""
+    N.call('oi_stream_wait', N.stream_handle(device))
 
 
 class Plan:

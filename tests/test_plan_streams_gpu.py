@@ -32,3 +32,35 @@ def test_tables_of_another_stream(what):
     torch.cuda.synchronize()
     for c, w in zip(copies, want):
         assert torch.equal(c, w)
+
+
+def test_plan_built_while_another_thread_captures():
+    """The wait for a plan's tables does not break a capture (of the mode that forbids other threads to wait)."""
+    import threading
+    from opticalimaging_b200 import engine as eng
+    dev, band = torch.device('cuda', torch.cuda.current_device()), eng.Band(-29, 59, -29, 59)
+    eng.Plan(512, 512, band, dev)        # its memory stays with the allocator
+    torch.cuda.synchronize()
+    x, built = torch.ones(1000, device=dev), []
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode='global'):
+        y = x * 2.0
+        t = threading.Thread(target=lambda: built.append(eng.Plan(512, 512, band, dev)))
+        t.start()
+        t.join()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert len(built) == 1 and float(y[0]) == 2.0
+
+
+def test_tables_built_inside_a_capture():
+    from opticalimaging_b200 import engine as eng
+    dev, band = torch.device('cuda', torch.cuda.current_device()), eng.Band(-29, 59, -29, 59)
+    want = eng.Plan(512, 512, band, dev).coarse_fft_tables()
+    plan = eng.Plan(512, 512, band, dev)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [t.clone() for t in plan.coarse_fft_tables()]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
